@@ -7,15 +7,153 @@
 // (hqc/pbc/slater.py:42-104) for walker batches.  FP64 throughout.  The
 // k-point variant (eval_pbc_ao_kpt, gto.py:371-427) weights each lattice
 // term with exp(i k_d t) and returns complex Bloch AO values.
+#include <algorithm>
+#include <cmath>
+#include <vector>
+
 #include "common.cuh"
+#include "exp_table.cuh"
 #include "zmath.cuh"
 #include "kernels.h"
 
 namespace hqcgb {
 
 constexpr int kPtMaxPrim = 16;
+constexpr int kPtMaxAo = 16;   // AOs per atom and 1D images of k_ao_cell
+constexpr int kPtMaxLat = 65;
 
-// One thread per (point, atom): out[pt][A * nb + j].
+__device__ inline double2 zmul(double a, double2 b) { return make_double2(a * b.x, a * b.y); }
+__device__ inline double zmul(double a, double b) { return a * b; }
+__device__ inline void zfma(double w, double p, double &s) { s = fma(w, p, s); }
+__device__ inline void zfma(double w, double2 p, double2 &s) {
+  s.x = fma(w, p.x, s.x);
+  s.y = fma(w, p.y, s.y);
+}
+template <typename Z> __device__ inline Z zzero();
+template <> __device__ inline double zzero<double>() { return 0.0; }
+template <> __device__ inline double2 zzero<double2>() { return make_double2(0.0, 0.0); }
+
+// AO values, one thread per (point, atom), for the images lat[t] = (t - tm) a
+// of a periodic box, t = 0..2 tm (Z = double2: image t weighted with phase
+// ph[d][t]).  Relative to the image nearest along each axis, u = x - t0 a,
+// image t0 + m contributes exp(-alpha m a (m a -+ 2 |u|)) <= 1, and the three
+// nearest ones share one exponential:
+//   f_x f_y f_z = exp(-alpha |u|^2) prod_d sum_m w_m,d  (l = 1: (u - m a) w).
+// Factors below e^-41 (1.6e-18 of the nearest image's term) are left out;
+// their exponents are tested in FP32.  For sharp primitives no other image
+// counts, so a point and atom take about 25 exponentials of 11 FP64
+// instructions (exp_table.cuh) where the image sums of all axes and primitives
+// take 105 of 30; the kernel is bound by the FP64 pipe.  Measured with 54
+// atoms, dzvp, box 8 Bohr: AO values of 2048 walkers 25.4 -> 9.0 ms, of one
+// walker 238 -> 167 us a call.
+template <int NB, typename Z>
+__global__ void __launch_bounds__(128)
+    k_ao_cell(int n_atoms, int nb, int nprim, int tm, double a, const double *__restrict__ tables,
+              const int *__restrict__ ao_l, const int *__restrict__ ao_cart, const double *__restrict__ xp,
+              long long npts, int pts_per_group, const double *__restrict__ xe, Z *__restrict__ out) {
+  constexpr bool kPhase = sizeof(Z) > sizeof(double);
+  __shared__ double s_exp[kExpTable], s_alpha[kPtMaxPrim], s_coef[NB * kPtMaxPrim];
+  __shared__ double2 s_ph[kPhase ? 3 * kPtMaxLat : 1];
+  __shared__ int s_type[NB];  // 0: s, 1 + axis: p
+  const int nlat = 2 * tm + 1;
+  for (int k = threadIdx.x; k < kExpTable; k += blockDim.x) s_exp[k] = tables[k];
+  for (int k = threadIdx.x; k < nprim; k += blockDim.x) s_alpha[k] = tables[kExpTable + k];
+  for (int k = threadIdx.x; k < nb * nprim; k += blockDim.x) s_coef[k] = tables[kExpTable + nprim + k];
+  if (kPhase)
+    for (int k = threadIdx.x; k < 3 * nlat; k += blockDim.x) {
+      const double *p = tables + kExpTable + nprim + nb * nprim + 2 * k;
+      s_ph[k] = make_double2(p[0], p[1]);
+    }
+  for (int k = threadIdx.x; k < nb; k += blockDim.x) s_type[k] = ao_l[k] == 1 ? 1 + ao_cart[k] : 0;
+  __syncthreads();
+  const long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  if (idx >= npts * n_atoms) return;
+  long long pt, grp;
+  if (npts * n_atoms < (1LL << 32)) {  // 32-bit divisions
+    pt = (unsigned)idx / (unsigned)n_atoms;
+    grp = (unsigned)pt / (unsigned)pts_per_group;
+  } else {
+    pt = idx / n_atoms;
+    grp = pt / pts_per_group;
+  }
+  const int A = (int)(idx - pt * n_atoms);
+  const double *xa = xp + (grp * n_atoms + A) * 3;
+  const double *r = xe + pt * 3;
+  const double inv_a = 1.0 / a;
+  double u[3];
+  float rel[3];  // 2 u / a
+  int t0[3];
+#pragma unroll
+  for (int d = 0; d < 3; ++d) {
+    const double x = r[d] - xa[d];
+    const double t = fmin(fmax(rint(x * inv_a), -(double)tm), (double)tm);
+    t0[d] = (int)t;
+    u[d] = __dsub_rn(x, __dmul_rn(t, a));  // the image sums' x - lat[t]
+    rel[d] = 2.f * (float)(u[d] * inv_a);
+  }
+  const double r2 = u[0] * u[0] + u[1] * u[1] + u[2] * u[2];
+  Z v[NB];
+#pragma unroll
+  for (int j = 0; j < NB; ++j) v[j] = zzero<Z>();
+  for (int q = 0; q < nprim; ++q) {
+    const double al = s_alpha[q], ala = -al * a;
+    const float alf = (float)ala * (float)a;
+    Z S0[3], S1[3];
+#pragma unroll
+    for (int d = 0; d < 3; ++d) {
+      auto phase = [&](int m) {
+        if constexpr (kPhase) return s_ph[d * nlat + t0[d] + tm + m];
+        else return 1.0;
+      };
+      S0[d] = phase(0);
+      S1[d] = zmul(u[d], phase(0));
+#pragma unroll
+      for (int side = -1; side <= 1; side += 2) {
+        // image t0 + side m lies at u - side m a
+        const int most = side > 0 ? tm - t0[d] : tm + t0[d];
+        if (most < 1 || !(alf * (1.f - side * rel[d]) > -41.f)) continue;
+        const double w1 = exp_neg(ala * (a - 2 * side * u[d]), s_exp);
+        zfma(w1, phase(side), S0[d]);
+        zfma(w1 * (u[d] - side * a), phase(side), S1[d]);
+        for (int m = 2; m <= most; ++m) {
+          if (!(alf * m * (m - side * rel[d]) > -41.f)) break;
+          const double ma = m * a, w = exp_neg(-al * ma * (ma - 2 * side * u[d]), s_exp);
+          zfma(w, phase(side * m), S0[d]);
+          zfma(w * (u[d] - side * ma), phase(side * m), S1[d]);
+        }
+      }
+    }
+    const double e = exp_neg(-al * r2, s_exp);
+    const Z yz = zmul(S0[1], S0[2]), ex = zmul(e, S0[0]);
+    const Z P0 = zmul(ex, yz), P1 = zmul(zmul(e, S1[0]), yz), P2 = zmul(ex, zmul(S1[1], S0[2])),
+            P3 = zmul(ex, zmul(S0[1], S1[2]));
+#pragma unroll
+    for (int j = 0; j < NB; ++j) {
+      if (j >= nb) break;
+      const double c = s_coef[j * nprim + q];
+      if (c == 0.0) continue;
+      const int ty = s_type[j];
+      zfma(c, ty == 0 ? P0 : ty == 1 ? P1 : ty == 2 ? P2 : P3, v[j]);
+    }
+  }
+  const long long nao = (long long)n_atoms * nb;
+#pragma unroll
+  for (int j = 0; j < NB; ++j)
+    if (j < nb) out[pt * nao + (long long)A * nb + j] = v[j];
+}
+
+// Whether lat[0..n) are the images (t - tm) a, t = 0..2 tm, of a box (host).
+static bool box_images(int n, const double *lat, int *tm, double *a) {
+  if (n % 2 == 0 || n > kPtMaxLat) return false;
+  *tm = n / 2;
+  *a = n > 1 ? lat[n / 2 + 1] : 1.0;
+  if (!(*a > 0)) return false;
+  for (int t = 0; t < n; ++t)
+    if (!(std::fabs(lat[t] - (t - *tm) * *a) <= 4e-16 * std::fabs(lat[t]))) return false;
+  return true;
+}
+
+// Any image list or basis size: one thread per (point, atom): out[pt][A * nb + j].
 __global__ void k_ao_points(int n_atoms, int nb, int nprim, const double *__restrict__ alpha,
                             const double *__restrict__ coef, const int *__restrict__ ao_l,
                             const int *__restrict__ ao_cart, int nlat, const double *__restrict__ lat,
@@ -55,6 +193,117 @@ __global__ void k_ao_points(int n_atoms, int nb, int nprim, const double *__rest
   }
 }
 
+
+// k-point AO values (complex): one thread per (point, atom), out[pt][A * nb + j].
+__global__ void k_ao_points_kpt(int n_atoms, int nb, int nprim, const double *__restrict__ alpha,
+                                const double *__restrict__ coef, const int *__restrict__ ao_l,
+                                const int *__restrict__ ao_cart, int nlat,
+                                const double *__restrict__ lat, double k0, double k1, double k2,
+                                const double *__restrict__ xp, long long npts, int pts_per_group,
+                                const double *__restrict__ xe, double2 *__restrict__ out) {
+  const long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  if (idx >= npts * n_atoms) return;
+  const int A = (int)(idx % n_atoms);
+  const long long pt = idx / n_atoms;
+  const long long grp = pt / pts_per_group;
+  const double *xa = xp + (grp * n_atoms + A) * 3;
+  const double *r = xe + pt * 3;
+  const double kk[3] = {k0, k1, k2};
+  double2 f[3][kPtMaxPrim][2];
+  for (int d = 0; d < 3; ++d) {
+    const double x = r[d] - xa[d];
+    for (int a = 0; a < nprim; ++a) f[d][a][0] = f[d][a][1] = make_double2(0.0, 0.0);
+    for (int t = 0; t < nlat; ++t) {
+      const double u = x - lat[t];
+      double sn, cs;
+      sincos(kk[d] * lat[t], &sn, &cs);
+      for (int a = 0; a < nprim; ++a) {
+        const double g = exp(-alpha[a] * u * u);
+        f[d][a][0].x += g * cs;
+        f[d][a][0].y += g * sn;
+        f[d][a][1].x += u * g * cs;
+        f[d][a][1].y += u * g * sn;
+      }
+    }
+  }
+  const long long nao = (long long)n_atoms * nb;
+  for (int j = 0; j < nb; ++j) {
+    const int l = ao_l[j], ca = ao_cart[j];
+    const int px = (l == 1 && ca == 0), py = (l == 1 && ca == 1), pz = (l == 1 && ca == 2);
+    double2 v = make_double2(0.0, 0.0);
+    for (int a = 0; a < nprim; ++a) {
+      const double2 t = zmul(zmul(f[0][a][px], f[1][a][py]), f[2][a][pz]);
+      v.x += coef[j * nprim + a] * t.x;
+      v.y += coef[j * nprim + a] * t.y;
+    }
+    out[pt * nao + (long long)A * nb + j] = v;
+  }
+}
+
+// AO values at npts points; kpt NULL: real, else complex (interleaved).  The
+// tables go to the device in one copy.  k_ao_cell where the images are those
+// of a box and the basis fits its registers (every basis of the package up to
+// 16 AOs an atom); the image sums otherwise.
+static void ao_points(int n_atoms, int nb, int nprim, const double *alpha, const double *coef, const int *ao_l,
+                      const int *ao_cart, int nlat, const double *lat, const double *kpt, const double *xp,
+                      long long npts, int pts_per_group, const double *xe, double *out, cudaStream_t st) {
+  int tm = 0;
+  double a = 0;
+  const bool cell = nb <= kPtMaxAo && box_images(nlat, lat, &tm, &a);
+  const size_t nc = (size_t)nb * nprim;
+  std::vector<double> h((cell ? kExpTable : 0) + nprim + nc + (cell ? (kpt ? 6 * nlat : 0) : nlat) + nb);
+  double *w = h.data();
+  if (cell) {
+    exp_table(w);
+    w += kExpTable;
+  }
+  w = std::copy(alpha, alpha + nprim, w);
+  w = std::copy(coef, coef + nc, w);
+  if (!cell) w = std::copy(lat, lat + nlat, w);
+  else if (kpt)
+    for (int d = 0; d < 3; ++d)
+      for (int t = 0; t < nlat; ++t) {
+        *w++ = std::cos(kpt[d] * lat[t]);
+        *w++ = std::sin(kpt[d] * lat[t]);
+      }
+  int *hl = reinterpret_cast<int *>(w);  // 2 nb ints in the last nb doubles
+  std::copy(ao_l, ao_l + nb, hl);
+  std::copy(ao_cart, ao_cart + nb, hl + nb);
+  StreamBuf blk(h.size() * sizeof(double), st);
+  double *d = blk.as<double>();
+  const int *dl = reinterpret_cast<const int *>(d + (h.size() - nb));
+  HQ_CUDA(cudaMemcpyAsync(d, h.data(), h.size() * sizeof(double), cudaMemcpyHostToDevice, st));
+  const int grid = ceil_div(npts * n_atoms, 128);
+  if (cell) {
+    auto go = [&](auto kernel, auto *o) {
+      kernel<<<grid, 128, 0, st>>>(n_atoms, nb, nprim, tm, a, d, dl, dl + nb, xp, npts, pts_per_group, xe, o);
+    };
+    double2 *z = reinterpret_cast<double2 *>(out);
+    if (kpt) {
+      if (nb <= 1) go(k_ao_cell<1, double2>, z);
+      else if (nb <= 2) go(k_ao_cell<2, double2>, z);
+      else if (nb <= 5) go(k_ao_cell<5, double2>, z);
+      else go(k_ao_cell<kPtMaxAo, double2>, z);
+    } else {
+      if (nb <= 1) go(k_ao_cell<1, double>, out);
+      else if (nb <= 2) go(k_ao_cell<2, double>, out);
+      else if (nb <= 5) go(k_ao_cell<5, double>, out);
+      else go(k_ao_cell<kPtMaxAo, double>, out);
+    }
+  } else if (kpt) {
+    k_ao_points_kpt<<<grid, 128, 0, st>>>(n_atoms, nb, nprim, d, d + nprim, dl, dl + nb, nlat, d + nprim + nc, kpt[0],
+                                          kpt[1], kpt[2], xp, npts, pts_per_group, xe,
+                                          reinterpret_cast<double2 *>(out));
+  } else {
+    k_ao_points<<<grid, 128, 0, st>>>(n_atoms, nb, nprim, d, d + nprim, dl, dl + nb, nlat, d + nprim + nc, xp, npts,
+                                      pts_per_group, xe, out);
+  }
+  HQ_LAUNCH_CHECK();
+  // before the tables are freed: memory freed ahead of a synchronisation goes
+  // back to the system there, and allocating it again costs 90 us a call
+  HQ_CUDA(cudaStreamSynchronize(st));
+}
+
 }  // namespace hqcgb
 
 // C ABI: AO values of n_atoms protons at npts points.  Basis tables as in
@@ -76,28 +325,15 @@ extern "C" int hqcgb_ao_points(int n_atoms, int nao_atom, int n_prim, const doub
       HQ_REQUIRE((ao_l[k] == 0 || ao_l[k] == 1) && ao_cart[k] >= 0 && ao_cart[k] < 3,
                  "only s and p AOs are supported");
     if (npts == 0) return HQCGB_OK;
-    const size_t nd = (size_t)n_prim + (size_t)nao_atom * n_prim + n_lat1d, ni = 2 * (size_t)nao_atom;
-    StreamBuf blk(nd * sizeof(double) + ni * sizeof(int), st);
-    double *d = blk.as<double>();
-    int *iv = reinterpret_cast<int *>(d + nd);
-    HQ_CUDA(cudaMemcpyAsync(d, alpha, n_prim * sizeof(double), cudaMemcpyHostToDevice, st));
-    HQ_CUDA(cudaMemcpyAsync(d + n_prim, coef, (size_t)nao_atom * n_prim * sizeof(double),
-                            cudaMemcpyHostToDevice, st));
-    HQ_CUDA(cudaMemcpyAsync(d + n_prim + (size_t)nao_atom * n_prim, lat1d, n_lat1d * sizeof(double),
-                            cudaMemcpyHostToDevice, st));
-    HQ_CUDA(cudaMemcpyAsync(iv, ao_l, nao_atom * sizeof(int), cudaMemcpyHostToDevice, st));
-    HQ_CUDA(cudaMemcpyAsync(iv + nao_atom, ao_cart, nao_atom * sizeof(int), cudaMemcpyHostToDevice, st));
-    const long long total = npts * n_atoms;
-    k_ao_points<<<ceil_div(total, 128), 128, 0, st>>>(n_atoms, nao_atom, n_prim, d, d + n_prim, iv,
-                                                      iv + nao_atom, n_lat1d,
-                                                      d + n_prim + (size_t)nao_atom * n_prim, xp, npts,
-                                                      pts_per_group, xe, out);
-    HQ_LAUNCH_CHECK();
-    HQ_CUDA(cudaStreamSynchronize(st));
+    ao_points(n_atoms, nao_atom, n_prim, alpha, coef, ao_l, ao_cart, n_lat1d, lat1d, nullptr, xp, npts, pts_per_group,
+              xe, out, st);
     return HQCGB_OK;
   } catch (const Error &e) {
     set_error(e.msg);
     return e.status;
+  } catch (const std::exception &e) {  // host memory
+    set_error(e.what());
+    return HQCGB_CUDA_ERROR;
   }
 }
 
@@ -155,56 +391,13 @@ extern "C" int hqcgb_slater(int n, int nao_atom, int n_prim, const double *alpha
   } catch (const Error &e) {
     set_error(e.msg);
     return e.status;
+  } catch (const std::exception &e) {  // host memory
+    set_error(e.what());
+    return HQCGB_CUDA_ERROR;
   }
 }
 
 namespace hqcgb {
-
-// k-point AO values (complex): one thread per (point, atom), out[pt][A * nb + j].
-__global__ void k_ao_points_kpt(int n_atoms, int nb, int nprim, const double *__restrict__ alpha,
-                                const double *__restrict__ coef, const int *__restrict__ ao_l,
-                                const int *__restrict__ ao_cart, int nlat,
-                                const double *__restrict__ lat, double k0, double k1, double k2,
-                                const double *__restrict__ xp, long long npts, int pts_per_group,
-                                const double *__restrict__ xe, double2 *__restrict__ out) {
-  const long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (idx >= npts * n_atoms) return;
-  const int A = (int)(idx % n_atoms);
-  const long long pt = idx / n_atoms;
-  const long long grp = pt / pts_per_group;
-  const double *xa = xp + (grp * n_atoms + A) * 3;
-  const double *r = xe + pt * 3;
-  const double kk[3] = {k0, k1, k2};
-  double2 f[3][kPtMaxPrim][2];
-  for (int d = 0; d < 3; ++d) {
-    const double x = r[d] - xa[d];
-    for (int a = 0; a < nprim; ++a) f[d][a][0] = f[d][a][1] = make_double2(0.0, 0.0);
-    for (int t = 0; t < nlat; ++t) {
-      const double u = x - lat[t];
-      double sn, cs;
-      sincos(kk[d] * lat[t], &sn, &cs);
-      for (int a = 0; a < nprim; ++a) {
-        const double g = exp(-alpha[a] * u * u);
-        f[d][a][0].x += g * cs;
-        f[d][a][0].y += g * sn;
-        f[d][a][1].x += u * g * cs;
-        f[d][a][1].y += u * g * sn;
-      }
-    }
-  }
-  const long long nao = (long long)n_atoms * nb;
-  for (int j = 0; j < nb; ++j) {
-    const int l = ao_l[j], ca = ao_cart[j];
-    const int px = (l == 1 && ca == 0), py = (l == 1 && ca == 1), pz = (l == 1 && ca == 2);
-    double2 v = make_double2(0.0, 0.0);
-    for (int a = 0; a < nprim; ++a) {
-      const double2 t = zmul(zmul(f[0][a][px], f[1][a][py]), f[2][a][pz]);
-      v.x += coef[j * nprim + a] * t.x;
-      v.y += coef[j * nprim + a] * t.y;
-    }
-    out[pt * nao + (long long)A * nb + j] = v;
-  }
-}
 
 __global__ void k_gather_cols_z(const double2 *__restrict__ mo, int nao, int nmo,
                                 const int *__restrict__ idx, int m, double2 *__restrict__ M) {
@@ -234,28 +427,15 @@ extern "C" int hqcgb_ao_points_kpt(int n_atoms, int nao_atom, int n_prim, const 
       HQ_REQUIRE((ao_l[k] == 0 || ao_l[k] == 1) && ao_cart[k] >= 0 && ao_cart[k] < 3,
                  "only s and p AOs are supported");
     if (npts == 0) return HQCGB_OK;
-    const size_t nd = (size_t)n_prim + (size_t)nao_atom * n_prim + n_lat1d, ni = 2 * (size_t)nao_atom;
-    StreamBuf blk(nd * sizeof(double) + ni * sizeof(int), st);
-    double *d = blk.as<double>();
-    int *iv = reinterpret_cast<int *>(d + nd);
-    HQ_CUDA(cudaMemcpyAsync(d, alpha, n_prim * sizeof(double), cudaMemcpyHostToDevice, st));
-    HQ_CUDA(cudaMemcpyAsync(d + n_prim, coef, (size_t)nao_atom * n_prim * sizeof(double),
-                            cudaMemcpyHostToDevice, st));
-    HQ_CUDA(cudaMemcpyAsync(d + n_prim + (size_t)nao_atom * n_prim, lat1d, n_lat1d * sizeof(double),
-                            cudaMemcpyHostToDevice, st));
-    HQ_CUDA(cudaMemcpyAsync(iv, ao_l, nao_atom * sizeof(int), cudaMemcpyHostToDevice, st));
-    HQ_CUDA(cudaMemcpyAsync(iv + nao_atom, ao_cart, nao_atom * sizeof(int), cudaMemcpyHostToDevice, st));
-    const long long total = npts * n_atoms;
-    k_ao_points_kpt<<<ceil_div(total, 128), 128, 0, st>>>(
-        n_atoms, nao_atom, n_prim, d, d + n_prim, iv, iv + nao_atom, n_lat1d,
-        d + n_prim + (size_t)nao_atom * n_prim, kpt[0], kpt[1], kpt[2], xp, npts, pts_per_group, xe,
-        reinterpret_cast<double2 *>(out));
-    HQ_LAUNCH_CHECK();
-    HQ_CUDA(cudaStreamSynchronize(st));
+    ao_points(n_atoms, nao_atom, n_prim, alpha, coef, ao_l, ao_cart, n_lat1d, lat1d, kpt, xp, npts, pts_per_group, xe,
+              out, st);
     return HQCGB_OK;
   } catch (const Error &e) {
     set_error(e.msg);
     return e.status;
+  } catch (const std::exception &e) {  // host memory
+    set_error(e.what());
+    return HQCGB_CUDA_ERROR;
   }
 }
 
@@ -301,5 +481,8 @@ extern "C" int hqcgb_slater_kpt(int n, int nao_atom, int n_prim, const double *a
   } catch (const Error &e) {
     set_error(e.msg);
     return e.status;
+  } catch (const std::exception &e) {  // host memory
+    set_error(e.what());
+    return HQCGB_CUDA_ERROR;
   }
 }
