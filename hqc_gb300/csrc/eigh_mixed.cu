@@ -356,12 +356,20 @@ constexpr double kOaFinalUpdate = 1e-7;
 // (error of order 1e-8).
 constexpr double kOaConvergedLoose = 1e-9;
 constexpr double kOaFinalUpdateLoose = 1e-4;
+// Tight mode (the FP64 path): never without an update, and the last one below
+// 1e-9, whose square is under FP64 rounding.
+constexpr double kOaConvergedTight = 0.0;
+constexpr double kOaFinalUpdateTight = 1e-9;
+static double oa_converged(EigLevel l) {
+  return l == EigLevel::Loose ? kOaConvergedLoose : l == EigLevel::Full ? kOaConverged : kOaConvergedTight;
+}
 static double oa_iteration(int n, const double *A, double *X, double *w, MixedEigWork &ws,
                            cudaStream_t st, int max_cluster = kMaxClusterFock,
-                           bool *final_update = nullptr, bool loose = false) {
+                           bool *final_update = nullptr, EigLevel level = EigLevel::Full) {
   if (final_update) *final_update = false;
-  const double conv = loose ? kOaConvergedLoose : kOaConverged;
-  const double fin_thr = loose ? kOaFinalUpdateLoose : kOaFinalUpdate;
+  const double conv = oa_converged(level);
+  const double fin_thr = level == EigLevel::Loose ? kOaFinalUpdateLoose
+                         : level == EigLevel::Full ? kOaFinalUpdate : kOaFinalUpdateTight;
   const long long nn = (long long)n * n;
   const int grid = (int)std::min<long long>(ceil_div(nn, kOaThreads), 148);
   double *red = ws.emax + 8;  // [0..4] grid reductions
@@ -417,10 +425,10 @@ static double oa_iteration(int n, const double *A, double *X, double *w, MixedEi
 // Full solve: FP32 stage (eigh_f32.cu; the QL solver of eigh_fp64.cu when
 // `wide`), then refinement until the relative
 // off-diagonal norm measured before a step is at rounding level (1e-12).
-// Returns false when the refinement does not get there within 8 steps (the
+// Returns false when the refinement does not get there within its steps (the
 // caller then uses the FP64 solver).
 bool eigh_mixed(int n, const double *A, double *V, double *w, MixedEigWork &ws, cudaStream_t st,
-                bool wide, bool loose) {
+                bool wide, EigLevel level) {
   HQ_STAGE(ST_JACOBI, st);
   long long nn = (long long)n * n;
   k_f64_to_f32<<<ceil_div(nn, 256), 256, 0, st>>>(nn, A, ws.A32);
@@ -454,10 +462,15 @@ bool eigh_mixed(int n, const double *A, double *V, double *w, MixedEigWork &ws, 
   }
   k_f32_to_f64<<<ceil_div(nn, 256), 256, 0, st>>>(nn, ws.V32, V);
   HQ_LAUNCH_CHECK();
-  for (int it = 0; it < 8; ++it) {
+  // a perfect lattice's clusters take the tight level about ten steps; one
+  // step costs a hundredth of the FP64 QL solve it saves
+  const int steps = level == EigLevel::Tight ? 16 : 8;
+  for (int it = 0; it < steps; ++it) {
     bool fin = false;
-    double off = oa_iteration(n, A, V, w, ws, st, wide ? kMaxCluster : kMaxClusterFock, &fin, loose);
-    if (off < (loose ? kOaConvergedLoose : kOaConverged) || fin) {
+    double off = oa_iteration(n, A, V, w, ws, st, wide ? kMaxCluster : kMaxClusterFock, &fin, level);
+    // starting vectors that far out do not come from a separated spectrum
+    if (level == EigLevel::Tight && !wide && it == 0 && !(off < 1e-3)) return false;
+    if (off < oa_converged(level) || fin) {
       sort_eigpairs(n, w, V, ws, st);
       return true;
     }
@@ -471,15 +484,15 @@ bool eigh_mixed(int n, const double *A, double *V, double *w, MixedEigWork &ws, 
 // too far (relative off-diagonal norm above 2e-3) or the iteration stalls; the
 // caller then runs the full solve.
 bool eigh_mixed_warm(int n, const double *A, const double *X0, double *V, double *w,
-                     MixedEigWork &ws, cudaStream_t st, bool loose) {
+                     MixedEigWork &ws, cudaStream_t st, EigLevel level) {
   HQ_STAGE(ST_JACOBI, st);
   HQ_CUDA(cudaMemcpyAsync(V, X0, sizeof(double) * n * n, cudaMemcpyDeviceToDevice, st));
   double prev = 1e300;
   for (int it = 0; it < 8; ++it) {
     bool fin = false;
-    double off = oa_iteration(n, A, V, w, ws, st, kMaxClusterFock, &fin, loose);
+    double off = oa_iteration(n, A, V, w, ws, st, kMaxClusterFock, &fin, level);
     if (!(off < 2e-3)) return false;
-    if (off < (loose ? kOaConvergedLoose : kOaConverged) || fin) {
+    if (off < oa_converged(level) || fin) {
       sort_eigpairs(n, w, V, ws, st);
       return true;
     }

@@ -139,10 +139,13 @@ struct MixedEigWork {
   double *T1, *S, *G, *E, *emax, *wbuf;  // wbuf: 2 n^2 (cluster blocks); emax: 16
   int *status, *iwork;                    // iwork: 5 n + 1
 };
+// How far the refinement goes: Loose for vectors that only feed the next SCF
+// density of the mixed path, Full to about 1e-12, Tight to FP64 rounding.
+enum class EigLevel { Loose, Full, Tight };
 bool eigh_mixed_warm(int n, const double *A, const double *X0, double *V, double *w,
-                     MixedEigWork &ws, cudaStream_t st, bool loose = false);
+                     MixedEigWork &ws, cudaStream_t st, EigLevel level = EigLevel::Full);
 bool eigh_mixed(int n, const double *A, double *V, double *w, MixedEigWork &ws, cudaStream_t st,
-                bool wide = false, bool loose = false);
+                bool wide = false, EigLevel level = EigLevel::Full);
 
 // fft (FP32 transforms)
 void launch_fft3d_f32(float2 *c, int ng, int batch, const double2 *tw, bool inverse,

@@ -133,6 +133,19 @@ static constexpr double kExxOccFloor = 1e-14;
 static constexpr int kPsiDrain = 2;
 static constexpr int kThinOcc = 64;  // occupied-block GEMMs up to this many orbitals
 
+// Matrices from this size on take the refined FP32 solve on the FP64 path
+// too.  FP64 runs at 1/64 of the FP32 rate here, and the QL sweeps' rotations
+// come from one thread, so the FP64 solver is slow and serial; the refinement
+// (FP64 products over many SMs) ends at the same residual.  Random spectra,
+// FP64 QL against the refined solve: n = 8 0.36 / 0.35 ms, 16 0.87 / 0.40,
+// 64 9.6 / 0.9, 270 157 / 11; ||A V - V w|| / ||A|| 2e-15 / 5e-16 at 64.  The
+// orbitals' max |C^T S C - 1|, QL / refined: H32 dzv 9.7e-12 / 2.0e-12, H14
+// dzvp 1.7e-11 / 2.5e-11, H54 dzvp 6.7e-11 / 4.0e-11, a perfect bcc H16 dzvp
+// 3.8e-9 / 1.5e-10.  FP64 SCFs: H32 dzv LDA 65^3 335 -> 140 ms, H14 dzvp PBE
+// 49^3 with forces 329 -> 117, H54 dzvp LDA 25^3 2464 -> 220, perfect bcc H54
+// 27^3 (the QL fallback's steps) 1666 -> 734.
+static constexpr int kRefinedEigN = 12;
+
 // HQCGB_TRACE=1 prints one line per SCF iteration (energy, error norm) to stderr.
 static bool trace_on() {
   static const bool v = [] {
@@ -199,6 +212,7 @@ struct hqcgb_plan {
   float2 *cbuf32 = nullptr;
   int *tc_err = nullptr;
   MixedEigWork mew{};
+  bool eig_wide = false;       // FP64 path: this geometry's Fock matrices need the FP32 QL sweep
   // exact exchange in the occupied-pair form (exchange.cu); R = double on
   // the FP64 path, float on the mixed path
   bool exx_fused = false;
@@ -362,6 +376,17 @@ static void create(const hqcgb_params *in, hqcgb_plan *p) {
     p->cbuf32 = p->alloc<float2>(N);
     p->tc_err = p->alloc<int>(1);
     HQ_CUDA(cudaMemset(p->tc_err, 0, sizeof(int)));
+    p->c1_prev = p->alloc<double>(nn);
+    p->Yd = p->alloc<double>((size_t)nao * kThinOcc);
+    p->Y2 = p->alloc<double>((size_t)nao * kThinOcc);
+    p->xerr = p->alloc<double>(nn);
+    p->F1d32 = p->alloc<float>((size_t)n * 3 * p->ng * P.n_prim * 6);
+    if (p->orb_forces) {
+      p->psi32 = p->alloc<float>((size_t)(p->gga ? 4 : 1) * tc_psi_max(false) * N);
+      p->Y32 = p->alloc<float>((size_t)nao * tc_psi_max(false));
+    }
+  }
+  if (p->mixed || nao >= kRefinedEigN) {
     p->mew.A32 = p->alloc<float>(nn);
     p->mew.V32 = p->alloc<float>(nn);
     p->mew.w32 = p->alloc<float>(nao);
@@ -375,15 +400,6 @@ static void create(const hqcgb_params *in, hqcgb_plan *p) {
     p->mew.emax = p->alloc<double>(16);
     p->mew.wbuf = p->alloc<double>(2 * nn);
     p->mew.iwork = p->alloc<int>(5 * (size_t)nao + 1);
-    p->c1_prev = p->alloc<double>(nn);
-    p->Yd = p->alloc<double>((size_t)nao * kThinOcc);
-    p->Y2 = p->alloc<double>((size_t)nao * kThinOcc);
-    p->xerr = p->alloc<double>(nn);
-    p->F1d32 = p->alloc<float>((size_t)n * 3 * p->ng * P.n_prim * 6);
-    if (p->orb_forces) {
-      p->psi32 = p->alloc<float>((size_t)(p->gga ? 4 : 1) * tc_psi_max(false) * N);
-      p->Y32 = p->alloc<float>((size_t)nao * tc_psi_max(false));
-    }
   }
   p->ph = p->alloc<double2>((size_t)n * 3 * p->ng);
   p->ovq = p->alloc<double>(ovl_scratch_doubles(n, P.n_prim));
@@ -488,19 +504,34 @@ static void sync_scalars(Ctx &c) {
   HQ_CUDA(cudaStreamSynchronize(c.st));
 }
 
-// Symmetric eigensolver: Householder + QL (eigh_fp64.cu); the Jacobi solver
-// is kept as the fallback when a QL sweep limit is hit.
+// Symmetric eigensolver: FP32 solve and FP64 Ogita-Aishima refinement (to
+// rounding level on the FP64 path); where that does not converge, Householder
+// + QL (eigh_fp64.cu), and the Jacobi solver when a QL sweep limit is hit.
 static void eigh(Ctx &c, const double *A, double *vecs, double *vals, bool wide = false,
                  bool loose = false) {
   hqcgb_plan *p = c.p;
   int n = p->nao;
   if (p->mixed) {
-    // FP32 solve, then FP64 Ogita-Aishima refinement
-    if (eigh_mixed(n, A, vecs, vals, p->mew, c.st, wide, loose)) {
+    if (eigh_mixed(n, A, vecs, vals, p->mew, c.st, wide, loose ? EigLevel::Loose : EigLevel::Full)) {
       HQ_CUDA(cudaMemsetAsync(p->jstat, 0, sizeof(int), c.st));
       return;
     }
     if (trace_on()) fprintf(stderr, "eigh: mixed solve did not converge, FP64 solve\n");
+  } else if (n >= kRefinedEigN) {
+    axpby(n, 0.5, A, 0.5, A, true, p->jA, c.st);  // exactly symmetric, as the refinement needs
+    // Spectra with large clusters (a perfect lattice's bands) leave the
+    // inverse iteration's vectors too far for the refinement; the FP32 QL
+    // sweep's are near enough, there and in the SCF iterations that follow.
+    bool done = (wide || !p->eig_wide) && eigh_mixed(n, p->jA, vecs, vals, p->mew, c.st, wide, EigLevel::Tight);
+    if (!done && !wide) {
+      p->eig_wide = true;
+      done = eigh_mixed(n, p->jA, vecs, vals, p->mew, c.st, true, EigLevel::Tight);
+    }
+    if (done) {
+      HQ_CUDA(cudaMemsetAsync(p->jstat, 0, sizeof(int), c.st));
+      return;
+    }
+    if (trace_on()) fprintf(stderr, "eigh: refinement did not converge, QL solve\n");
   }
   HQ_CUDA(cudaMemcpyAsync(p->jA, A, sizeof(double) * n * n, cudaMemcpyDeviceToDevice, c.st));
   eigh_tql(n, 1, p->jA, vecs, vals, p->jtmp, p->jstat, c.st);
@@ -528,7 +559,7 @@ static void diagonalize(Ctx &c, const double *Fm) {
   }
   // mixed: refine the previous iteration's eigenvectors when they are close
   bool done = p->mixed && p->have_prev && p->allow_warm &&
-              eigh_mixed_warm(n, p->Fp, p->c1_prev, p->c1, p->w, p->mew, c.st, true);
+              eigh_mixed_warm(n, p->Fp, p->c1_prev, p->c1, p->w, p->mew, c.st, EigLevel::Loose);
   if (!done) eigh(c, p->Fp, p->c1, p->w, false, p->mixed);
   if (p->mixed) {
     HQ_CUDA(cudaMemcpyAsync(p->c1_prev, p->c1, sizeof(double) * n * n, cudaMemcpyDeviceToDevice, c.st));
@@ -543,7 +574,7 @@ static void diagonalize(Ctx &c, const double *Fm) {
 static void refine_last(Ctx &c) {
   hqcgb_plan *p = c.p;
   const int n = p->nao;
-  if (!eigh_mixed_warm(n, p->Fp, p->c1_prev, p->c1, p->w, p->mew, c.st, false))
+  if (!eigh_mixed_warm(n, p->Fp, p->c1_prev, p->c1, p->w, p->mew, c.st))
     eigh(c, p->Fp, p->c1, p->w);
   HQ_CUDA(cudaMemcpyAsync(p->c1_prev, p->c1, sizeof(double) * n * n, cudaMemcpyDeviceToDevice, c.st));
   gemm(false, false, n, n, n, 1.0, p->vorth, n, p->c1, n, nullptr, 0.0, p->C, n, c.st);
@@ -871,6 +902,7 @@ static int scf_one(hqcgb_plan *p, const double *xp_dev, const hqcgb_scf_out *out
   p->have_state = false;
   p->have_prev = false;
   p->allow_warm = false;
+  p->eig_wide = false;
   geometry(c, xp_dev);
   // Hcore guess (solver.py:739-745)
   diagonalize(c, p->H);
