@@ -9,7 +9,11 @@
 //
 // The Ewald energy follows hqc/pbc/potential.py:6-67,103-130 (nearest-image
 // real space, reciprocal sphere |G| <= Gmax, Madelung self term, Rydberg).
+#include <cmath>
+#include <vector>
+
 #include "common.cuh"
+#include "exp_table.cuh"
 #include "kernels.h"
 
 namespace hqcgb {
@@ -40,6 +44,13 @@ __constant__ int kMidx[20][3] = {{0, 0, 0}, {1, 0, 0}, {0, 1, 0}, {0, 0, 1}, {2,
                                  {0, 2, 0}, {0, 0, 2}, {1, 1, 0}, {1, 0, 1}, {0, 1, 1},
                                  {3, 0, 0}, {0, 3, 0}, {0, 0, 3}, {2, 1, 0}, {2, 0, 1},
                                  {1, 2, 0}, {0, 2, 1}, {1, 0, 2}, {0, 1, 2}, {1, 1, 1}};
+// the same as a function, which folds in unrolled loops (registers, no constant loads)
+__device__ constexpr int midx(int q, int d) {
+  const int t[20][3] = {{0, 0, 0}, {1, 0, 0}, {0, 1, 0}, {0, 0, 1}, {2, 0, 0}, {0, 2, 0}, {0, 0, 2},
+                        {1, 1, 0}, {1, 0, 1}, {0, 1, 1}, {3, 0, 0}, {0, 3, 0}, {0, 0, 3}, {2, 1, 0},
+                        {2, 0, 1}, {1, 2, 0}, {0, 2, 1}, {1, 0, 2}, {0, 1, 2}, {1, 1, 1}};
+  return t[q][d];
+}
 constexpr int kNq = 20;  // slots per (i, j, a, b): QS[20], QT[20]
 
 __device__ inline int midx_of(int m0, int m1, int m2) {
@@ -48,6 +59,7 @@ __device__ inline int midx_of(int m0, int m1, int m2) {
   return 0;
 }
 
+// The general form, for any list of lattice vectors.
 // KPT: each lattice term also carries exp(-i k.t) (hqc/pbc/solver.py:257-274);
 // the real and imaginary sums are stored side by side, Q[(i,j,a,b)][4][kNq] =
 // {QS re, QT re, QS im, QT im}.
@@ -120,6 +132,195 @@ __global__ void k_ovl_lattice(const double *__restrict__ xp, int n, int nprim,
       out[3 * kNq + k] = qti[k];
     }
   }
+}
+
+// The lattice sums where the lattice is a sphere (or any set symmetric in
+// every axis) of a cubic lattice: exp(-mu |R + t|^2) h_m0 h_m1 h_m2 is a product
+// over the axes, so with x_i(t) = exp(-mu (R_x + t)^2) h_i (likewise y, z) and
+// the set's rows |t_z| <= m(t_x, t_y),
+//   sum = sum_{ty} y_j sum_{tx} x_i Zc_k[m(tx, ty)],  Zc_k[m] = sum_{|tz| <= m} z_k(tz):
+// an exponential a translation and axis instead of one a lattice vector, and
+// (KD + 1)(KD + 2) / 2 multiply-adds a row of the sphere instead of the NQ
+// triple products (and their six Laplacian terms) a vector.  One thread per
+// (i <= j; a, b); the pair (j, i; b, a) follows from R -> -R, t -> -t: a sign
+// (-1)^|m| (and the conjugate at a k-point).  Bound by the FP64 pipe; one-warp
+// blocks, so that a few atoms' pairs still spread over the chip.  Measured, S
+// and T of one configuration, vector by vector -> by rows: H54 dzvp (box 8 Bohr)
+// 1.99 -> 0.13 ms, H8 szv (box 4.1 Bohr, 870 vectors) 4.7 -> 0.1 ms.
+template <typename Z> struct OvlZ;
+template <> struct OvlZ<double> {
+  static __device__ double zero() { return 0.0; }
+  static __device__ double phase(double, double) { return 1.0; }
+  static __device__ double conj(double a) { return a; }
+};
+template <> struct OvlZ<double2> {
+  static __device__ double2 zero() { return make_double2(0.0, 0.0); }
+  static __device__ double2 phase(double k, double t) {  // exp(-i k t)
+    double s, c;
+    sincos(-k * t, &s, &c);
+    return make_double2(c, s);
+  }
+  static __device__ double2 conj(double2 a) { return make_double2(a.x, -a.y); }
+};
+__device__ inline double ovl_scale(double s, double z) { return s * z; }
+__device__ inline double2 ovl_scale(double s, double2 z) { return make_double2(s * z.x, s * z.y); }
+__device__ inline void ovl_fma(double a, double b, double &s) { s = fma(a, b, s); }
+__device__ inline void ovl_fma(double2 a, double2 b, double2 &s) {
+  s.x = fma(a.x, b.x, fma(-a.y, b.y, s.x));
+  s.y = fma(a.x, b.y, fma(a.y, b.x, s.y));
+}
+__device__ inline void ovl_add(double a, double &s) { s += a; }
+__device__ inline void ovl_add(double2 a, double2 &s) {
+  s.x += a.x;
+  s.y += a.y;
+}
+
+template <int NQ, typename Z>
+__global__ void __launch_bounds__(32)
+    k_ovl_rows(const double *__restrict__ xp, int n, int nprim, const double *__restrict__ alpha,
+               const __grid_constant__ OvlRows rows, const double *__restrict__ kpt, double *__restrict__ Q) {
+  constexpr bool KPT = sizeof(Z) > sizeof(double);
+  constexpr int KD = NQ == 10 ? 4 : 5;  // Hermite orders 0..KD along an axis
+  using O = OvlZ<Z>;
+  __shared__ double tab[kExpTable];
+  for (int k = threadIdx.x; k < kExpTable; k += 32) tab[k] = exp2(k / 64.0);
+  __syncwarp();
+  const long long idx = (long long)blockIdx.x * 32 + threadIdx.x;
+  const int npair = n * (n + 1) / 2, np2 = nprim * nprim;
+  if (idx >= (long long)npair * np2) return;
+  const int ab = (int)(idx / npair), a = ab / nprim, b = ab % nprim;
+  const int pr = (int)(idx % npair);  // pair i <= j at j (j + 1) / 2 + i
+  int j = (int)((sqrtf(8.f * pr + 1.f) - 1.f) * 0.5f);
+  while (j * (j + 1) / 2 > pr) --j;
+  while ((j + 1) * (j + 2) / 2 <= pr) ++j;
+  const int i = pr - j * (j + 1) / 2;
+  const double asum = alpha[a] + alpha[b], mu = alpha[a] * alpha[b] / asum, s = M_PI / asum;
+  const double K = s * sqrt(s);
+  const int tm = rows.tmax, side = 2 * tm + 1;
+  // h_k(u) exp(-mu u^2), k = 0..KD, with the phase of translation t; false (nothing) below e^-60
+  auto term = [&](double R, double t, double kc, Z *out) {
+    const double u = R + t, arg = mu * u * u;
+    if (arg > 60.0) return false;
+    const double e = exp_neg(-arg, tab), g = -2.0 * mu * u;
+    const Z ph = O::phase(kc, t);
+    double h0 = e, h1 = g * e;
+    out[0] = ovl_scale(h0, ph);
+    out[1] = ovl_scale(h1, ph);
+#pragma unroll
+    for (int k = 1; k < KD; ++k) {
+      const double h2 = g * h1 - 2.0 * k * mu * h0;
+      out[k + 1] = ovl_scale(h2, ph);
+      h0 = h1;
+      h1 = h2;
+    }
+    return true;
+  };
+  double R[3], kc[3] = {0, 0, 0};
+  for (int d = 0; d < 3; ++d) {
+    R[d] = xp[i * 3 + d] - xp[j * 3 + d];
+    if (KPT) kc[d] = kpt[d];
+  }
+  Z X[2 * kOvlMaxT + 1][KD + 1], Zc[kOvlMaxT + 1][KD + 1], y[KD + 1], acc[KD + 1];
+  int lo = side, hi = -1;  // the x translations that count
+  for (int t = 0; t < side; ++t)
+    if (term(R[0], (t - tm) * rows.a, kc[0], X[t])) {
+      lo = min(lo, t);
+      hi = t;
+    }
+#pragma unroll
+  for (int k = 0; k <= KD; ++k) acc[k] = O::zero();
+  for (int m = 0; m <= tm; ++m) {
+    for (int sg = m == 0 ? 1 : -1; sg <= 1; sg += 2)
+      if (term(R[2], sg * (m * rows.a), kc[2], y))
+#pragma unroll
+        for (int k = 0; k <= KD; ++k) ovl_add(y[k], acc[k]);
+#pragma unroll
+    for (int k = 0; k <= KD; ++k) Zc[m][k] = acc[k];
+  }
+  Z qs[NQ], qt[NQ];
+#pragma unroll
+  for (int k = 0; k < NQ; ++k) qs[k] = qt[k] = O::zero();
+  for (int ty = 0; ty < side; ++ty) {
+    if (!term(R[1], (ty - tm) * rows.a, kc[1], y)) continue;
+    Z P[KD + 1][KD + 1];
+#pragma unroll
+    for (int p = 0; p <= KD; ++p)
+#pragma unroll
+      for (int k = 0; k <= KD - p; ++k) P[p][k] = O::zero();
+    for (int tx = lo; tx <= hi; ++tx) {
+      const int m = rows.m[tx * side + ty];
+      if (m < 0) continue;
+#pragma unroll
+      for (int p = 0; p <= KD; ++p)
+#pragma unroll
+        for (int k = 0; k <= KD - p; ++k) ovl_fma(X[tx][p], Zc[m][k], P[p][k]);
+    }
+#pragma unroll
+    for (int q = 0; q < NQ; ++q) {
+      const int m0 = midx(q, 0), m1 = midx(q, 1), m2 = midx(q, 2);
+      ovl_fma(y[m1], P[m0][m2], qs[q]);
+      ovl_fma(y[m1], P[m0 + 2][m2], qt[q]);
+      ovl_fma(y[m1 + 2], P[m0][m2], qt[q]);
+      ovl_fma(y[m1], P[m0][m2 + 2], qt[q]);
+    }
+  }
+  constexpr int W = (KPT ? 4 : 2) * kNq;
+  double *out = Q + (((long long)i * n + j) * np2 + ab) * W;
+  double *mir = Q + (((long long)j * n + i) * np2 + b * nprim + a) * W;
+#pragma unroll
+  for (int q = 0; q < NQ; ++q) {
+    const double sg = (midx(q, 0) + midx(q, 1) + midx(q, 2)) & 1 ? -K : K;
+    const Z vs = ovl_scale(K, qs[q]), vt = ovl_scale(K, qt[q]);
+    const Z ms = ovl_scale(sg, O::conj(qs[q])), mt = ovl_scale(sg, O::conj(qt[q]));
+    if constexpr (KPT) {
+      out[q] = vs.x; out[kNq + q] = vt.x; out[2 * kNq + q] = vs.y; out[3 * kNq + q] = vt.y;
+      if (i != j) { mir[q] = ms.x; mir[kNq + q] = mt.x; mir[2 * kNq + q] = ms.y; mir[3 * kNq + q] = mt.y; }
+    } else {
+      out[q] = vs; out[kNq + q] = vt;
+      if (i != j) { mir[q] = ms; mir[kNq + q] = mt; }
+    }
+  }
+}
+
+OvlRows ovl_rows(const double *lattice, int nlat) {
+  OvlRows r{};
+  r.tmax = -1;
+  double a = 0;
+  for (int k = 0; k < 3 * nlat; ++k) {
+    const double v = std::fabs(lattice[k]);
+    if (!std::isfinite(v)) return r;
+    if (v > 0 && (a == 0 || v < a)) a = v;
+  }
+  if (nlat < 1) return r;
+  if (a == 0) a = 1.0;
+  int tm = 0;
+  for (int k = 0; k < 3 * nlat; ++k) {
+    const double q = lattice[k] / a, z = std::rint(q);
+    if (std::fabs(z) > kOvlMaxT || std::fabs(lattice[k] - z * a) > 4e-16 * std::fabs(lattice[k])) return r;
+    tm = std::max(tm, (int)std::fabs(z));
+  }
+  const int side = 2 * tm + 1;
+  std::vector<int> seen((size_t)side * side * side, 0);
+  for (int k = 0; k < nlat; ++k) {
+    int c[3];
+    for (int d = 0; d < 3; ++d) c[d] = (int)std::rint(lattice[3 * k + d] / a) + tm;
+    if (seen[(c[0] * side + c[1]) * side + c[2]]++) return r;  // a vector twice
+  }
+  for (int x = 0; x < side; ++x)
+    for (int y = 0; y < side; ++y) {
+      const int *col = seen.data() + (x * side + y) * side;
+      int m = -1;
+      while (m < tm && col[tm + m + 1]) ++m;
+      for (int z = 0; z < side; ++z)
+        if (col[z] != (std::abs(z - tm) <= m ? 1 : 0)) return r;  // not |t_z| <= m
+      r.m[x * side + y] = (signed char)m;
+    }
+  for (int x = 0; x < side; ++x)
+    for (int y = 0; y < side; ++y)
+      if (r.m[x * side + y] != r.m[(side - 1 - x) * side + side - 1 - y]) return r;
+  r.a = a;
+  r.tmax = tm;
+  return r;
 }
 
 __global__ void k_ovl_contract(int n, int nb, int nprim, const double *__restrict__ alpha,
@@ -259,12 +460,17 @@ __global__ void k_reduce_pair_grad(const double *__restrict__ gpart, int n, int 
 
 void launch_overlap_kinetic(const double *xp, int n, int nb, int nprim, const double *alpha,
                             const double *coef, const int *ao_l, const int *ao_cart,
-                            const double *lattice, int nlat, double *S, double *T, const double *D,
-                            const double *W, double *gpart, double *grad, double *Q,
+                            const double *lattice, int nlat, const OvlRows &rows, double *S, double *T,
+                            const double *D, const double *W, double *gpart, double *grad, double *Q,
                             cudaStream_t st) {
   HQ_STAGE(ST_OVERLAP, st);
   const long long terms = (long long)n * n * nprim * nprim;
-  if (gpart)
+  const int blocks = ceil_div((long long)(n * (n + 1) / 2) * nprim * nprim, 32);
+  if (rows.tmax >= 0 && gpart)
+    k_ovl_rows<20, double><<<blocks, 32, 0, st>>>(xp, n, nprim, alpha, rows, nullptr, Q);
+  else if (rows.tmax >= 0)
+    k_ovl_rows<10, double><<<blocks, 32, 0, st>>>(xp, n, nprim, alpha, rows, nullptr, Q);
+  else if (gpart)
     k_ovl_lattice<20, false><<<ceil_div(terms, 128), 128, 0, st>>>(xp, n, nprim, alpha, lattice, nlat,
                                                                    nullptr, Q);
   else
@@ -284,12 +490,17 @@ void launch_overlap_kinetic(const double *xp, int n, int nb, int nprim, const do
 // S^k, T^k at k-point kpt (device, 1/Bohr): complex Hermitian, interleaved.
 void launch_overlap_kinetic_kpt(const double *xp, int n, int nb, int nprim, const double *alpha,
                                 const double *coef, const int *ao_l, const int *ao_cart,
-                                const double *lattice, int nlat, const double *kpt, double2 *S,
-                                double2 *T, double *Q, cudaStream_t st, const double2 *D,
+                                const double *lattice, int nlat, const OvlRows &rows, const double *kpt,
+                                double2 *S, double2 *T, double *Q, cudaStream_t st, const double2 *D,
                                 const double2 *W, double *gpart, double *grad) {
   HQ_STAGE(ST_OVERLAP, st);
   const long long terms = (long long)n * n * nprim * nprim;
-  if (gpart)
+  const int blocks = ceil_div((long long)(n * (n + 1) / 2) * nprim * nprim, 32);
+  if (rows.tmax >= 0 && gpart)
+    k_ovl_rows<20, double2><<<blocks, 32, 0, st>>>(xp, n, nprim, alpha, rows, kpt, Q);
+  else if (rows.tmax >= 0)
+    k_ovl_rows<10, double2><<<blocks, 32, 0, st>>>(xp, n, nprim, alpha, rows, kpt, Q);
+  else if (gpart)
     k_ovl_lattice<20, true><<<ceil_div(terms, 128), 128, 0, st>>>(xp, n, nprim, alpha, lattice, nlat,
                                                                   kpt, Q);
   else

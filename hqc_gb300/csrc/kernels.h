@@ -65,9 +65,18 @@ void antisym(int n, const double *X, double *e, cudaStream_t st);
 
 // integrals_fp64.cu
 size_t ovl_scratch_doubles(int n, int nprim);
+// The rows |t_z| <= m[t_x][t_y] of a lattice sphere, t = a * integer (host);
+// tmax < 0 when the vectors are no such set (the sums then run vector by vector).
+constexpr int kOvlMaxT = 16;
+struct OvlRows {
+  double a;
+  int tmax;
+  signed char m[(2 * kOvlMaxT + 1) * (2 * kOvlMaxT + 1)];
+};
+OvlRows ovl_rows(const double *lattice, int nlat);
 void launch_overlap_kinetic(const double *xp, int n, int nb, int nprim, const double *alpha,
                             const double *coef, const int *ao_l, const int *ao_cart,
-                            const double *lattice, int nlat, double *S, double *T, const double *D,
+                            const double *lattice, int nlat, const OvlRows &rows, double *S, double *T, const double *D,
                             const double *W, double *gpart, double *grad, double *Q,
                             cudaStream_t st);
 size_t ewald_work_doubles(int n, int gmax);
@@ -101,8 +110,8 @@ size_t ovl_scratch_doubles_kpt(int n, int nprim);
 // for Hermitian D, W (S and T may then be NULL).
 void launch_overlap_kinetic_kpt(const double *xp, int n, int nb, int nprim, const double *alpha,
                                 const double *coef, const int *ao_l, const int *ao_cart,
-                                const double *lattice, int nlat, const double *kpt, double2 *S,
-                                double2 *T, double *Q, cudaStream_t st, const double2 *D = nullptr,
+                                const double *lattice, int nlat, const OvlRows &rows, const double *kpt,
+                                double2 *S, double2 *T, double *Q, cudaStream_t st, const double2 *D = nullptr,
                                 const double2 *W = nullptr, double *gpart = nullptr,
                                 double *grad = nullptr);
 // forces_kpt.cu

@@ -431,6 +431,7 @@ struct hqcgb_kplan {
   long long N = 0;
   double L = 0, Omega = 0, dV = 0;
   bool gga = false, hf = false, mixed = false;
+  OvlRows ovl_rows{};  // the S/T lattice sphere by rows
   std::vector<void *> allocs;
   // mixed precision: the real embedding X [2n][ld] (FP32), its TF32 pieces
   // (K-blocked), the quadrature operand pieces, the grid-major K-blocked copy
@@ -559,6 +560,7 @@ static void kcreate(const hqcgb_params &P, hqcgb_kplan *p) {
   kupload(p->lat1d, P.lat1d, sizeof(double) * P.n_lat1d);
   p->lattice = p->alloc<double>(3 * (size_t)P.n_lattice);
   kupload(p->lattice, P.lattice, sizeof(double) * 3 * P.n_lattice);
+  p->ovl_rows = ovl_rows(P.lattice, P.n_lattice);
   std::vector<double2> tw(p->ng);
   for (int k = 0; k < p->ng; ++k) {
     const double a = -2.0 * M_PI * k / p->ng;
@@ -946,7 +948,7 @@ static void kgeometry(KCtx &c, const double *xp_dev, const double *kpt_host) {
     }
   }
   launch_overlap_kinetic_kpt(p->xp, p->n, p->nb, p->nprim, p->alpha, p->coef, p->ao_l, p->ao_cart,
-                             p->lattice, P.n_lattice, p->kpt, p->S, p->T, p->ovq, c.st);
+                             p->lattice, P.n_lattice, p->ovl_rows, p->kpt, p->S, p->T, p->ovq, c.st);
   launch_vloc_G(p->xp, p->n, p->ng, p->L, p->ph, p->cbuf, c.st);
   launch_fft3d(p->cbuf, p->ng, 1, p->tw, true, c.st);
   launch_complex_real(p->cbuf, N, 1.0, p->vloc, c.st);
@@ -1165,7 +1167,7 @@ static void kforces(hqcgb_kplan *p, double *grad, cudaStream_t st) {
   HQ_LAUNCH_CHECK();
   zgemm('N', 'C', n, n, n, kOne, p->t1, n, p->C, n, kZero, p->t2, n, st);
   launch_overlap_kinetic_kpt(p->xp, na, p->nb, p->nprim, p->alpha, p->coef, p->ao_l, p->ao_cart, p->lattice,
-                             P.n_lattice, p->kpt, nullptr, nullptr, p->ovq, st, p->D, p->t2, p->gpart, grad);
+                             P.n_lattice, p->ovl_rows, p->kpt, nullptr, nullptr, p->ovq, st, p->D, p->t2, p->gpart, grad);
   // X = D phibar, rho (and grad rho) from it in FP64
   zgemm('N', 'N', n, (int)N, n, kOne, p->D, n, p->phi, (int)N, kZero, p->fX, (int)N, st);
   launch_rho_from_x_kpt(p->phi, p->gga ? p->dphi : nullptr, p->fX, n, N, p->rho, p->gga ? p->grho : nullptr,

@@ -38,16 +38,17 @@ extern "C" int hqcgb_overlap(int n_atoms, int nao_atom, int n_prim, const double
     HQ_CUDA(cudaMemcpyAsync(d_lat, lattice, 3 * (size_t)n_lattice * sizeof(double), cudaMemcpyHostToDevice, st));
     HQ_CUDA(cudaMemcpyAsync(d_l, ao_l, nao_atom * sizeof(int), cudaMemcpyHostToDevice, st));
     HQ_CUDA(cudaMemcpyAsync(d_c, ao_cart, nao_atom * sizeof(int), cudaMemcpyHostToDevice, st));
+    const OvlRows rows = ovl_rows(lattice, n_lattice);
     for (int b = 0; b < n_cfg; ++b) {
       const double *x = xp + (size_t)b * 3 * n_atoms;
       double *Sb = S + (size_t)b * cw * nn, *Tb = T ? T + (size_t)b * cw * nn : d_t;
       if (kp) {
         HQ_CUDA(cudaMemcpyAsync(d_k, kpts + 3 * (size_t)b, 3 * sizeof(double), cudaMemcpyHostToDevice, st));
         launch_overlap_kinetic_kpt(x, n_atoms, nao_atom, n_prim, d_alpha, d_coef, d_l, d_c, d_lat, n_lattice,
-                                   d_k, reinterpret_cast<double2 *>(Sb), reinterpret_cast<double2 *>(Tb),
+                                   rows, d_k, reinterpret_cast<double2 *>(Sb), reinterpret_cast<double2 *>(Tb),
                                    d_q, st);
       } else {
-        launch_overlap_kinetic(x, n_atoms, nao_atom, n_prim, d_alpha, d_coef, d_l, d_c, d_lat, n_lattice, Sb,
+        launch_overlap_kinetic(x, n_atoms, nao_atom, n_prim, d_alpha, d_coef, d_l, d_c, d_lat, n_lattice, rows, Sb,
                                T ? Tb : nullptr, nullptr, nullptr, nullptr, nullptr, d_q, st);
       }
     }
@@ -56,5 +57,8 @@ extern "C" int hqcgb_overlap(int n_atoms, int nao_atom, int n_prim, const double
   } catch (const Error &e) {
     set_error(e.msg);
     return e.status;
+  } catch (const std::exception &e) {  // host memory
+    set_error(e.what());
+    return HQCGB_CUDA_ERROR;
   }
 }

@@ -163,6 +163,7 @@ struct hqcgb_plan {
   long long N = 0;
   double L = 0, Omega = 0, dV = 0;
   bool gga = false, need_dphi = false, hf = false;
+  OvlRows ovl_rows{};          // the S/T lattice sphere by rows
   std::vector<void *> allocs;
 
   // constant tables
@@ -335,6 +336,7 @@ static void create(const hqcgb_params *in, hqcgb_plan *p) {
   upload(p->lattice, P.lattice, sizeof(double) * 3 * P.n_lattice);
   p->lat1d_cap = P.n_lat1d;
   p->lattice_cap = P.n_lattice;
+  p->ovl_rows = ovl_rows(P.lattice, P.n_lattice);
   std::vector<double2> tw(p->ng);
   for (int k = 0; k < p->ng; ++k) {
     double a = -2.0 * M_PI * k / p->ng;
@@ -868,7 +870,7 @@ static void geometry(Ctx &c, const double *xp_dev) {
                              p->dphiT32 + (size_t)d * N * tc_ldk(n), c.st);
   }
   launch_overlap_kinetic(p->xp, p->n, p->nb, p->nprim, p->alpha, p->coef, p->ao_l, p->ao_cart,
-                         p->lattice, P.n_lattice, p->S, p->T, nullptr, nullptr, nullptr, nullptr,
+                         p->lattice, P.n_lattice, p->ovl_rows, p->S, p->T, nullptr, nullptr, nullptr, nullptr,
                          p->ovq, c.st);
   launch_vloc_G(p->xp, p->n, p->ng, p->L, p->ph, p->cbuf, c.st);
   launch_fft3d(p->cbuf, p->ng, 1, p->tw, true, c.st);
@@ -1063,7 +1065,7 @@ static void forces(hqcgb_plan *p, double *grad, cudaStream_t st) {
   launch_axpy_grid(n, n, 1.0, p->occ, p->w, p->psi, st);   // psi = f * eps
   gemm(false, true, n, n, n, 1.0, p->C, n, p->C, n, p->psi, 0.0, p->t2, n, st);
   launch_overlap_kinetic(p->xp, p->n, p->nb, p->nprim, p->alpha, p->coef, p->ao_l, p->ao_cart,
-                         p->lattice, P.n_lattice, nullptr, nullptr, p->D, p->t2, p->gpart, grad,
+                         p->lattice, P.n_lattice, p->ovl_rows, nullptr, nullptr, p->D, p->t2, p->gpart, grad,
                          p->ovq, st);
   if (p->orb_forces) {
     orbital_forces(c, grad);
@@ -1270,6 +1272,7 @@ static void set_box(hqcgb_plan *p, double L, double rcut, cudaStream_t st) {
   }
   HQ_CUDA(cudaMemcpyAsync(p->lat1d, p->h_lat1d.data(), sizeof(double) * n1, cudaMemcpyHostToDevice, st));
   HQ_CUDA(cudaMemcpyAsync(p->lattice, p->h_lattice.data(), sizeof(double) * 3 * n3, cudaMemcpyHostToDevice, st));
+  p->ovl_rows = ovl_rows(p->h_lattice.data(), n3);
   p->P.n_lat1d = n1;
   p->P.n_lattice = n3;
   p->P.L = L;
