@@ -7,8 +7,6 @@
 //    those factors contracted over primitives (hqc/pbc/gto.py:341-369);
 //  * density: rho(g) = sum_p phi_p(g) (D phi)_p(g)  (hqc/pbc/solver.py:690),
 //    plus grad rho for GGA;
-//  * gemm_nt_partial: split-K quadrature  M_pq = sum_g A_p(g) w(g) B_q(g)
-//    (hqc/pbc/solver.py:693, the Vxc/J/Vep contractions);
 //  * pointwise xc / energy kernels.
 //
 // Layouts: grid index g = (ix * n + iy) * n + iz with x_i = i L / n; AO-major
@@ -161,76 +159,6 @@ void launch_density(const double *phi, const double *dphi, const double *D, int 
   HQ_LAUNCH_CHECK();
 }
 
-// Split-K quadrature partials: P[c][p][q] = sum_{g in chunk c} A_p(g) w(g) B_q(g).
-// 32x32 output tile per block (256 threads, 4 outputs each), K staged by 32.
-constexpr int kQuadChunk = 2048;
-
-__global__ void k_gemm_nt_partial(const double *__restrict__ A, const double *__restrict__ B,
-                                  const double *__restrict__ w, int nao, long long N, int sym,
-                                  double *__restrict__ P) {
-  __shared__ double As[32][33];
-  __shared__ double Bs[32][33];
-  int pt = blockIdx.x, qt = blockIdx.y, chunk = blockIdx.z;
-  if (sym && qt < pt) return;
-  int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
-  int p0 = pt * 32, q0 = qt * 32;
-  long long k0 = (long long)chunk * kQuadChunk;
-  long long k1 = k0 + kQuadChunk < N ? k0 + kQuadChunk : N;
-  double acc[4] = {0, 0, 0, 0};
-  for (long long kb = k0; kb < k1; kb += 32) {
-    long long k = kb + tx;
-    bool kin = k < k1;
-    double wk = (w && kin) ? w[k] : 1.0;
-    for (int r = ty; r < 32; r += 8) {
-      int p = p0 + r, q = q0 + r;
-      As[r][tx] = (kin && p < nao) ? A[(long long)p * N + k] * wk : 0.0;
-      Bs[r][tx] = (kin && q < nao) ? B[(long long)q * N + k] : 0.0;
-    }
-    __syncthreads();
-#pragma unroll 8
-    for (int kk = 0; kk < 32; ++kk) {
-      double b = Bs[tx][kk];
-#pragma unroll
-      for (int r = 0; r < 4; ++r) acc[r] += As[ty + 8 * r][kk] * b;
-    }
-    __syncthreads();
-  }
-  for (int r = 0; r < 4; ++r) {
-    int p = p0 + ty + 8 * r, q = q0 + tx;
-    if (p < nao && q < nao) P[((long long)chunk * nao + p) * nao + q] = acc[r];
-  }
-}
-
-// M[p][q] = scale * sum_c P[c][p][q] (+ mirror for the symmetric case).
-__global__ void k_reduce_partials(const double *__restrict__ P, int nchunk, int nao, int sym,
-                                  double scale, int accumulate, double *__restrict__ M) {
-  int idx = blockIdx.x * blockDim.x + threadIdx.x;
-  if (idx >= nao * nao) return;
-  int p = idx / nao, q = idx % nao;
-  int pp = p, qq = q;
-  if (sym && (q / 32) < (p / 32)) { pp = q; qq = p; }
-  double s = 0;
-  for (int c = 0; c < nchunk; ++c) s += P[((long long)c * nao + pp) * nao + qq];
-  s *= scale;
-  M[idx] = accumulate ? M[idx] + s : s;
-}
-
-int quad_chunks(long long N) { return ceil_div(N, kQuadChunk); }
-
-void launch_quadrature(const double *A, const double *B, const double *w, int nao, long long N,
-                       bool sym, double scale, bool accumulate, double *partial, double *M,
-                       cudaStream_t st) {
-  HQ_STAGE(ST_QUAD, st);
-  int nt = ceil_div(nao, 32);
-  int nchunk = quad_chunks(N);
-  dim3 grid(nt, nt, nchunk);
-  k_gemm_nt_partial<<<grid, 256, 0, st>>>(A, B, w, nao, N, sym ? 1 : 0, partial);
-  HQ_LAUNCH_CHECK();
-  k_reduce_partials<<<ceil_div((long long)nao * nao, 256), 256, 0, st>>>(
-      partial, nchunk, nao, sym ? 1 : 0, scale, accumulate ? 1 : 0, M);
-  HQ_LAUNCH_CHECK();
-}
-
 // ---------------------------------------------------------------------------
 // pointwise: exchange-correlation on the grid.
 //   in : rho, grho (GGA), vh (Hartree potential)
@@ -297,26 +225,6 @@ void launch_xc_pointwise(int kind, const double *rho, const double *grho, const 
     k_xc_pointwise<true><<<xc_blocks(N), 256, 0, st>>>(kind, rho, grho, vh, N, dV, w, vxc_out, u, part);
   else
     k_xc_pointwise<false><<<xc_blocks(N), 256, 0, st>>>(kind, rho, grho, vh, N, dV, w, vxc_out, u, part);
-  HQ_LAUNCH_CHECK();
-}
-
-// Z_p(g) = 0.5 w(g) phi_p(g) + dV sum_c u_c(g) dphi_c,p(g)   (GGA Fock operand;
-// M = Z phi^T + phi Z^T reproduces v_rho phi phi + u.(grad phi phi + phi grad phi)).
-__global__ void k_gga_operand(const double *__restrict__ phi, const double *__restrict__ dphi,
-                              const double *__restrict__ w, const double *__restrict__ u,
-                              int nao, long long N, double dV, double *__restrict__ Z) {
-  long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (idx >= (long long)nao * N) return;
-  long long g = idx % N;
-  long long NN = (long long)nao * N;
-  Z[idx] = 0.5 * w[g] * phi[idx] +
-           dV * (u[g] * dphi[idx] + u[N + g] * dphi[NN + idx] + u[2 * N + g] * dphi[2 * NN + idx]);
-}
-
-void launch_gga_operand(const double *phi, const double *dphi, const double *w, const double *u,
-                        int nao, long long N, double dV, double *Z, cudaStream_t st) {
-  HQ_STAGE(ST_XC, st);
-  k_gga_operand<<<ceil_div((long long)nao * N, 256), 256, 0, st>>>(phi, dphi, w, u, nao, N, dV, Z);
   HQ_LAUNCH_CHECK();
 }
 

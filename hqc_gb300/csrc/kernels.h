@@ -12,18 +12,41 @@ void launch_phi(const double *F, const double *coef, const int *ao_l, const int 
                 cudaStream_t st);
 void launch_density(const double *phi, const double *dphi, const double *D, int nao, long long N,
                     double *rho, double *grho, double *Xout, cudaStream_t st);
-int quad_chunks(long long N);
-void launch_quadrature(const double *A, const double *B, const double *w, int nao, long long N,
-                       bool sym, double scale, bool accumulate, double *partial, double *M,
-                       cudaStream_t st);
 int xc_blocks(long long N);
 void launch_xc_pointwise(int kind, const double *rho, const double *grho, const double *vh,
                          long long N, double dV, double *w, double *vxc_out, double *u,
                          double *part, cudaStream_t st, bool fp32 = false);
-void launch_gga_operand(const double *phi, const double *dphi, const double *w, const double *u,
-                        int nao, long long N, double dV, double *Z, cudaStream_t st);
 void launch_sum_partials(const double *part, int nblk, int stride, int nout, double scale,
                          double *out, bool accumulate, cudaStream_t st);
+
+// quad_f64.cu: FP64 quadratures on the tensor cores (digits of 7 bits).
+// Workspace of one plan: digits, exponents and scales of the weighted operand
+// (A), of the AOs (B) and, for a second operand of quad64_pair, X; the tables
+// of block maxima of the AOs and their gradients, of the weights, and of other
+// operands; FP64 partial tiles; the tensor-core error word.
+struct Quad64 {
+  int n = 0;
+  char *A = nullptr, *B = nullptr, *X = nullptr;
+  int *eA = nullptr, *eB = nullptr, *eX = nullptr, *err = nullptr;
+  double *sA = nullptr, *sB = nullptr, *sX = nullptr, *part = nullptr;
+  float *tab = nullptr, *wtab = nullptr, *xtab = nullptr;
+};
+size_t quad64_operand_bytes(int n, long long N);
+long long quad64_table(long long N);  // entries of a maxima table's row
+size_t quad64_partial_doubles(int n);
+// AOs (and gradients) of a geometry: maxima, exponents and digits (B)
+void quad64_basis(const Quad64 &q, const double *phi, const double *dphi, long long N, cudaStream_t st);
+// M = scale sum_g phi_p w phi_q (w NULL: 1), both after quad64_basis
+void quad64_weighted(const Quad64 &q, const double *phi, const double *w, long long N, double scale, double *M,
+                     cudaStream_t st);
+// M = Z phi^T + phi Z^T, Z = 0.5 w phi + dV u . dphi (after quad64_basis with dphi)
+void quad64_gga(const Quad64 &q, const double *phi, const double *dphi, const double *w, const double *u, double dV,
+                long long N, double *M, cudaStream_t st);
+// M (+)= Q Q^T
+void quad64_gram(const Quad64 &q, const double *Q, long long N, bool accumulate, double *M, cudaStream_t st);
+// M (+)= scale sum_g phi_p w Y_q (after quad64_basis)
+void quad64_pair(const Quad64 &q, const double *phi, const double *w, const double *Y, long long N, double scale,
+                 bool accumulate, double *M, cudaStream_t st);
 
 // fft_fp64.cu
 void launch_fft3d(double2 *c, int ng, int batch, const double2 *tw, bool inverse, cudaStream_t st);

@@ -187,7 +187,7 @@ struct hqcgb_plan {
          *DPsi = nullptr, *W = nullptr, *psi = nullptr;
   double2 *cbuf = nullptr;
   long long cbuf_batch = 0;
-  double *qpart = nullptr, *xpart = nullptr, *fpart = nullptr, *gpart = nullptr, *vpart = nullptr;
+  double *xpart = nullptr, *fpart = nullptr, *gpart = nullptr, *vpart = nullptr;
   // mixed-precision grid data (row stride ld floats)
   bool mixed = false;
   long long ld = 0;
@@ -212,6 +212,7 @@ struct hqcgb_plan {
   double *tcq_part = nullptr, *tcd_part = nullptr;
   float2 *cbuf32 = nullptr;
   int *tc_err = nullptr;
+  Quad64 q64{};                // FP64 quadratures
   MixedEigWork mew{};
   bool eig_wide = false;       // FP64 path: this geometry's Fock matrices need the FP32 QL sweep
   // exact exchange in the occupied-pair form (exchange.cu); R = double on
@@ -428,14 +429,13 @@ static void create(const hqcgb_params *in, hqcgb_plan *p) {
   if (p->gga) {
     p->grho = p->alloc<double>(3 * N);
     p->u = p->alloc<double>(3 * N);
-    if (!p->mixed || fp64_forces) p->Z = p->alloc<double>((size_t)nao * N);
+    if (fp64_forces) p->Z = p->alloc<double>((size_t)nao * N);
   }
   if (fp64_forces || p->hf) {
     p->X = p->alloc<double>((size_t)nao * N);
     if (!p->Z) p->Z = p->alloc<double>((size_t)nao * N);
   }
   if (fp64_forces && p->gga) p->DPsi = p->alloc<double>((size_t)nao * N);
-  long long qcols = N;
   p->exx_fused = p->hf && exx_fused_supported(p->ng, P.n_prim, !p->mixed);
   if (p->exx_fused) {
     // orbitals per group: T and Q within about 1.5 GB
@@ -470,7 +470,6 @@ static void create(const hqcgb_params *in, hqcgb_plan *p) {
     } else {
       p->exx_ldq = gK;
       p->exx_Q = p->alloc<double>((size_t)nao * gK);
-      qcols = std::max(qcols, gK);
       launch_exx_weights<double>(p->ng, p->L, p->dV, (double *)wsq, 0);
     }
     p->exx = ExxGeom{p->ng, nao, p->nb, p->nprim, p->tw, p->coef, p->ao_l, p->ao_cart, wsq};
@@ -481,7 +480,28 @@ static void create(const hqcgb_params *in, hqcgb_plan *p) {
   p->cbuf_batch = (p->hf && !p->exx_fused) ? nao : 1;
   if (p->hf && !p->exx_fused) p->W = p->alloc<double>((size_t)nao * N);
   p->cbuf = p->alloc<double2>((size_t)p->cbuf_batch * N);
-  if (!p->mixed || p->hf) p->qpart = p->alloc<double>((size_t)quad_chunks(qcols) * nn);
+  if (!p->mixed || p->hf) {
+    // FP64 quadratures: Fock, V, S~ and the Gram matrix of the FP64 exchange
+    const long long gK = p->exx_fused && !p->mixed ? (long long)p->exx_g * exx_pair_len(p->ng) : 0;
+    const long long most = std::max(N, gK), tabN = quad64_table(N);
+    const bool legacy = p->hf && !p->exx_fused;
+    Quad64 &q = p->q64;
+    q.n = nao;
+    q.B = p->alloc<char>(quad64_operand_bytes(nao, N));
+    if (!p->mixed || legacy) q.A = p->alloc<char>(quad64_operand_bytes(nao, most));
+    if (legacy) q.X = p->alloc<char>(quad64_operand_bytes(nao, N));
+    for (int **e : {&q.eA, &q.eB, &q.eX}) *e = p->alloc<int>(nao);
+    for (double **sc : {&q.sA, &q.sB, &q.sX}) *sc = p->alloc<double>(nao);
+    q.tab = p->alloc<float>((size_t)(p->gga && !p->mixed ? 4 : 1) * nao * tabN);
+    q.wtab = p->alloc<float>(4 * tabN);
+    if (p->hf) q.xtab = p->alloc<float>((size_t)nao * quad64_table(most));
+    q.part = p->alloc<double>(quad64_partial_doubles(nao));
+    if (!p->tc_err) {
+      p->tc_err = p->alloc<int>(1);
+      HQ_CUDA(cudaMemset(p->tc_err, 0, sizeof(int)));
+    }
+    q.err = p->tc_err;
+  }
   p->xpart = p->alloc<double>((size_t)2 * xc_blocks(N));
   if (P.want_forces) {
     p->fpart = p->alloc<double>(std::max((size_t)nao * force_grid_blocks(N) * 3,
@@ -690,7 +710,7 @@ static void exchange(Ctx &c) {
                                p->exx_T, c.st);
       launch_exx_column_q<double>(p->exx, p->exx_T, g, p->exx_Q, NK, false, c.st);
       const double *Q = static_cast<const double *>(p->exx_Q);
-      launch_quadrature(Q, Q, nullptr, n, NK, true, 1.0, true, p->qpart, p->K, c.st);
+      quad64_gram(p->q64, Q, NK, true, p->K, c.st);
     }
   }
   exchange_madelung(c);
@@ -714,7 +734,7 @@ static void exchange_legacy(Ctx &c, double *Zacc) {
     launch_scale_complex(p->cbuf, p->coul, N, n, c.st);
     launch_fft3d(p->cbuf, p->ng, n, p->tw, true, c.st);
     launch_complex_real(p->cbuf, (long long)n * N, 1.0, p->W, c.st);
-    launch_quadrature(p->phi, p->W, p->psi, n, N, false, f * p->dV, true, p->qpart, p->K, c.st);
+    quad64_pair(p->q64, p->phi, p->psi, p->W, N, f * p->dV, true, p->K, c.st);
     if (Zacc) {
       launch_density(p->W, nullptr, p->D, n, N, p->vh /*scratch*/, nullptr, p->X, c.st);
       launch_axpy_grid((long long)n * N, N, f, p->psi, p->X, Zacc, c.st);
@@ -798,11 +818,9 @@ static double fock(Ctx &c) {
                       p->gga ? p->u : nullptr, p->xpart, c.st);
   launch_sum_partials(p->xpart, xc_blocks(N), 2, 2, 1.0, p->scal + S_EXC, false, c.st);
   if (p->gga) {
-    launch_gga_operand(p->phi, p->dphi, p->wq, p->u, n, N, p->dV, p->Z, c.st);
-    launch_quadrature(p->Z, p->phi, nullptr, n, N, false, 1.0, false, p->qpart, p->t1, c.st);
-    axpby(n, 1.0, p->t1, 1.0, p->t1, true, p->F2e, c.st);
+    quad64_gga(p->q64, p->phi, p->dphi, p->wq, p->u, p->dV, N, p->F2e, c.st);
   } else {
-    launch_quadrature(p->phi, p->phi, p->wq, n, N, true, 1.0, false, p->qpart, p->F2e, c.st);
+    quad64_weighted(p->q64, p->phi, p->wq, N, 1.0, p->F2e, c.st);
   }
   }
   if (p->hf) {
@@ -857,6 +875,7 @@ static void geometry(Ctx &c, const double *xp_dev) {
   if (p->phi)
     launch_phi(p->F1d, p->coef, p->ao_l, p->ao_cart, p->nb, p->nprim, n, p->ng, p->phi, p->dphi,
                c.st);
+  if (p->q64.n) quad64_basis(p->q64, p->phi, p->gga && !p->mixed ? p->dphi : nullptr, N, c.st);
   if (p->mixed) {
     launch_to_float((long long)p->n * 3 * p->ng * P.n_prim * 6, p->F1d, p->F1d32, c.st);
     launch_phi32(p->F1d32, p->coef, p->ao_l, p->ao_cart, p->nb, p->nprim, n, p->ng, p->ld, p->phi32,
@@ -881,10 +900,10 @@ static void geometry(Ctx &c, const double *xp_dev) {
     launch_tc_quadrature(p->phi32, nullptr, p->phihl, p->w32, nullptr, (float)p->dV, n, N, p->ld, false,
                          1.0, p->tcq_part, p->V, p->tc_err, c.st, 1, p->zhl);
   } else {
-    launch_quadrature(p->phi, p->phi, p->vloc, n, N, true, p->dV, false, p->qpart, p->V, c.st);
+    quad64_weighted(p->q64, p->phi, p->vloc, N, p->dV, p->V, c.st);
   }
   axpby(n, 1.0, p->T, 1.0, p->V, false, p->H, c.st);
-  if (p->hf) launch_quadrature(p->phi, p->phi, nullptr, n, N, true, p->dV, false, p->qpart, p->St, c.st);
+  if (p->hf) quad64_weighted(p->q64, p->phi, nullptr, N, p->dV, p->St, c.st);
   // S^{-1/2} as U w^{-1/2} (solver.py:729-730)
   HQ_CUDA(cudaMemsetAsync(p->ibad, 0, sizeof(int), c.st));
   eigh(c, p->S, p->c1, p->ws, true);
@@ -982,7 +1001,7 @@ static int scf_one(hqcgb_plan *p, const double *xp_dev, const hqcgb_scf_out *out
     stopped = loop != P.max_cycle;
   }
   check_eig(c);
-  if (p->mixed) {
+  if (p->tc_err) {
     int te = 0;
     HQ_CUDA(cudaMemcpyAsync(&te, p->tc_err, sizeof(int), cudaMemcpyDeviceToHost, st));
     HQ_CUDA(cudaStreamSynchronize(st));
