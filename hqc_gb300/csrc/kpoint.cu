@@ -948,7 +948,7 @@ static void kgeometry(KCtx &c, const double *xp_dev, const double *kpt_host) {
     }
   }
   launch_overlap_kinetic_kpt(p->xp, p->n, p->nb, p->nprim, p->alpha, p->coef, p->ao_l, p->ao_cart,
-                             p->lattice, P.n_lattice, p->ovl_rows, p->kpt, p->S, p->T, p->ovq, c.st);
+                             p->lattice, P.n_lattice, OvlRows{0.0, -1, {}}, p->kpt, p->S, p->T, p->ovq, c.st);
   launch_vloc_G(p->xp, p->n, p->ng, p->L, p->ph, p->cbuf, c.st);
   launch_fft3d(p->cbuf, p->ng, 1, p->tw, true, c.st);
   launch_complex_real(p->cbuf, N, 1.0, p->vloc, c.st);

@@ -888,9 +888,12 @@ static void geometry(Ctx &c, const double *xp_dev) {
         launch_transpose_phi(p->dphi32 + (size_t)d * n * p->ld, n, N, p->ld,
                              p->dphiT32 + (size_t)d * N * tc_ldk(n), c.st);
   }
+  // The SCF's S and T keep the sums vector by vector: a nearly dependent basis
+  // multiplies a change in the last digit of S by cond(S), 1e7 for dzvp in a
+  // dense box, in the density matrix.  The gradient takes the rows.
   launch_overlap_kinetic(p->xp, p->n, p->nb, p->nprim, p->alpha, p->coef, p->ao_l, p->ao_cart,
-                         p->lattice, P.n_lattice, p->ovl_rows, p->S, p->T, nullptr, nullptr, nullptr, nullptr,
-                         p->ovq, c.st);
+                         p->lattice, P.n_lattice, OvlRows{0.0, -1, {}}, p->S, p->T, nullptr, nullptr,
+                         nullptr, nullptr, p->ovq, c.st);
   launch_vloc_G(p->xp, p->n, p->ng, p->L, p->ph, p->cbuf, c.st);
   launch_fft3d(p->cbuf, p->ng, 1, p->tw, true, c.st);
   launch_complex_real(p->cbuf, N, 1.0, p->vloc, c.st);

@@ -25,8 +25,10 @@
 // destination tile, a copy thread, an MMA thread and eight drain warps.
 //
 // Bounds.  One 32-point stage is 72 MMAs of 128 x 64 x 16: the kernel is bound
-// by the tensor pipe, at 36 products a term.  Measured, weights, digits and
-// sums included: @QF@.
+// by the tensor pipe, at 36 products a term.  Measured, digits
+// of the weighted operand and sums included, FP64 pipe -> this: 64 AOs and 65^3
+// points 2.24 -> 0.24 ms, 70 AOs and 49^3 points with the gradient term 2.21 ->
+// 0.31 ms, 8 AOs and 41^3 points 0.57 -> 0.12 ms.
 #include <algorithm>
 #include <cmath>
 
