@@ -48,6 +48,24 @@ void quad64_gram(const Quad64 &q, const double *Q, long long N, bool accumulate,
 void quad64_pair(const Quad64 &q, const double *phi, const double *w, const double *Y, long long N, double scale,
                  bool accumulate, double *M, cudaStream_t st);
 
+// density_f64.cu: FP64 density from the orbitals on the tensor cores, up to
+// density64_max_ao() AOs.  A: digits of phi^T (and of the gradient's fields),
+// sA [fields][N], e [N] scratch; B, eY: digits and exponents of Y^T.
+struct Density64 {
+  int n = 0;
+  char *A = nullptr, *B = nullptr;
+  double *sA = nullptr;
+  int *e = nullptr, *eY = nullptr, *err = nullptr;
+};
+int density64_max_ao();
+size_t density64_field_bytes(int nao, long long N);
+size_t density64_orbital_bytes(int nao);
+void density64_basis(const Density64 &d, const double *phi, const double *dphi, long long N, cudaStream_t st);
+// rho (and grad rho) of the first nuse orbitals (nuse >= 1); psi not null:
+// sqrt(f_k) psi_k into psi [nuse][N]
+void density64(const Density64 &d, const double *C, const double *occ, int nuse, bool gga, long long N, double *rho,
+               double *grho, double *psi, cudaStream_t st);
+
 // fft_fp64.cu
 void launch_fft3d(double2 *c, int ng, int batch, const double2 *tw, bool inverse, cudaStream_t st);
 void launch_real_to_complex(const double *a, const double *s, long long N, int batch, double2 *c,

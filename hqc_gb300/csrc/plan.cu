@@ -213,6 +213,8 @@ struct hqcgb_plan {
   float2 *cbuf32 = nullptr;
   int *tc_err = nullptr;
   Quad64 q64{};                // FP64 quadratures
+  Density64 d64{};             // FP64 density from the orbitals
+  int nuse_64 = 0;             // orbitals it runs over
   MixedEigWork mew{};
   bool eig_wide = false;       // FP64 path: this geometry's Fock matrices need the FP32 QL sweep
   // exact exchange in the occupied-pair form (exchange.cu); R = double on
@@ -502,6 +504,17 @@ static void create(const hqcgb_params *in, hqcgb_plan *p) {
     }
     q.err = p->tc_err;
   }
+  if (!p->mixed && nao <= density64_max_ao()) {
+    const int fields = p->gga ? 4 : 1;
+    Density64 &d = p->d64;
+    d.n = nao;
+    d.A = p->alloc<char>(fields * density64_field_bytes(nao, N));
+    d.B = p->alloc<char>(density64_orbital_bytes(nao));
+    d.sA = p->alloc<double>(fields * N);
+    d.e = p->alloc<int>(N);
+    d.eY = p->alloc<int>(nao);
+    d.err = p->tc_err;
+  }
   p->xpart = p->alloc<double>((size_t)2 * xc_blocks(N));
   if (P.want_forces) {
     p->fpart = p->alloc<double>(std::max((size_t)nao * force_grid_blocks(N) * 3,
@@ -610,7 +623,8 @@ static void density_matrix(Ctx &c) {
               P.search_cycle, P.search_tol, occ_shift(p), p->w, p->occ, p->mu, c.st);
   p->nuse_dm = 0;
   p->exx_psi_ready = false;
-  if (p->mixed || p->hf) {
+  p->nuse_64 = std::max(1, P.n_atoms / 2);
+  if (p->mixed || p->hf || (P.smearing && p->d64.n)) {
     // The one host copy of the occupations per iteration: the mixed density
     // and the exchange of the Fock build that follows size their launches
     // from it.  Orbitals with a non-negligible occupation come first
@@ -622,6 +636,9 @@ static void density_matrix(Ctx &c) {
     for (int k = 0; k < n; ++k)
       if (p->hocc[k] > 1e-14) nuse = k + 1;
     p->nuse_occ = nuse;
+    // FP64 density: what is left out is below 1e-18 of |psi|^2
+    for (int k = 0; k < n; ++k)
+      if (!(p->hocc[k] <= 1e-18)) p->nuse_64 = std::max(p->nuse_64, k + 1);
     if (p->mixed && nuse >= 1 && nuse <= kThinOcc) {
       launch_occ_block(p->C, p->occ, n, nuse, p->Yd, c.st);
       gemm(false, true, n, n, nuse, 1.0, p->Yd, nuse, p->Yd, nuse, nullptr, 0.0, p->D, n, c.st);
@@ -811,8 +828,14 @@ static double fock(Ctx &c) {
     launch_tc_quadrature(p->phi32, p->dphi32, p->phihl, p->w32, p->u32, (float)p->dV, n, N, p->ld,
                          p->gga, 1.0, p->tcq_part, p->F2e, p->tc_err, c.st, p->hf ? 1 : 4, p->zhl);
   } else {
-  launch_density(p->phi, p->gga ? p->dphi : nullptr, p->D, n, N, p->rho, p->gga ? p->grho : nullptr,
-                 nullptr, c.st);
+  if (p->d64.n) {
+    double *psi = p->exx_fused ? static_cast<double *>(p->exx_psi) : nullptr;  // the exchange takes them
+    density64(p->d64, p->C, p->occ, p->nuse_64, p->gga, N, p->rho, p->gga ? p->grho : nullptr, psi, c.st);
+    p->exx_psi_ready = psi != nullptr;
+  } else {
+    launch_density(p->phi, p->gga ? p->dphi : nullptr, p->D, n, N, p->rho, p->gga ? p->grho : nullptr,
+                   nullptr, c.st);
+  }
   poisson(c, p->rho, p->vh);
   launch_xc_pointwise(kind, p->rho, p->gga ? p->grho : nullptr, p->vh, N, p->dV, p->wq, p->vxc,
                       p->gga ? p->u : nullptr, p->xpart, c.st);
@@ -875,6 +898,7 @@ static void geometry(Ctx &c, const double *xp_dev) {
   if (p->phi)
     launch_phi(p->F1d, p->coef, p->ao_l, p->ao_cart, p->nb, p->nprim, n, p->ng, p->phi, p->dphi,
                c.st);
+  if (p->d64.n) density64_basis(p->d64, p->phi, p->gga ? p->dphi : nullptr, N, c.st);
   if (p->q64.n) quad64_basis(p->q64, p->phi, p->gga && !p->mixed ? p->dphi : nullptr, N, c.st);
   if (p->mixed) {
     launch_to_float((long long)p->n * 3 * p->ng * P.n_prim * 6, p->F1d, p->F1d32, c.st);

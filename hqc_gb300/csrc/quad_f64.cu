@@ -32,14 +32,13 @@
 #include <algorithm>
 #include <cmath>
 
+#include "digits.cuh"
 #include "kernels.h"
-#include "tc_ptx.cuh"
 
 namespace hqcgb {
 
 using namespace tc;
 
-constexpr int kQfDigits = 8, kQfPairs = kQfDigits / 2;
 constexpr int kQfK = 32;                                // points per stage
 constexpr int kQfChain = 16;                            // stages per TMEM sum (512 points)
 constexpr int kQfM = 128, kQfN = 64;
@@ -132,19 +131,6 @@ __global__ void __launch_bounds__(128)
   }
 }
 
-// The digits of x 2^-e as unsigned 7-bit fields, each 64 above the digit.
-__device__ __forceinline__ unsigned long long qf_fields(double x, int e) {
-  constexpr long long kBias = 64LL * ((1LL << 0) + (1LL << 7) + (1LL << 14) + (1LL << 21) + (1LL << 28) +
-                                      (1LL << 35) + (1LL << 42) + (1LL << 49));
-  const long long bits = __double_as_longlong(x);
-  const int ex = (int)((bits >> 52) & 0x7ff);
-  const int sh = ex - 1075 + 7 * kQfDigits - e;  // x 2^-e 128^8 = m 2^sh
-  const long long m = (bits & 0xfffffffffffffLL) | (1LL << 52);
-  long long I = 0;
-  if (ex > 0 && sh > -54) I = sh >= 0 ? m << min(sh, 3) : (m + (1LL << (-sh - 1))) >> -sh;
-  return (unsigned long long)((bits < 0 ? -I : I) + kBias);
-}
-
 // Digits of X (MODE 0), w X (1) or 0.5 w X + dV u.dX (2) into the operand
 // layout; blockIdx.x = block of 32 points, a warp takes 8 rows x 4 chunks of
 // 8 points.  Points beyond N become zeros; rows beyond n are left alone (they
@@ -168,8 +154,7 @@ __global__ void __launch_bounds__(256)
       for (int i = 0; i < 8; ++i) uv[d * 8 + i] = i < cnt ? dV * u[(long long)d * N + g0 + i] : 0.0;
   for (int p = (threadIdx.x >> 5) * 8 + (lane >> 2); p < n; p += 64) {
     const int ep = e[p];
-    unsigned pk[kQfDigits][4];
-    float lo[kQfDigits];
+    QfPack pack;
 #pragma unroll
     for (int i = 0; i < 8; ++i) {
       double x = 0.0;
@@ -181,21 +166,11 @@ __global__ void __launch_bounds__(256)
 #pragma unroll
           for (int d = 0; d < 3; ++d) x += uv[d * 8 + i] * dX[(long long)d * n * N + at];
       }
-      const unsigned long long J = qf_fields(x, ep);
-#pragma unroll
-      for (int s = 0; s < kQfDigits; ++s) {
-        const unsigned f = (unsigned)(J >> (7 * (kQfDigits - 1 - s))) & (s ? 127u : 255u);
-        const float v = __uint_as_float(0x4B000000u | f) - 8388672.f;  // 2^23 + f - (2^23 + 64), exact
-        if (i & 1) pk[s][i >> 1] = __byte_perm(__float_as_uint(lo[s]), __float_as_uint(v), 0x7632);
-        else lo[s] = v;
-      }
+      pack.put(i, x, ep);
     }
     char *row = out + ((kb * rbn + p / rb) * kQfPairs * (long long)rb + p % rb) * 128;
     const int r = p % rb;
-#pragma unroll
-    for (int s = 0; s < kQfDigits; ++s)
-      *reinterpret_cast<uint4 *>(row + (long long)(s >> 1) * rb * 128 + (((s & 1) * 4 + c) ^ (r & 7)) * 16) =
-          make_uint4(pk[s][0], pk[s][1], pk[s][2], pk[s][3]);
+    pack.store(row, (long long)rb * 128, c, r);
   }
 }
 
@@ -212,26 +187,6 @@ struct QfPipe {
   uint64_t full[kQfRing], empty[kQfRing], acc_full, acc_empty;
   uint32_t tmem_base;
 };
-
-__device__ inline void bulk_copy(uint32_t dst, const void *src, uint32_t bytes, uint64_t *bar) {
-  asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(dst),
-               "l"(src), "r"(bytes), "r"(smem_u32(bar))
-               : "memory");
-}
-
-__device__ inline void mma_bf16(uint32_t dtmem, uint64_t a, uint64_t b, uint32_t idesc, int acc) {
-  asm volatile(
-      "{\n\t.reg .pred p;\n\t"
-      "setp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}"
-      ::"r"(dtmem), "l"(a), "l"(b), "r"(idesc), "r"(acc));
-}
-
-__device__ inline void tmem_ld4_nowait(uint32_t taddr, uint32_t *r) {
-  asm volatile("tcgen05.ld.sync.aligned.32x32b.x4.b32 {%0,%1,%2,%3}, [%4];"
-               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
-               : "r"(taddr));
-}
 
 __global__ void __launch_bounds__(kQfThreads, 1) k_qf_gemm(const __grid_constant__ QfArgs a) {
   extern __shared__ __align__(1024) char smraw[];
