@@ -6,8 +6,8 @@
 //     T = Q^T A Q with the matrix in shared memory (k_tridiag_f32, the
 //     global-memory form of eigh_tridiag.cuh, above 310 AOs), reflectors
 //     stored contiguously.
-//  2. k_tri_eig_f32 (one block, a thread per eigenvalue): the eigenvalues of
-//     T by bisection on Sturm counts (W. Barth, R. S. Martin, J. H.
+//  2. k_tri_values_f32 (a thread per eigenvalue): the eigenvalues of T by
+//     bisection on Sturm counts (W. Barth, R. S. Martin, J. H.
 //     Wilkinson, "Calculation of the eigenvalues of a symmetric tridiagonal
 //     matrix by the method of bisection", Numer. Math. 9 (1967) 386-393), all
 //     in parallel; then the eigenvectors of T by inverse iteration with a
@@ -56,21 +56,28 @@ __global__ void __launch_bounds__(kTriThreads)
 // budget (n <= 310).
 __device__ inline int tri_ix(int i, int j) { return i * (i + 1) / 2 + j; }
 
-__global__ void __launch_bounds__(kTriThreads)
+// Bound by latency, not arithmetic: 270 dependent steps of one block.  So the
+// block's sums take one barrier (every warp adds the warps' parts itself), the
+// reflector's scalars are computed by every thread, and a warp works on four
+// rows of the triangle at a time.  n = 270: 2.0 -> 1.57 ms.
+constexpr int kTriSmemThreads = 1024;
+constexpr int kTriRows = 4;  // rows a warp works on at a time
+__global__ void __launch_bounds__(kTriSmemThreads)
     k_tridiag_f32_smem(int n, const float *__restrict__ A, float *__restrict__ dg,
                        float *__restrict__ eg, float *__restrict__ taug, float *__restrict__ hv) {
   extern __shared__ __align__(16) float tsh[];
   float *L = tsh, *d = L + n * (n + 1) / 2, *e = d + n, *tau = e + n, *v = tau + n, *p = v + n;
-  __shared__ float red[32];
-  __shared__ float s_beta[2];
+  __shared__ float red[2][32];
   const int tid = threadIdx.x, nt = blockDim.x, lane = tid & 31, warp = tid >> 5, nw = nt >> 5;
-  for (int idx = tid; idx < n * (n + 1) / 2; idx += nt) {
-    // row i of the packed triangle: the largest i with i (i + 1) / 2 <= idx
-    int i = (int)((sqrtf(8.f * (float)idx + 1.f) - 1.f) * 0.5f);
-    while (i * (i + 1) / 2 > idx) --i;
-    while ((i + 1) * (i + 2) / 2 <= idx) ++i;
-    L[idx] = A[(long long)i * n + (idx - i * (i + 1) / 2)];
-  }
+  // sum over the block, to every thread; `buf` alternates between calls
+  auto sum = [&](float x, int buf) {
+    x = warp_sum(x);
+    if (lane == 0) red[buf][warp] = x;
+    __syncthreads();
+    return warp_sum(lane < nw ? red[buf][lane] : 0.f);
+  };
+  for (int i = warp; i < n; i += nw)
+    for (int j = lane; j <= i; j += 32) L[tri_ix(i, j)] = A[(long long)i * n + j];
   __syncthreads();
   for (int k = 0; k < n - 2; ++k) {
     const int m = n - k - 1;  // trailing rows k+1 .. n-1
@@ -79,22 +86,18 @@ __global__ void __launch_bounds__(kTriThreads)
       float x = L[tri_ix(k + 1 + i, k)];
       s2 += x * x;
     }
-    s2 = block_sum(s2, red);
-    if (tid == 0) {
-      const float x0 = L[tri_ix(k + 1, k)];
-      if (s2 == 0.f) {
-        tau[k] = 0.f;
-        e[k] = x0;
-        s_beta[0] = 0.f;
-      } else {
-        const float beta = -copysignf(sqrtf(x0 * x0 + s2), x0);
-        tau[k] = (beta - x0) / beta;
-        e[k] = beta;
-        s_beta[0] = 1.f / (x0 - beta);
-      }
+    s2 = sum(s2, 0);
+    const float x0 = L[tri_ix(k + 1, k)];
+    float tk = 0.f, sc = 0.f, beta = x0;
+    if (s2 != 0.f) {
+      beta = -copysignf(sqrtf(x0 * x0 + s2), x0);
+      tk = (beta - x0) / beta;
+      sc = 1.f / (x0 - beta);
     }
-    __syncthreads();
-    const float tk = tau[k], sc = s_beta[0];
+    if (tid == 0) {
+      tau[k] = tk;
+      e[k] = beta;
+    }
     for (int i = tid; i < m; i += nt) {
       v[i] = (i == 0) ? 1.f : (tk == 0.f ? 0.f : L[tri_ix(k + 1 + i, k)] * sc);
       hv[(long long)k * n + i] = v[i];
@@ -103,31 +106,46 @@ __global__ void __launch_bounds__(kTriThreads)
     if (tk == 0.f) continue;
     // p = tau A22 v, one warp per row i: sum over j <= i of L[i][j] v_j and
     // over j > i of L[j][i] v_j (trailing block indices)
-    for (int i = warp; i < m; i += nw) {
-      const int gi = k + 1 + i;
-      float sum = 0.f;
+    for (int i0 = warp; i0 < m; i0 += kTriRows * nw) {
+      float acc[kTriRows];
+#pragma unroll
+      for (int r = 0; r < kTriRows; ++r) acc[r] = 0.f;
       for (int j = lane; j < m; j += 32) {
-        const int gj = k + 1 + j;
-        sum += (j <= i ? L[tri_ix(gi, gj)] : L[tri_ix(gj, gi)]) * v[j];
+        const float vj = v[j];
+        const int col = tri_ix(k + 1 + j, k + 1);
+#pragma unroll
+        for (int r = 0; r < kTriRows; ++r) {
+          const int i = i0 + r * nw;
+          if (i < m) acc[r] += L[j <= i ? tri_ix(k + 1 + i, k + 1) + j : col + i] * vj;
+        }
       }
-      sum = warp_sum(sum);
-      if (lane == 0) p[i] = tk * sum;
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1)
+#pragma unroll
+        for (int r = 0; r < kTriRows; ++r) acc[r] += __shfl_xor_sync(0xffffffffu, acc[r], o);
+      if (lane == 0)
+#pragma unroll
+        for (int r = 0; r < kTriRows; ++r)
+          if (i0 + r * nw < m) p[i0 + r * nw] = tk * acc[r];
     }
     __syncthreads();
     float pv = 0.f;
     for (int i = tid; i < m; i += nt) pv += p[i] * v[i];
-    pv = block_sum(pv, red);
+    pv = sum(pv, 1);
     const float alpha = -0.5f * tk * pv;
     for (int i = tid; i < m; i += nt) p[i] += alpha * v[i];  // p becomes w
     __syncthreads();
     // rank-2 update of the trailing lower triangle
-    const int tri = m * (m + 1) / 2;
-    for (int idx = tid; idx < tri; idx += nt) {
-      int i = (int)((sqrtf(8.f * (float)idx + 1.f) - 1.f) * 0.5f);
-      while (i * (i + 1) / 2 > idx) --i;
-      while ((i + 1) * (i + 2) / 2 <= idx) ++i;
-      const int j = idx - i * (i + 1) / 2;
-      L[tri_ix(k + 1 + i, k + 1 + j)] -= v[i] * p[j] + p[i] * v[j];
+    for (int i0 = warp; i0 < m; i0 += kTriRows * nw) {
+      const int last = min(m - 1, i0 + (kTriRows - 1) * nw);
+      for (int j = lane; j <= last; j += 32) {
+        const float vj = v[j], pj = p[j];
+#pragma unroll
+        for (int r = 0; r < kTriRows; ++r) {
+          const int i = i0 + r * nw;
+          if (i < m && j <= i) L[tri_ix(k + 1 + i, k + 1) + j] -= v[i] * pj + p[i] * vj;
+        }
+      }
     }
     __syncthreads();
   }
@@ -152,185 +170,271 @@ __device__ inline int sturm_count(int n, const float *__restrict__ d, const floa
   return c;
 }
 
-// Eigenpairs of the tridiagonal (d, e): w ascending, Z[r][c] column c the
-// eigenvector of w[c].  scr: 6 n x n floats (LU factors and the vector of
-// each cluster leader, interleaved by leader).
-__global__ void __launch_bounds__(kTriThreads)
-    k_tri_eig_f32(int n, const float *__restrict__ dg, const float *__restrict__ eg,
-                  float *__restrict__ w, float *__restrict__ Z, float *__restrict__ scr) {
+// Gershgorin interval [lo, hi] and the scales of the tridiagonal (d, e).
+struct TriScale {
+  float tnorm, pivmin, lo, hi;
+};
+
+// Eigenvalues of the tridiagonal, w ascending: a warp per eigenvalue and block
+// (every block forms the interval from all of d and e).  A Sturm count is a
+// chain of n divisions, so its length is what a bisection costs: speculating
+// five halvings ahead takes a fifth of the chains.  n = 270: 0.47 -> 0.11 ms.
+__global__ void __launch_bounds__(32)
+    k_tri_values_f32(int n, const float *__restrict__ dg, const float *__restrict__ eg, float *__restrict__ w,
+                     TriScale *__restrict__ scale) {
   extern __shared__ __align__(16) float ssh[];
-  float *d = ssh, *e = d + n, *e2 = e + n, *lam = e2 + n;
-  __shared__ float red[32];
-  const int tid = threadIdx.x, nt = blockDim.x;
+  float *d = ssh, *e2 = d + n;
   float lo = FLT_MAX, hi = -FLT_MAX, emax2 = 0.f;
-  for (int i = tid; i < n; i += nt) {
+  for (int i = threadIdx.x; i < n; i += 32) {
     d[i] = dg[i];
-    e[i] = i < n - 1 ? eg[i] : 0.f;
-    e2[i] = e[i] * e[i];
+    const float ei = i < n - 1 ? eg[i] : 0.f;
+    e2[i] = ei * ei;
     float r = (i > 0 ? fabsf(eg[i - 1]) : 0.f) + (i < n - 1 ? fabsf(eg[i]) : 0.f);
     lo = fminf(lo, dg[i] - r);
     hi = fmaxf(hi, dg[i] + r);
     emax2 = fmaxf(emax2, e2[i]);
   }
-  lo = -block_max(-lo, red);
-  hi = block_max(hi, red);
-  emax2 = block_max(emax2, red);
+  for (int o = 16; o > 0; o >>= 1) {
+    lo = fminf(lo, __shfl_xor_sync(0xffffffffu, lo, o));
+    hi = fmaxf(hi, __shfl_xor_sync(0xffffffffu, hi, o));
+    emax2 = fmaxf(emax2, __shfl_xor_sync(0xffffffffu, emax2, o));
+  }
+  __syncwarp();
   const float tnorm = fmaxf(fabsf(lo), fabsf(hi));
   const float pivmin = FLT_MIN * fmaxf(1.f, emax2);
   // widen the Gershgorin interval so that both ends are strict bounds
   const float pad = 2.f * FLT_EPSILON * tnorm + 4.f * pivmin;
   lo -= pad;
   hi += pad;
-
-  // --- eigenvalue i by bisection: count(lo) <= i < count(hi)
-  for (int i = tid; i < n; i += nt) {
-    float a = lo, b = hi;
-    for (int it = 0; it < 80; ++it) {
-      float mid = 0.5f * (a + b);
-      if (mid <= a || mid >= b) break;
-      if (b - a <= 2.f * FLT_EPSILON * fmaxf(fabsf(a), fabsf(b)) + pivmin) break;
-      if (sturm_count(n, d, e2, mid, pivmin) <= i) a = mid;
-      else b = mid;
+  if (blockIdx.x == 0 && threadIdx.x == 0) *scale = TriScale{tnorm, pivmin, lo, hi};
+  // eigenvalue i by bisection, count(lo) <= i < count(hi), five halvings a
+  // round: lane l evaluates node l of the tree of midpoints (children of l: 2 l
+  // below, 2 l + 1 above it), then the warp walks the path that the counts give
+  const int i = blockIdx.x, lane = threadIdx.x;
+  float a = lo, b = hi;
+  for (int it = 0; it < 80;) {
+    float la = a, lb = b;
+    for (int bit = 30 - __clz(max(lane, 1)); bit >= 0; --bit) {
+      const float mid = 0.5f * (la + lb);
+      if ((lane >> bit) & 1) la = mid;
+      else lb = mid;
     }
-    lam[i] = 0.5f * (a + b);
+    const int above = sturm_count(n, d, e2, 0.5f * (la + lb), pivmin) <= i;
+    const unsigned up = __ballot_sync(0xffffffffu, above);
+    bool done = false;
+    for (int node = 1; node < 32 && it < 80; ++it) {
+      const float mid = 0.5f * (a + b);
+      done = mid <= a || mid >= b || b - a <= 2.f * FLT_EPSILON * fmaxf(fabsf(a), fabsf(b)) + pivmin;
+      if (done) break;
+      const int right = (up >> node) & 1;
+      if (right) a = mid;
+      else b = mid;
+      node = 2 * node + right;
+    }
+    if (done) break;
   }
-  __syncthreads();
-  for (int i = tid; i < n; i += nt) w[i] = lam[i];
+  if (lane == 0) w[i] = 0.5f * (a + b);
+}
 
-  // --- eigenvectors by inverse iteration; the first member of each cluster
-  // computes the cluster's vectors in order
+// Eigenvectors of the tridiagonal by inverse iteration, Z[r][c] column c that
+// of w[c]; the first member of each cluster computes the cluster's vectors in
+// order.  A warp per leader and block: the solves are chains of dependent
+// steps that every lane follows in shared memory (30 cycles a step where they
+// took an L2 round trip), sums run in the same order from values that the lanes
+// fetch 32 at a time, and what is independent is spread over the lanes.
+// n = 270, with k_tri_values_f32: 2.15 -> 0.78 ms.
+__global__ void __launch_bounds__(32)
+    k_tri_vectors_f32(int n, const float *__restrict__ dg, const float *__restrict__ eg, const float *__restrict__ lam,
+                      const TriScale *__restrict__ scale, float *__restrict__ Z) {
+  extern __shared__ __align__(16) float ssh[];
+  const int lane = threadIdx.x, i0 = blockIdx.x;
+  float *d = ssh, *e = d + n, *u1 = e + n, *u2 = u1 + n, *u3 = u2 + n, *lm = u3 + n, *x = lm + n;
+  unsigned *swap = reinterpret_cast<unsigned *>(x + n);  // bit k: rows k, k + 1 swapped
+  const float tnorm = scale->tnorm, pivmin = scale->pivmin;
   // clusters: eigenvalues within 1e-4 ||T||; vectors of eigenvalues further
   // apart are orthogonal to FP32 eps ||T|| / gap <= 1e-3, which the FP64
   // refinement removes
   const float sep = 1e-4f * tnorm;
   const float tiny = FLT_EPSILON * tnorm + pivmin;
-  for (int i0 = tid; i0 < n; i0 += nt) {
-    if (i0 > 0 && lam[i0] - lam[i0 - 1] <= sep) continue;
-    int i1 = i0;
-    while (i1 + 1 < n && lam[i1 + 1] - lam[i1] <= sep) ++i1;
-    // per-leader arrays interleaved by leader (element k of leader i0 at
-    // k * n + i0): the leaders step through k together, so a warp's accesses
-    // are one coalesced line instead of 32 scattered ones
-    float *u1 = scr + i0, *u2 = u1 + (long long)n * n, *u3 = u2 + (long long)n * n,
-          *lm = u3 + (long long)n * n, *pv = lm + (long long)n * n, *x = pv + (long long)n * n;
-#define U1(k) u1[(long long)(k) * n]
-#define U2(k) u2[(long long)(k) * n]
-#define U3(k) u3[(long long)(k) * n]
-#define LM(k) lm[(long long)(k) * n]
-#define PV(k) pv[(long long)(k) * n]
-#define XX(k) x[(long long)(k) * n]
-    float shift_prev = 0.f;
-    for (int j = i0; j <= i1; ++j) {
-      // equal eigenvalues in a cluster are separated a little so that the
-      // solves differ (the Gram-Schmidt step makes the vectors orthogonal)
-      float lj = lam[j];
-      if (j > i0 && lj - shift_prev < 10.f * tiny) lj = shift_prev + 10.f * tiny;
-      shift_prev = lj;
-      // LU with partial pivoting of T - lj I (rows k, k+1 swapped when the
-      // subdiagonal entry is the larger pivot); U has two superdiagonals
-      float b = d[0] - lj, c = n > 1 ? e[0] : 0.f;
-      for (int k = 0; k < n - 1; ++k) {
-        const float a = e[k], bn = d[k + 1] - lj, cn = k + 1 < n - 1 ? e[k + 1] : 0.f;
-        if (fabsf(b) >= fabsf(a)) {
-          if (b == 0.f) b = tiny;
-          const float l = a / b;
-          U1(k) = b; U2(k) = c; U3(k) = 0.f; LM(k) = l; PV(k) = 0.f;
-          b = bn - l * c;
-          c = cn;
-        } else {
-          const float l = b / a;
-          U1(k) = a; U2(k) = bn; U3(k) = cn; LM(k) = l; PV(k) = 1.f;
-          b = c - l * bn;
-          c = -l * cn;
-        }
+  if (i0 > 0 && lam[i0] - lam[i0 - 1] <= sep) return;
+  for (int i = lane; i < n; i += 32) {
+    d[i] = dg[i];
+    e[i] = i < n - 1 ? eg[i] : 0.f;
+  }
+  __syncwarp();
+  int i1 = i0;
+  while (i1 + 1 < n && lam[i1 + 1] - lam[i1] <= sep) ++i1;
+  float shift_prev = 0.f;
+  for (int j = i0; j <= i1; ++j) {
+    // equal eigenvalues in a cluster are separated a little so that the
+    // solves differ (the Gram-Schmidt step makes the vectors orthogonal)
+    float lj = lam[j];
+    if (j > i0 && lj - shift_prev < 10.f * tiny) lj = shift_prev + 10.f * tiny;
+    shift_prev = lj;
+    // LU with partial pivoting of T - lj I (rows k, k+1 swapped when the
+    // subdiagonal entry is the larger pivot); U has two superdiagonals
+    float b = d[0] - lj, c = n > 1 ? e[0] : 0.f;
+    unsigned bits = 0;
+    for (int k = 0; k < n - 1; ++k) {
+      const float a = e[k], bn = d[k + 1] - lj, cn = k + 1 < n - 1 ? e[k + 1] : 0.f;
+      float p1, p2, p3, l;
+      if (fabsf(b) >= fabsf(a)) {
+        if (b == 0.f) b = tiny;
+        l = a / b;
+        p1 = b; p2 = c; p3 = 0.f;
+        b = bn - l * c;
+        c = cn;
+      } else {
+        l = b / a;
+        p1 = a; p2 = bn; p3 = cn;
+        b = c - l * bn;
+        c = -l * cn;
+        bits |= 1u << (k & 31);
       }
-      U1(n - 1) = fabsf(b) < tiny ? (b < 0.f ? -tiny : tiny) : b;
-      for (int k = 0; k < n - 1; ++k)
-        if (fabsf(U1(k)) < tiny) U1(k) = U1(k) < 0.f ? -tiny : tiny;
-      // start vector: deterministic, not orthogonal to any eigenvector in practice
-      for (int k = 0; k < n; ++k) XX(k) = 1.f + 0.37f * __sinf(0.7f * (float)k + 1.3f * (float)j);
-      for (int it = 0; it < 3; ++it) {
-        // L y = P x
-        for (int k = 0; k < n - 1; ++k) {
-          if (PV(k) != 0.f) {
-            float t = XX(k);
-            XX(k) = XX(k + 1);
-            XX(k + 1) = t;
-          }
-          XX(k + 1) -= LM(k) * XX(k);
-        }
-        // U z = y
-        XX(n - 1) /= U1(n - 1);
-        if (n > 1) XX(n - 2) = (XX(n - 2) - U2(n - 2) * XX(n - 1)) / U1(n - 2);
-        for (int k = n - 3; k >= 0; --k)
-          XX(k) = (XX(k) - U2(k) * XX(k + 1) - U3(k) * XX(k + 2)) / U1(k);
-        // orthogonalise against the cluster's earlier vectors, normalise
-        for (int q = i0; q < j; ++q) {
-          float s = 0.f;
-          for (int k = 0; k < n; ++k) s += Z[(long long)k * n + q] * XX(k);
-          for (int k = 0; k < n; ++k) XX(k) -= s * Z[(long long)k * n + q];
-        }
-        float nrm = 0.f;
-        for (int k = 0; k < n; ++k) nrm += XX(k) * XX(k);
-        nrm = nrm > 0.f ? rsqrtf(nrm) : 0.f;
-        for (int k = 0; k < n; ++k) XX(k) *= nrm;
+      if (lane == 0) {
+        u1[k] = fabsf(p1) < tiny ? (p1 < 0.f ? -tiny : tiny) : p1;
+        u2[k] = p2; u3[k] = p3; lm[k] = l;
+        if ((k & 31) == 31 || k == n - 2) swap[k >> 5] = bits;
       }
-      for (int k = 0; k < n; ++k) Z[(long long)k * n + j] = XX(k);
+      if ((k & 31) == 31) bits = 0;
     }
-#undef U1
-#undef U2
-#undef U3
-#undef LM
-#undef PV
-#undef XX
+    if (lane == 0) u1[n - 1] = fabsf(b) < tiny ? (b < 0.f ? -tiny : tiny) : b;
+    // start vector: deterministic, not orthogonal to any eigenvector in practice
+    for (int k = lane; k < n; k += 32) x[k] = 1.f + 0.37f * __sinf(0.7f * (float)k + 1.3f * (float)j);
+    __syncwarp();
+    for (int it = 0; it < 3; ++it) {
+      // L y = P x
+      float x0 = x[0];
+      unsigned word = 0;
+      for (int k = 0; k < n - 1; ++k) {
+        if ((k & 31) == 0) word = swap[k >> 5];
+        float x1 = x[k + 1];
+        if ((word >> (k & 31)) & 1) {
+          const float t = x0;
+          x0 = x1;
+          x1 = t;
+        }
+        x1 -= lm[k] * x0;
+        if (lane == 0) x[k] = x0;
+        x0 = x1;
+      }
+      __syncwarp();
+      // U z = y
+      float z1 = x0 / u1[n - 1], z2 = 0.f;
+      if (lane == 0) x[n - 1] = z1;
+      if (n > 1) {
+        z2 = z1;
+        z1 = (x[n - 2] - u2[n - 2] * z2) / u1[n - 2];
+        __syncwarp();
+        if (lane == 0) x[n - 2] = z1;
+      }
+      for (int k = n - 3; k >= 0; --k) {
+        const float z = (x[k] - u2[k] * z1 - u3[k] * z2) / u1[k];
+        z2 = z1;
+        z1 = z;
+        __syncwarp();
+        if (lane == 0) x[k] = z;
+      }
+      __syncwarp();
+      // orthogonalise against the cluster's earlier vectors, normalise
+      for (int q = i0; q < j; ++q) {
+        float s = 0.f;
+        for (int k0 = 0; k0 < n; k0 += 32) {
+          const int k = k0 + lane;
+          const float zv = k < n ? Z[(long long)k * n + q] : 0.f, xv = k < n ? x[k] : 0.f;
+          const int cnt = min(32, n - k0);
+          for (int l = 0; l < cnt; ++l)
+            s += __shfl_sync(0xffffffffu, zv, l) * __shfl_sync(0xffffffffu, xv, l);
+        }
+        __syncwarp();
+        for (int k = lane; k < n; k += 32) x[k] -= s * Z[(long long)k * n + q];
+        __syncwarp();
+      }
+      float nrm = 0.f;
+#pragma unroll 8
+      for (int k = 0; k < n; ++k) nrm += x[k] * x[k];
+      nrm = nrm > 0.f ? rsqrtf(nrm) : 0.f;
+      __syncwarp();
+      for (int k = lane; k < n; k += 32) x[k] *= nrm;
+      __syncwarp();
+    }
+    for (int k = lane; k < n; k += 32) Z[(long long)k * n + j] = x[k];
+    __syncwarp();
   }
 }
 
 // V = Q Z for 32 columns per block: Z tile in shared memory, reflectors
 // H_k = I - tau_k v_k v_k^T (rows k+1..n-1) applied for k = n-3 .. 0; eight
-// threads (one warp quarter) own a column.
+// threads (one warp quarter) own a column.  The next reflector is on its way
+// in registers while one is applied; rows of 36 floats keep the eight threads
+// of four columns in different banks.  n = 270: 0.96 -> 0.27 ms.
+constexpr int kBackLd = 36, kBackFetch = (kMaxNao + 255) / 256;
 __global__ void __launch_bounds__(256)
     k_backtransform_f32(int n, const float *__restrict__ hv, const float *__restrict__ tau,
                         const float *__restrict__ Z, float *__restrict__ V) {
-  extern __shared__ __align__(16) float zt[];  // [n][33]
+  extern __shared__ __align__(16) float zt[];  // [n][kBackLd], then 2 [n]
+  float *vbuf = zt + n * kBackLd;
   const int c0 = blockIdx.x * 32;
   const int tid = threadIdx.x, cc = tid >> 3, part = tid & 7;
   for (int idx = tid; idx < n * 32; idx += blockDim.x) {
     int r = idx >> 5, c = idx & 31;
-    zt[r * 33 + c] = (c0 + c < n) ? Z[(long long)r * n + c0 + c] : 0.f;
+    zt[r * kBackLd + c] = (c0 + c < n) ? Z[(long long)r * n + c0 + c] : 0.f;
   }
-  __syncthreads();
+  float next[kBackFetch], tnext = 0.f;
+  auto fetch = [&](int k) {
+#pragma unroll
+    for (int q = 0; q < kBackFetch; ++q)
+      if (q * 256 + tid < n - k - 1) next[q] = hv[(long long)k * n + q * 256 + tid];
+    tnext = tau[k];
+  };
+  auto put = [&](int k) {
+#pragma unroll
+    for (int q = 0; q < kBackFetch; ++q)
+      if (q * 256 + tid < n - k - 1) vbuf[(k & 1) * n + q * 256 + tid] = next[q];
+  };
+  float tk = 0.f;
+  if (n >= 3) {
+    fetch(n - 3);
+    put(n - 3);
+    tk = tnext;
+  }
   for (int k = n - 3; k >= 0; --k) {
-    const float tk = tau[k];
-    if (tk == 0.f) continue;
+    __syncthreads();
+    if (k > 0) fetch(k - 1);
     const int m = n - k - 1;
-    const float *vk = hv + (long long)k * n;
-    float s = 0.f;
-    for (int i = part; i < m; i += 8) s += vk[i] * zt[(k + 1 + i) * 33 + cc];
-    s += __shfl_xor_sync(0xffffffffu, s, 1);
-    s += __shfl_xor_sync(0xffffffffu, s, 2);
-    s += __shfl_xor_sync(0xffffffffu, s, 4);
-    s *= tk;
-    for (int i = part; i < m; i += 8) zt[(k + 1 + i) * 33 + cc] -= s * vk[i];
-    __syncwarp();
+    const float *vk = vbuf + (k & 1) * n;
+    float *z = zt + (k + 1) * kBackLd + cc;
+    if (tk != 0.f) {
+      float s = 0.f;
+#pragma unroll 4
+      for (int i = part; i < m; i += 8) s += vk[i] * z[i * kBackLd];
+      s += __shfl_xor_sync(0xffffffffu, s, 1);
+      s += __shfl_xor_sync(0xffffffffu, s, 2);
+      s += __shfl_xor_sync(0xffffffffu, s, 4);
+      s *= tk;
+#pragma unroll 4
+      for (int i = part; i < m; i += 8) z[i * kBackLd] -= s * vk[i];
+    }
+    if (k > 0) put(k - 1);
+    tk = tnext;
   }
   __syncthreads();
   for (int idx = tid; idx < n * 32; idx += blockDim.x) {
     int r = idx >> 5, c = idx & 31;
-    if (c0 + c < n) V[(long long)r * n + c0 + c] = zt[r * 33 + c];
+    if (c0 + c < n) V[(long long)r * n + c0 + c] = zt[r * kBackLd + c];
   }
 }
 
-size_t eigh_f32_scratch_floats(int n) { return (size_t)6 * n * n + (size_t)n * n + 4 * (size_t)n; }
+size_t eigh_f32_scratch_floats(int n) { return (size_t)n * n + 4 * (size_t)n + 8; }
 
 // A (n x n, destroyed) -> w ascending, V columns.  scr: eigh_f32_scratch_floats(n).
 void eigh_f32(int n, float *A, float *V, float *w, float *scr, cudaStream_t st) {
   HQ_STAGE(ST_JACOBI, st);
-  float *lu = scr, *hv = lu + (size_t)6 * n * n, *dg = hv + (size_t)n * n, *eg = dg + n,
-        *taug = eg + n;
+  float *hv = scr, *dg = hv + (size_t)n * n, *eg = dg + n, *taug = eg + n;
+  TriScale *scale = reinterpret_cast<TriScale *>(taug + n);
   size_t sm1 = (size_t)5 * n * sizeof(float);
-  size_t sm2 = (size_t)4 * n * sizeof(float);
-  size_t sm3 = (size_t)n * 33 * sizeof(float);
+  size_t sm2 = (size_t)(7 * n + (n + 31) / 32) * sizeof(float);
+  size_t sm3 = (size_t)n * (kBackLd + 2) * sizeof(float);
   HQ_REQUIRE(sm3 <= 200 * 1024, "matrix too large for the FP32 eigensolver");
   ensure_dyn_smem((const void *)k_backtransform_f32, sm3);
   const bool tr = std::getenv("HQCGB_TRACE") != nullptr;
@@ -341,14 +445,16 @@ void eigh_f32(int n, float *A, float *V, float *w, float *scr, cudaStream_t st) 
   const size_t smt = ((size_t)n * (n + 1) / 2 + 5 * (size_t)n) * sizeof(float);
   if (smt <= 200 * 1024) {
     ensure_dyn_smem((const void *)k_tridiag_f32_smem, smt);
-    k_tridiag_f32_smem<<<1, kTriThreads, smt, st>>>(n, A, dg, eg, taug, hv);
+    k_tridiag_f32_smem<<<1, kTriSmemThreads, smt, st>>>(n, A, dg, eg, taug, hv);
   } else {
     k_tridiag_f32<<<1, kTriThreads, sm1, st>>>(n, A, dg, eg, taug, hv);
   }
   HQ_LAUNCH_CHECK();
   if (tr) cudaEventRecord(ev[1], st);
   // Z (tridiagonal eigenvectors) goes to V, then V = Q Z in place per tile
-  k_tri_eig_f32<<<1, kTriThreads, sm2, st>>>(n, dg, eg, w, V, lu);
+  k_tri_values_f32<<<n, 32, 2 * n * sizeof(float), st>>>(n, dg, eg, w, scale);
+  HQ_LAUNCH_CHECK();
+  k_tri_vectors_f32<<<n, 32, sm2, st>>>(n, dg, eg, w, scale, V);
   HQ_LAUNCH_CHECK();
   if (tr) cudaEventRecord(ev[2], st);
   k_backtransform_f32<<<ceil_div(n, 32), 256, sm3, st>>>(n, hv, taug, V, V);

@@ -49,9 +49,7 @@ __global__ void k_f32_to_f64(long long n, const float *__restrict__ a, double *_
 // update, emax[2] = 1 when a cluster was too large, emax[3] = cluster count.
 constexpr int kMaxCluster = 48;      // largest cluster rotated (wide spectra)
 constexpr int kMaxClusterFock = 12;  // ... for Fock matrices (keeps the pass short)
-constexpr int kShCluster = 12;       // clusters up to this size rotate in shared memory
 constexpr int kOaThreads = 256;
-constexpr int kOaJacobiThreads = 16;  // clusters rotated with their blocks in shared memory
 
 // non-negative doubles compare like their bit patterns
 __device__ inline void atomic_max_nonneg(double *a, double v) {
@@ -92,33 +90,40 @@ __global__ void __launch_bounds__(kOaThreads) k_oa_stats(int n, const double *__
   }
 }
 
-// Pass 2 (one block): estimates, separation, clusters and the Jacobi
-// rotations W_C of the cluster blocks.
+// Pass 2a (one block): estimates, separation and clusters.
 //
 // Clusters (Ogita, Aishima, "Iterative refinement for symmetric eigenvalue
 // decomposition II: clustered eigenvalues", Japan J. Indust. Appl. Math. 36
 // (2019) 435-459): estimates closer than delta form a cluster, within which
 // the basic update only re-orthogonalises.  Each cluster C is rotated first
-// by the eigenvectors W_C of its block S_CC (cyclic Jacobi, one thread per
-// cluster): X_C <- X_C W_C, S <- W^T S W and G <- W^T G W (passes 3 and 4),
-// after which the cluster's Ritz values are separated and the iteration
-// converges quadratically again.  Clusters larger than kMaxCluster are left
-// unrotated and flagged.
+// by the eigenvectors W_C of its block S_CC (pass 2b): X_C <- X_C W_C,
+// S <- W^T S W and G <- W^T G W (passes 3 and 4), after which the cluster's
+// Ritz values are separated and the iteration converges quadratically again.
+// Clusters larger than max_cluster are left unrotated and flagged.
 // Outputs: emax[1] = ||S - diag(l)||_F / ||A||_F, emax[2] = 1 when a cluster
 // was too large, emax[3] = cluster count, emax[4] = delta; iwork = order,
 // cluster id, cluster start / size / wbuf offset, then the count at 5n.
+//
+// The order compares the estimates as integers (an FP64 comparison takes the
+// FP64 pipe, 73 000 of them 60 us), and the scan is the block's.
 __global__ void __launch_bounds__(1024) k_oa_clusters(int n, const double *__restrict__ S,
                                                       const double *__restrict__ G,
                                                       const double *__restrict__ red,
                                                       double *__restrict__ lam,
                                                       double *__restrict__ emax,
-                                                      int *__restrict__ iwork,
-                                                      double *__restrict__ wbuf, int max_cluster) {
-  __shared__ int s_nclus;
+                                                      int *__restrict__ iwork, int max_cluster) {
+  extern __shared__ double s_val[];  // [n] estimates ascending, then keys, order, near, size, id
+  long long *s_key = reinterpret_cast<long long *>(s_val + n);
+  int *s_order = reinterpret_cast<int *>(s_key + n), *s_near = s_order + n, *s_size = s_near + n, *s_id = s_size + n;
   const int tid = threadIdx.x, nt = blockDim.x;
   int *order = iwork, *cid = iwork + n, *cstart = iwork + 2 * n, *csize = iwork + 3 * n,
       *coff = iwork + 4 * n;
-  for (int i = tid; i < n; i += nt) lam[i] = S[(long long)i * n + i] / G[(long long)i * n + i];
+  for (int i = tid; i < n; i += nt) {
+    const double l = S[(long long)i * n + i] / G[(long long)i * n + i];
+    lam[i] = l;
+    const long long bits = __double_as_longlong(l + 0.0);  // -0 counts as 0
+    s_key[i] = bits < 0 ? bits ^ 0x7fffffffffffffffLL : bits;
+  }
   __syncthreads();
   // off-diagonal part of ||S - diag(l)||: the diagonal of S - diag(l) is
   // s_ii (1 - 1/g_ii), negligible, and is left out
@@ -131,57 +136,86 @@ __global__ void __launch_bounds__(1024) k_oa_clusters(int n, const double *__res
   // lumps whole bands of a 270-AO Fock matrix into one cluster.)
   const double delta = fmax(10.0 * cmax, 1e-6 * sqrt(a2 / n));
   for (int i = tid; i < n; i += nt) {
-    double li = lam[i];
+    const long long ki = s_key[i];
     int r = 0;
+#pragma unroll 8
     for (int j = 0; j < n; ++j) {
-      double lj = lam[j];
-      r += (lj < li) || (lj == li && j < i);
+      const long long kj = s_key[j];
+      r += (kj < ki) || (kj == ki && j < i);
     }
+    s_order[r] = i;
     order[r] = i;
+    s_val[r] = lam[i];
   }
   __syncthreads();
-  if (tid == 0) {
-    int nclus = 0, bad = 0, off = 0;
-    for (int i = 0; i < n;) {
-      int j = i;
-      while (j + 1 < n && lam[order[j + 1]] - lam[order[j]] <= delta) ++j;
-      int k = j - i + 1;
-      if (k >= 2 && k <= max_cluster) {
-        cstart[nclus] = i;
-        csize[nclus] = k;
-        coff[nclus] = off;
-        off += 2 * k * k;
-        for (int m = i; m <= j; ++m) cid[order[m]] = nclus;
-        ++nclus;
-      } else {
-        if (k > max_cluster) bad = 1;
-        for (int m = i; m <= j; ++m) cid[order[m]] = -1;
-      }
-      i = j + 1;
+  for (int i = tid; i + 1 < n; i += nt) s_near[i] = s_val[i + 1] - s_val[i] <= delta;
+  __syncthreads();
+  // a thread per cluster's first member measures it; the first warp numbers the rotated ones
+  for (int i = tid; i < n; i += nt) {
+    int k = 0;
+    if (i == 0 || !s_near[i - 1]) {
+      k = 1;
+      while (i + k < n && s_near[i + k - 1]) ++k;
     }
-    s_nclus = nclus;
-    iwork[5 * n] = nclus;
-    emax[1] = sqrt(s2) / fmax(sqrt(a2), 1e-300);
-    emax[2] = bad;
-    emax[3] = nclus;
-    emax[4] = delta;
+    s_size[i] = k;
   }
   __syncthreads();
-  const int nclus = s_nclus;
-  // cyclic Jacobi on each cluster block B = S_CC (in shared memory); W
-  // accumulates the rotations and goes to wbuf for the rotation passes
-  __shared__ double jb[kOaJacobiThreads][2 * kShCluster * kShCluster];
-  for (int c = tid; c < nclus; c += nt) {
-    const int k = csize[c], s0 = cstart[c];
-    const bool in_sh = tid < kOaJacobiThreads && k <= kShCluster;
-    double *B = in_sh ? jb[tid] : wbuf + coff[c];
-    double *W = B + k * k;
-    for (int a = 0; a < k; ++a)
-      for (int b = 0; b < k; ++b) {
-        long long ia = order[s0 + a], ib = order[s0 + b];
-        B[a * k + b] = 0.5 * (S[ia * n + ib] + S[ib * n + ia]);
-        W[a * k + b] = (a == b) ? 1.0 : 0.0;
+  if (tid < 32) {
+    int nclus = 0, off = 0, bad = 0;
+    for (int i0 = 0; i0 < n; i0 += 32) {
+      const int i = i0 + tid, k = i < n ? s_size[i] : 0;
+      const bool rotate = k >= 2 && k <= max_cluster;
+      bad |= __any_sync(0xffffffffu, k > max_cluster);
+      const unsigned mask = __ballot_sync(0xffffffffu, rotate);
+      int add = rotate ? 2 * k * k : 0;  // running sum of the blocks' sizes
+      for (int o = 1; o < 32; o <<= 1) {
+        const int v = __shfl_up_sync(0xffffffffu, add, o);
+        if (tid >= o) add += v;
       }
+      const int id = nclus + __popc(mask & ((1u << tid) - 1));
+      if (rotate) {
+        cstart[id] = i;
+        csize[id] = k;
+        coff[id] = off + add - 2 * k * k;
+      }
+      if (i < n) s_id[i] = k ? (rotate ? id : -1) : -2;  // -2: a member, not the first
+      nclus += __popc(mask);
+      off += __shfl_sync(0xffffffffu, add, 31);
+    }
+    if (tid == 0) {
+      iwork[5 * n] = nclus;
+      emax[1] = sqrt(s2) / fmax(sqrt(a2), 1e-300);
+      emax[2] = bad;
+      emax[3] = nclus;
+      emax[4] = delta;
+    }
+  }
+  __syncthreads();
+  for (int i = tid; i < n; i += nt)
+    if (s_size[i])
+      for (int m = 0; m < s_size[i]; ++m) cid[s_order[i + m]] = s_id[i];
+}
+
+// Pass 2b: the rotations W_C, cyclic Jacobi on each cluster's block S_CC in
+// shared memory, W into wbuf.  A warp per cluster in blocks of its own, lanes
+// over the rows and columns that a rotation changes: clusters are few, so the
+// blocks spread over the SMs and a rotation costs one pass over its lines
+// where a single thread walked them.
+__global__ void __launch_bounds__(32) k_oa_jacobi(int n, const double *__restrict__ S, const int *__restrict__ iwork,
+                                                  double *__restrict__ wbuf) {
+  const int *order = iwork, *cstart = iwork + 2 * n, *csize = iwork + 3 * n, *coff = iwork + 4 * n;
+  extern __shared__ double B[];  // [k][k], then W [k][k]
+  const int nclus = iwork[5 * n], lane = threadIdx.x;
+  for (int c = blockIdx.x; c < nclus; c += gridDim.x) {
+    const int k = csize[c], s0 = cstart[c];
+    double *W = B + k * k;
+    for (int m = lane; m < k * k; m += 32) {
+      const int a = m / k, b = m % k;
+      const long long ia = order[s0 + a], ib = order[s0 + b];
+      B[m] = 0.5 * (S[ia * n + ib] + S[ib * n + ia]);
+      W[m] = (a == b) ? 1.0 : 0.0;
+    }
+    __syncwarp();
     for (int sweep = 0; sweep < 40; ++sweep) {
       double offd = 0, diag = 0;
       for (int a = 0; a < k; ++a) {
@@ -192,29 +226,29 @@ __global__ void __launch_bounds__(1024) k_oa_clusters(int n, const double *__res
       if (offd <= 1e-30 * diag || offd == 0.0) break;
       for (int a = 0; a < k - 1; ++a)
         for (int b = a + 1; b < k; ++b) {
-          double bab = B[a * k + b];
+          const double bab = B[a * k + b];
           if (bab == 0.0) continue;
-          double theta = (B[b * k + b] - B[a * k + a]) / (2.0 * bab);
-          double t = (theta >= 0 ? 1.0 : -1.0) / (fabs(theta) + sqrt(theta * theta + 1.0));
-          double cs = 1.0 / sqrt(t * t + 1.0), sn = t * cs;
-          for (int m = 0; m < k; ++m) {  // B <- B J, W <- W J
+          const double theta = (B[b * k + b] - B[a * k + a]) / (2.0 * bab);
+          const double t = (theta >= 0 ? 1.0 : -1.0) / (fabs(theta) + sqrt(theta * theta + 1.0));
+          const double cs = 1.0 / sqrt(t * t + 1.0), sn = t * cs;
+          __syncwarp();
+          for (int m = lane; m < 2 * k; m += 32) {  // B <- B J, W <- W J (W follows B)
             double x = B[m * k + a], y = B[m * k + b];
             B[m * k + a] = cs * x - sn * y;
             B[m * k + b] = sn * x + cs * y;
-            x = W[m * k + a];
-            y = W[m * k + b];
-            W[m * k + a] = cs * x - sn * y;
-            W[m * k + b] = sn * x + cs * y;
           }
-          for (int m = 0; m < k; ++m) {  // B <- J^T B
+          __syncwarp();
+          for (int m = lane; m < k; m += 32) {  // B <- J^T B
             double x = B[a * k + m], y = B[b * k + m];
             B[a * k + m] = cs * x - sn * y;
             B[b * k + m] = sn * x + cs * y;
           }
+          __syncwarp();
         }
     }
-    if (in_sh)
-      for (int m = 0; m < k * k; ++m) wbuf[coff[c] + k * k + m] = W[m];
+    __syncwarp();
+    for (int m = lane; m < k * k; m += 32) wbuf[coff[c] + k * k + m] = W[m];
+    __syncwarp();
   }
 }
 
@@ -301,37 +335,39 @@ __global__ void __launch_bounds__(kOaThreads) k_oa_update(int n, const double *_
   if (threadIdx.x == 0) atomic_max_nonneg(&red[4], em);
 }
 
-// Sort eigenpairs ascending (stable): w, and the columns of X via scratch T.
-__global__ void __launch_bounds__(1024) k_sort_eigpairs(int n, double *__restrict__ w,
-                                                        double *__restrict__ X,
-                                                        double *__restrict__ T,
-                                                        int *__restrict__ rank) {
-  const int tid = threadIdx.x, nt = blockDim.x;
-  for (int i = tid; i < n; i += nt) {
-    double li = w[i];
+// Sort eigenpairs ascending (stable): ranks and w by one block, then the
+// columns of X through the scratch T by the grid.
+__global__ void __launch_bounds__(1024) k_sort_values(int n, double *__restrict__ w, int *__restrict__ rank) {
+  extern __shared__ double s_w[];  // [n], then keys [n]
+  long long *key = reinterpret_cast<long long *>(s_w + n);
+  for (int i = threadIdx.x; i < n; i += blockDim.x) {
+    s_w[i] = w[i];
+    const long long bits = __double_as_longlong(w[i] + 0.0);
+    key[i] = bits < 0 ? bits ^ 0x7fffffffffffffffLL : bits;
+  }
+  __syncthreads();
+  for (int i = threadIdx.x; i < n; i += blockDim.x) {
+    const long long ki = key[i];
     int r = 0;
-    for (int j = 0; j < n; ++j) {
-      double lj = w[j];
-      r += (lj < li) || (lj == li && j < i);
-    }
+#pragma unroll 8
+    for (int j = 0; j < n; ++j) r += (key[j] < ki) || (key[j] == ki && j < i);
     rank[i] = r;
+    w[r] = s_w[i];
   }
-  __syncthreads();
-  for (long long k = tid; k < (long long)n * n; k += nt) {
-    int row = (int)(k / n), col = (int)(k % n);
-    T[(long long)row * n + rank[col]] = X[k];
-  }
-  __syncthreads();
-  for (long long k = tid; k < (long long)n * n; k += nt) X[k] = T[k];
-  __syncthreads();
-  for (int i = tid; i < n; i += nt) T[rank[i]] = w[i];
-  __syncthreads();
-  for (int i = tid; i < n; i += nt) w[i] = T[i];
+}
+__global__ void __launch_bounds__(kOaThreads) k_sort_columns(int n, const double *__restrict__ X,
+                                                             const int *__restrict__ rank, double *__restrict__ T) {
+  const long long k = (long long)blockIdx.x * kOaThreads + threadIdx.x;
+  if (k < (long long)n * n) T[k / n * n + rank[k % n]] = X[k];
 }
 
 static void sort_eigpairs(int n, double *w, double *X, MixedEigWork &ws, cudaStream_t st) {
-  k_sort_eigpairs<<<1, 1024, 0, st>>>(n, w, X, ws.T1, reinterpret_cast<int *>(ws.E));
+  int *rank = reinterpret_cast<int *>(ws.E);
+  k_sort_values<<<1, std::min(1024, ceil_div(n, 32) * 32), 16 * n, st>>>(n, w, rank);
   HQ_LAUNCH_CHECK();
+  k_sort_columns<<<ceil_div((long long)n * n, kOaThreads), kOaThreads, 0, st>>>(n, X, rank, ws.T1);
+  HQ_LAUNCH_CHECK();
+  HQ_CUDA(cudaMemcpyAsync(X, ws.T1, sizeof(double) * n * n, cudaMemcpyDeviceToDevice, st));
 }
 
 // Rayleigh quotients l_i = s_ii / g_ii (the eigenvalue estimates of a
@@ -391,7 +427,11 @@ static double oa_iteration(int n, const double *A, double *X, double *w, MixedEi
     if (std::getenv("HQCGB_TRACE")) fprintf(stderr, "  oa off=%.3e (converged, no update)\n", off);
     return off;
   }
-  k_oa_clusters<<<1, 1024, 0, st>>>(n, ws.S, ws.G, red, w, ws.emax, ws.iwork, ws.wbuf, max_cluster);
+  k_oa_clusters<<<1, std::min(1024, ceil_div(n, 32) * 32), n * (8 + 8 + 16), st>>>(n, ws.S, ws.G, red, w, ws.emax,
+                                                                                     ws.iwork, max_cluster);
+  HQ_LAUNCH_CHECK();
+  k_oa_jacobi<<<std::min(128, std::max(1, n / 2)), 32, 2 * max_cluster * max_cluster * sizeof(double), st>>>(
+      n, ws.S, ws.iwork, ws.wbuf);
   HQ_LAUNCH_CHECK();
   k_oa_rotate_cols<<<grid, kOaThreads, 0, st>>>(n, X, ws.S, ws.G, ws.iwork, ws.wbuf);
   HQ_LAUNCH_CHECK();
