@@ -22,6 +22,7 @@
 // rotations generated by one thread) is replaced by work that is parallel
 // over eigenvalues; the FP64 refinement then fixes what single precision
 // leaves (inaccurate vectors within clusters included).
+#include <algorithm>
 #include <cfloat>
 #include <cstdio>
 #include <cstdlib>
@@ -425,7 +426,16 @@ __global__ void __launch_bounds__(256)
   }
 }
 
-size_t eigh_f32_scratch_floats(int n) { return (size_t)n * n + 4 * (size_t)n + 8; }
+size_t eigh_f32_scratch_floats(int n) {
+  return std::max((size_t)n * n + 4 * (size_t)n + 8, eigh_ql_f32_scratch_floats(n));
+}
+
+// From this size on the reduction runs on a cluster of eight SMs: below it a
+// step's arithmetic takes less than its two cluster barriers, and seven SMs
+// are better left to other streams.  One block / cluster, the reduction at
+// n = 270: 1.57 / 0.70 ms; whole solves at 64: 0.68 / 0.67, 128: 1.25 / 1.16,
+// 190: 2.40 / 2.08.
+constexpr int kClusterN = 96;
 
 // A (n x n, destroyed) -> w ascending, V columns.  scr: eigh_f32_scratch_floats(n).
 void eigh_f32(int n, float *A, float *V, float *w, float *scr, cudaStream_t st) {
@@ -443,7 +453,10 @@ void eigh_f32(int n, float *A, float *V, float *w, float *scr, cudaStream_t st) 
     for (auto &x : ev) cudaEventCreate(&x);
   if (tr) cudaEventRecord(ev[0], st);
   const size_t smt = ((size_t)n * (n + 1) / 2 + 5 * (size_t)n) * sizeof(float);
-  if (smt <= 200 * 1024) {
+  if (n >= kClusterN && tridiag_cluster_supported(n)) {
+    // one block keeps the lower triangle where it fits its shared memory, both triangles in global memory above
+    tridiag_cluster(n, smt <= 200 * 1024, A, dg, eg, taug, hv, st);
+  } else if (smt <= 200 * 1024) {
     ensure_dyn_smem((const void *)k_tridiag_f32_smem, smt);
     k_tridiag_f32_smem<<<1, kTriSmemThreads, smt, st>>>(n, A, dg, eg, taug, hv);
   } else {

@@ -476,7 +476,8 @@ bool eigh_mixed(int n, const double *A, double *V, double *w, MixedEigWork &ws, 
   if (wide) {
     // spectra spanning many orders of magnitude with dense near-degenerate
     // groups (the overlap matrix): the QL sweep's vectors refine reliably
-    eigh_tql_f32(n, 1, ws.A32, ws.V32, ws.w32, ws.work32, ws.status, st);
+    if (tridiag_cluster_supported(n)) eigh_ql_f32(n, ws.A32, ws.V32, ws.w32, ws.work32, ws.f32scr, ws.status, st);
+    else eigh_tql_f32(n, 1, ws.A32, ws.V32, ws.w32, ws.work32, ws.status, st);
     int hs = 0;
     HQ_CUDA(cudaMemcpyAsync(&hs, ws.status, sizeof(int), cudaMemcpyDeviceToHost, st));
     HQ_CUDA(cudaStreamSynchronize(st));

@@ -182,7 +182,13 @@ void gemm_batched_rowmajor(int M, int N, int K, const double *A, int lda, long l
 // eigh_fp64.cu / eigh_mixed.cu
 void eigh_tql_f32(int n, int batch, float *A, float *V, float *w, float *work, int *status,
                   cudaStream_t st);
-size_t eigh_f32_scratch_floats(int n);
+// eigh_ql_f32.cu: the QL form over several SMs, and its reduction (n <= 512)
+bool tridiag_cluster_supported(int n);
+void tridiag_cluster(int n, bool lower, const float *A, float *dg, float *eg, float *taug, float *hv,
+                     cudaStream_t st);
+size_t eigh_ql_f32_scratch_floats(int n);
+void eigh_ql_f32(int n, const float *A, float *V, float *w, float *Zt, float *scr, int *status, cudaStream_t st);
+size_t eigh_f32_scratch_floats(int n);  // covers both
 void eigh_f32(int n, float *A, float *V, float *w, float *scr, cudaStream_t st);
 struct MixedEigWork {
   float *A32, *V32, *w32, *work32, *f32scr;
