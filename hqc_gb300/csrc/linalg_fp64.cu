@@ -9,6 +9,8 @@
 //    (hqc/pbc/scf.py:174-194)
 //  * occupations: Fermi / Gauss smearing with the reference's bisection and
 //    Newton chemical-potential searches, quirks kept (hqc/tools/smearing.py)
+#include <algorithm>
+
 #include <cublas_v2.h>
 
 #include "common.cuh"
@@ -56,7 +58,78 @@ __global__ void k_gemm(int ta, int tb, int M, int N, int K, double alpha,
   }
 }
 
-// Plain FP64 GEMMs (no diagonal) go to cuBLAS: row-major C = op(A) op(B) is
+// C = op(A) op(B), row-major, for the SCF's square and thin products: T x T
+// outputs a block, one a thread, each a single chain of multiply-adds in the
+// order of k (what cuBLAS's kernels do for these shapes as well, so the results
+// are the same bits).  The FP64 pipe takes 64 cycles a warp and instruction,
+// which hides the two shared loads; what counts is that the outputs spread
+// evenly over the SMs: cuBLAS's 32 x 32 tiles occupy 81 of them at n = 270.
+// n = 270: 82 -> 40 us (the multiply-adds take 32), n = 70: 27 -> 7.
+constexpr int kDgK = 32;
+template <int T, bool TA, bool TB>
+__global__ void __launch_bounds__(T * T)
+    k_dgemm(int M, int N, int K, const double *__restrict__ A, int lda, const double *__restrict__ B, int ldb,
+            double *__restrict__ C, int ldc) {
+  constexpr int kPer = kDgK / T;  // elements of a K chunk a thread fetches, of either operand
+  __shared__ double As[2][kDgK][T + 1], Bs[2][kDgK][T + 1];
+  const int tid = threadIdx.x, tx = tid % T, ty = tid / T;
+  const int i0 = blockIdx.y * T, j0 = blockIdx.x * T;
+  double ra[kPer], rb[kPer];
+  auto fetch = [&](int k0) {
+#pragma unroll
+    for (int q = 0; q < kPer; ++q) {
+      const int f = q * T * T + tid;
+      {  // the index that is contiguous in memory runs fastest
+        const int k = TA ? f / T : f % kDgK, i = TA ? f % T : f / kDgK;
+        ra[q] = i0 + i < M && k0 + k < K ? (TA ? A[(long long)(k0 + k) * lda + i0 + i] : A[(long long)(i0 + i) * lda + k0 + k]) : 0.0;
+      }
+      {
+        const int k = TB ? f % kDgK : f / T, j = TB ? f / kDgK : f % T;
+        rb[q] = j0 + j < N && k0 + k < K ? (TB ? B[(long long)(j0 + j) * ldb + k0 + k] : B[(long long)(k0 + k) * ldb + j0 + j]) : 0.0;
+      }
+    }
+  };
+  auto put = [&](int b) {
+#pragma unroll
+    for (int q = 0; q < kPer; ++q) {
+      const int f = q * T * T + tid;
+      As[b][TA ? f / T : f % kDgK][TA ? f % T : f / kDgK] = ra[q];
+      Bs[b][TB ? f % kDgK : f / T][TB ? f / kDgK : f % T] = rb[q];
+    }
+  };
+  double acc = 0.0;
+  fetch(0);
+  put(0);
+  for (int k0 = 0, b = 0; k0 < K; k0 += kDgK, b ^= 1) {
+    __syncthreads();
+    if (k0 + kDgK < K) fetch(k0 + kDgK);
+#pragma unroll 8
+    for (int k = 0; k < kDgK; ++k) acc = fma(As[b][k][ty], Bs[b][k][tx], acc);
+    if (k0 + kDgK < K) put(b ^ 1);
+  }
+  if (i0 + ty < M && j0 + tx < N) C[(long long)(i0 + ty) * ldc + j0 + tx] = acc;
+}
+
+// From these sizes on the products are the engine's own; smaller ones go to
+// cuBLAS, whose kernels split K there.
+constexpr int kDgMin = 28;
+static void dgemm(bool ta, bool tb, int M, int N, int K, const double *A, int lda, const double *B, int ldb, double *C,
+                  int ldc, cudaStream_t st) {
+  auto go = [&](auto kernel, int t) {
+    kernel<<<dim3(ceil_div(N, t), ceil_div(M, t)), t * t, 0, st>>>(M, N, K, A, lda, B, ldb, C, ldc);
+    HQ_LAUNCH_CHECK();
+  };
+  // tiles of 8 while those of 16 leave half of the SMs idle
+  if (ceil_div(M, 16) * ceil_div(N, 16) <= 76) {
+    if (ta) tb ? go(k_dgemm<8, true, true>, 8) : go(k_dgemm<8, true, false>, 8);
+    else tb ? go(k_dgemm<8, false, true>, 8) : go(k_dgemm<8, false, false>, 8);
+  } else {
+    if (ta) tb ? go(k_dgemm<16, true, true>, 16) : go(k_dgemm<16, true, false>, 16);
+    else tb ? go(k_dgemm<16, false, true>, 16) : go(k_dgemm<16, false, false>, 16);
+  }
+}
+
+// Other plain FP64 GEMMs (no diagonal) go to cuBLAS: row-major C = op(A) op(B) is
 // column-major C^T = op(B)^T op(A)^T.  One handle per host thread (batch
 // workers run their own threads and streams).
 static cublasHandle_t blas_handle() {
@@ -72,6 +145,10 @@ void gemm(bool ta, bool tb, int M, int N, int K, double alpha, const double *A, 
           const double *B, int ldb, const double *d, double beta, double *C, int ldc,
           cudaStream_t st) {
   HQ_STAGE(ST_GEMM_SMALL, st);
+  if (!d && alpha == 1.0 && beta == 0.0 && std::max(M, N) >= kDgMin && (std::min(M, N) >= kDgMin || K >= kDgMin)) {
+    dgemm(ta, tb, M, N, K, A, lda, B, ldb, C, ldc, st);
+    return;
+  }
   if (!d) {
     cublasHandle_t h = blas_handle();
     cublasSetStream(h, st);
