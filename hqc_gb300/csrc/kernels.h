@@ -241,9 +241,10 @@ int tc_psi_max(bool gga);
 int tc_psi_width(int nuse);
 void launch_psi_operand(const double *C, const double *occ, int nao, int nmo, int nuse, int ldk,
                         float *Yhl, cudaStream_t st);
-void launch_tc_psi_density(const float *phiT, const float *dphiT, const float *Yhl, int npsi, int ldk,
-                           long long N, double *rho, double *grho, int *err, cudaStream_t st,
-                           float *psi_out = nullptr, int psi_drain = 1);
+bool tc_psi_resident(int npsi, int ldk);  // the form that reads the AO-major arrays
+void launch_tc_psi_density(const float *phi, const float *dphi, int nao, long long ld, const float *phiT,
+                           const float *dphiT, const float *Yhl, int npsi, int ldk, long long N, double *rho,
+                           double *grho, int *err, cudaStream_t st, float *psi_out = nullptr, int psi_drain = 1);
 // forces_mixed.cu
 int force_orb_blocks(long long N);
 void launch_force_operand(const double *C, const double *occ, int nao, int nuse, int npsi,

@@ -755,7 +755,7 @@ static int kx_density(KCtx &c) {
                                                                        p->Yhl);
     HQ_LAUNCH_CHECK();
     double *dst = c0 == 0 ? p->rho : p->rhoc;
-    launch_tc_psi_density(p->XT, nullptr, p->Yhl, npsi, p->ldk2, N, dst, nullptr, p->tc_err, c.st,
+    launch_tc_psi_density(p->X32, nullptr, 2 * n, p->ld, p->XT, nullptr, p->Yhl, npsi, p->ldk2, N, dst, nullptr, p->tc_err, c.st,
                           p->psi32 + (size_t)(c0 / 32) * 64 * N, 2);
     if (c0 > 0) {
       k_kx_add<<<ceil_div(N, 256), 256, 0, c.st>>>(N, p->rhoc, p->rho);

@@ -192,6 +192,7 @@ struct hqcgb_plan {
   bool mixed = false;
   long long ld = 0;
   float *dphiT32 = nullptr, *Yhl = nullptr;  // grid-major AO gradients; split Y^T
+  bool phiT_ready = false;                   // phiT32, dphiT32 hold this geometry
   double *ovq = nullptr;                     // lattice sums of the S/T Hermite products
   bool allow_warm = false;                   // warm eigen-refinement after the DIIS warm-up
   // mixed path: occupied block Y = C_occ sqrt(f) (n x nuse_dm) when few
@@ -783,6 +784,20 @@ static void exchange_gradient(Ctx &c, double *grad) {
   }
 }
 
+// The grid-major copies of phi and its gradient, once per geometry, for the
+// density forms that read them (many orbitals or AOs).
+static void grid_major(Ctx &c) {
+  hqcgb_plan *p = c.p;
+  if (p->phiT_ready) return;
+  const int n = p->nao;
+  launch_transpose_phi(p->phi32, n, p->N, p->ld, p->phiT32, c.st);
+  if (p->gga)
+    for (int d = 0; d < 3; ++d)
+      launch_transpose_phi(p->dphi32 + (size_t)d * n * p->ld, n, p->N, p->ld,
+                           p->dphiT32 + (size_t)d * p->N * tc_ldk(n), c.st);
+  p->phiT_ready = true;
+}
+
 // Two-electron part of the Fock matrix and the energy pieces for density D.
 // Leaves F = H + F2e in p->F; scalars in p->scal.
 static double fock(Ctx &c) {
@@ -803,8 +818,9 @@ static double fock(Ctx &c) {
       float *psi_out = p->keep_psi ? p->psi32 : nullptr;
       if (p->exx_fused && !psi_out) psi_out = static_cast<float *>(p->exx_psi);
       launch_psi_operand(p->C, p->occ, n, n, nuse, tc_ldk(n), p->Yhl, c.st);
-      launch_tc_psi_density(p->phiT32, p->dphiT32, p->Yhl, tc_psi_width(nuse), tc_ldk(n), N, p->rho,
-                            p->gga ? p->grho : nullptr, p->tc_err, c.st, psi_out, kPsiDrain);
+      if (!tc_psi_resident(tc_psi_width(nuse), tc_ldk(n))) grid_major(c);
+      launch_tc_psi_density(p->phi32, p->dphi32, n, p->ld, p->phiT32, p->dphiT32, p->Yhl, tc_psi_width(nuse),
+                            tc_ldk(n), N, p->rho, p->gga ? p->grho : nullptr, p->tc_err, c.st, psi_out, kPsiDrain);
       p->exx_psi_ready = p->exx_fused && psi_out == p->exx_psi;
       if (p->keep_psi) {
         p->npsi_kept = tc_psi_width(nuse);
@@ -813,6 +829,7 @@ static double fock(Ctx &c) {
     } else {
       if (p->keep_psi) p->npsi_kept = 0;
       launch_to_f32(p->D, n, n, n, 1.0, p->D32, tc_ldk(n), c.st);
+      grid_major(c);
       launch_tc_density(p->phi32, p->phiT32, p->dphi32, p->D32, n, N, p->ld, p->tcd_part, p->rho,
                         p->gga ? p->grho : nullptr, p->tc_err, c.st);
     }
@@ -906,11 +923,7 @@ static void geometry(Ctx &c, const double *xp_dev) {
                  p->dphi32, c.st);
     // phi split once per geometry into the TF32 pieces the quadrature reads
     launch_split_operand(p->phi32, nullptr, nullptr, nullptr, n, N, p->ld, p->ld, 1.f, 0.f, p->phihl, c.st);
-    launch_transpose_phi(p->phi32, n, N, p->ld, p->phiT32, c.st);
-    if (p->gga)
-      for (int d = 0; d < 3; ++d)
-        launch_transpose_phi(p->dphi32 + (size_t)d * n * p->ld, n, N, p->ld,
-                             p->dphiT32 + (size_t)d * N * tc_ldk(n), c.st);
+    p->phiT_ready = false;
   }
   // The SCF's S and T keep the sums vector by vector: a nearly dependent basis
   // multiplies a change in the last digit of S by cond(S), 1e7 for dzvp in a

@@ -610,8 +610,6 @@ constexpr size_t kPsiStageBytes = kPsiAPieces + 2 * kPsiBPiece;  // 48 KB
 constexpr size_t kPsiSmem = kPsiRing * kPsiStageBytes + 1024;
 
 struct PsiArgs {
-  const float *phiT;   // [N][ldk]
-  const float *dphiT;  // [3][N][ldk] (GGA) or null
   const float *Yhl;    // [2][npsi][ldk]: TF32 hi and lo pieces of Y^T
   long long N;
   int ldk, npsi, ncomp;
@@ -865,10 +863,15 @@ __global__ void __launch_bounds__(kPsiThreads, 1)
 // bytes are in flight per SM.
 //  * Y^T (both TF32 pieces, every K block) is loaded once per CTA and stays
 //    in shared memory (npsi x ldk x 8 B, 72 KB at npsi = 32, 288 AOs).
-//  * The TMA ring holds only raw fp32 A boxes (16 KB each, kPsrRing deep);
-//    the splitter warps copy a box into one of two split buffers as TF32
-//    hi/lo pieces and release the ring slot at once, so a slot is busy for
-//    the load latency plus one read rather than until its MMAs complete.
+//  * The TMA ring holds only raw fp32 A boxes (32 AOs x 128 points, 16 KB each,
+//    kPsrRing deep) of the AO-major arrays phi and grad phi as the SCF keeps
+//    them; the splitter warps turn a box into K-major rows of TF32 hi/lo
+//    pieces in one of two split buffers and release the ring slot at once, so a
+//    slot is busy for the load latency plus one read rather than until its
+//    MMAs complete.  Reading a box down its columns costs four times the
+//    shared loads of a row, and saves the
+//    grid-major copies: H54 shapes 0.764 -> 0.793 ms a launch, and four
+//    transpositions of 0.36 ms a geometry or call less.
 //  * The MMA reads A from the split buffer and B from the resident Y.
 // ---------------------------------------------------------------------------
 constexpr int kPsrMaxN = 32;
@@ -950,32 +953,28 @@ __global__ void __launch_bounds__(kPsiThreads, 1)
         const int g0 = (int)((blockIdx.x + t * gridDim.x) * (long long)kM);
         const uint32_t dst = smem_u32(raw + slot * kTile);
         mbar_expect_tx(&P.raw_full[slot], (uint32_t)kTile);
-        if (comp == 0) tma_load_3d(dst, &tmA, 0, g0, kb, &P.raw_full[slot]);
-        else tma_load_3d(dst, &tmD, 0, g0, (comp - 1) * nkb + kb, &P.raw_full[slot]);
+        if (comp == 0) tma_load_3d(dst, &tmA, g0, kb * kStageK, 0, &P.raw_full[slot]);
+        else tma_load_3d(dst, &tmD, g0, kb * kStageK, comp - 1, &P.raw_full[slot]);
       }
     }
   } else if (warp < kPsiPW) {
-    // splitters: raw box -> TF32 hi / lo pieces in the split buffer st % 2
-    const int cch = tid & 7;
+    // splitters: raw box -> TF32 hi / lo pieces in the split buffer st % 2, a
+    // thread per grid point: it reads its point's 32 AO values down the box
+    // (neighbouring lanes, neighbouring points) and writes them as a K-major row
     for (long long st = 0; st < S; ++st) {
       const int slot = (int)(st % kPsrRing), sb = (int)(st & 1);
       if (ok && !mbar_wait(&P.raw_full[slot], (unsigned)((st / kPsrRing) & 1), a.err, 51)) ok = false;
       if (ok && st >= 2 && !mbar_wait(&P.sp_empty[sb], (unsigned)(((st >> 1) - 1) & 1), a.err, 52)) ok = false;
       if (ok) {
-        const char *src = raw + slot * kTile;
+        const float *src = reinterpret_cast<const float *>(raw + slot * kTile) + tid;
         char *dst = spl + sb * 2 * kTile;
-        float4 v[kPsiRowsPerThread];
+        float v[kStageK];
 #pragma unroll
-        for (int j = 0; j < kPsiRowsPerThread; ++j) {
-          const int row = (tid >> 3) + (kPsiProducers / 8) * j;
-          v[j] = *reinterpret_cast<const float4 *>(src + swz(row, cch));
-        }
+        for (int k = 0; k < kStageK; ++k) v[k] = src[k * kM];
         mbar_arrive(&P.raw_empty[slot]);  // the box is in registers: the slot can be refilled
 #pragma unroll
-        for (int j = 0; j < kPsiRowsPerThread; ++j) {
-          const int row = (tid >> 3) + (kPsiProducers / 8) * j;
-          store_split4(dst, row, cch, v[j]);
-        }
+        for (int c = 0; c < kStageK / 4; ++c)
+          store_split4(dst, tid, c, make_float4(v[4 * c], v[4 * c + 1], v[4 * c + 2], v[4 * c + 3]));
       } else {
         mbar_arrive(&P.raw_empty[slot]);
       }
@@ -1811,6 +1810,30 @@ CUtensorMap tensor_map_3d_kblk(const float *base, long long rows, long long nkb,
   if (r != CUDA_SUCCESS) throw Error{HQCGB_CUDA_ERROR, "cuTensorMapEncodeTiled (3D) failed"};
   return m;
 }
+// AO-major fp32 values [comps][rows][ld] of N grid points as a map (x: the
+// point, y: the AO, z: the component) with unswizzled boxes of 128 points x 32
+// AOs; points from N on and AOs from `rows` on read as zero.
+CUtensorMap tensor_map_ao(const float *base, long long N, long long rows, long long comps, long long ld) {
+  static const PFN_cuTensorMapEncodeTiled_v12000 encode = [] {
+    void *fn = nullptr;
+    cudaDriverEntryPointQueryResult q;
+    HQ_CUDA(cudaGetDriverEntryPointByVersion("cuTensorMapEncodeTiled", &fn, 12000, cudaEnableDefault, &q));
+    HQ_REQUIRE(fn && q == cudaDriverEntryPointSuccess, "cuTensorMapEncodeTiled unavailable");
+    return reinterpret_cast<PFN_cuTensorMapEncodeTiled_v12000>(fn);
+  }();
+  HQ_REQUIRE(((uintptr_t)base & 15) == 0, "TMA base must be 16-byte aligned");
+  HQ_REQUIRE(ld % 4 == 0 && N >= 1 && N <= ld && rows >= 1, "TMA extents out of range");
+  CUtensorMap m;
+  cuuint64_t dims[3] = {(cuuint64_t)N, (cuuint64_t)rows, (cuuint64_t)comps};
+  cuuint64_t strides[2] = {(cuuint64_t)ld * sizeof(float), (cuuint64_t)rows * ld * sizeof(float)};
+  cuuint32_t box[3] = {(cuuint32_t)kM, (cuuint32_t)kStageK, 1};
+  cuuint32_t estr[3] = {1, 1, 1};
+  CUresult r = encode(&m, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 3, const_cast<float *>(base), dims, strides,
+                      box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
+                      CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  if (r != CUDA_SUCCESS) throw Error{HQCGB_CUDA_ERROR, "cuTensorMapEncodeTiled (AO) failed"};
+  return m;
+}
 }  // namespace tc
 
 // ---------------------------------------------------------------------------
@@ -1824,10 +1847,18 @@ void launch_psi_operand(const double *C, const double *occ, int nao, int nmo, in
   HQ_LAUNCH_CHECK();
 }
 
-// rho (and grad rho) from the grid-major AO values and the pre-split Y^T.
-void launch_tc_psi_density(const float *phiT, const float *dphiT, const float *Yhl, int npsi, int ldk,
-                           long long N, double *rho, double *grho, int *err, cudaStream_t st,
-                           float *psi_out, int psi_drain) {
+// The resident-Y form applies: Y^T fits its shared-memory region (knob
+// "psi_ring" = 1 selects the ring form for comparison).
+bool tc_psi_resident(int npsi, int ldk) {
+  return npsi <= tc::kPsrMaxN && tc::psr_y_bytes(npsi, ldk) <= tc::kPsrYMax && tune_get("psi_ring", 0) == 0;
+}
+
+// rho (and grad rho) from the AO values and the pre-split Y^T: the AO-major
+// phi [nao][ld] and dphi [3][nao][ld] (16-byte aligned, ld % 4 == 0) in the
+// resident-Y form, the grid-major K-blocked copies phiT and dphiT otherwise.
+void launch_tc_psi_density(const float *phi, const float *dphi, int nao, long long ld, const float *phiT,
+                           const float *dphiT, const float *Yhl, int npsi, int ldk, long long N, double *rho,
+                           double *grho, int *err, cudaStream_t st, float *psi_out, int psi_drain) {
   HQ_REQUIRE(psi_drain >= 1, "drain interval must be >= 1");
   HQ_STAGE(ST_PSI, st);
   HQ_REQUIRE(npsi >= 16 && npsi <= tc::kPsiMaxN && npsi % 16 == 0, "orbital count out of range");
@@ -1844,25 +1875,19 @@ void launch_tc_psi_density(const float *phiT, const float *dphiT, const float *Y
   ensure_dyn_smem((const void *)tc::k_tc_psi_density<48>, tc::kPsiSmem);
   ensure_dyn_smem((const void *)tc::k_tc_psi_density<64>, tc::kPsiSmem);
   tc::PsiArgs a;
-  a.phiT = phiT; a.dphiT = grho ? dphiT : nullptr; a.Yhl = Yhl; a.N = N; a.ldk = ldk;
+  a.Yhl = Yhl; a.N = N; a.ldk = ldk;
   a.npsi = npsi; a.ncomp = grho ? 4 : 1; a.rho = rho; a.grho = grho; a.err = err;
   a.psi_out = psi_out;
   a.drain = psi_drain;
-  HQ_REQUIRE(!grho || dphiT, "GGA density needs the gradient operand");
+  const bool resident = tc_psi_resident(npsi, ldk);
+  HQ_REQUIRE(!grho || (resident ? dphi : dphiT), "GGA density needs the gradient operand");
   HQ_REQUIRE(N <= (1LL << 29), "grid too large for 32-bit TMA row coordinates");
-  // boxes of 32 fp32 (128 B, the swizzle span) x rows; row strides ldk * 4 B
-  // phiT / dphiT are K-blocked ([component][AO block][g][32]): 3D maps whose
-  // 128-point x 32-AO boxes are contiguous
-  CUtensorMap tmA = tc::tensor_map_3d_kblk(phiT, N, ldk / tc::kStageK, tc::kM);
-  CUtensorMap tmD = tc::tensor_map_3d_kblk(grho ? dphiT : phiT, N, (grho ? 3 : 1) * (ldk / tc::kStageK), tc::kM);
   CUtensorMap tmY = tc::tensor_map_2d(Yhl, ldk, 2LL * npsi, npsi);
   long long ntiles = ceil_div(N, tc::kM);
   int grid = (int)std::min<long long>(ntiles, nsm);
-  // resident-Y form when Y^T fits its shared-memory region (knob
-  // "psi_ring" = 1 selects the ring form for comparison)
-  const bool resident = npsi <= tc::kPsrMaxN && tc::psr_y_bytes(npsi, ldk) <= tc::kPsrYMax &&
-                        tune_get("psi_ring", 0) == 0;
   if (resident) {
+    const CUtensorMap tmA = tc::tensor_map_ao(phi, N, nao, 1, ld),
+                      tmD = tc::tensor_map_ao(grho ? dphi : phi, N, nao, grho ? 3 : 1, ld);
     ensure_dyn_smem((const void *)tc::k_tc_psi_density_r<16>, tc::kPsrSmem);
     ensure_dyn_smem((const void *)tc::k_tc_psi_density_r<32>, tc::kPsrSmem);
     if (npsi == 16) tc::k_tc_psi_density_r<16><<<grid, tc::kPsiThreads, tc::kPsrSmem, st>>>(a, tmA, tmD, tmY);
@@ -1870,6 +1895,11 @@ void launch_tc_psi_density(const float *phiT, const float *dphiT, const float *Y
     HQ_LAUNCH_CHECK();
     return;
   }
+  // boxes of 32 fp32 (128 B, the swizzle span) x rows; row strides ldk * 4 B
+  // phiT / dphiT are K-blocked ([component][AO block][g][32]): 3D maps whose
+  // 128-point x 32-AO boxes are contiguous
+  CUtensorMap tmA = tc::tensor_map_3d_kblk(phiT, N, ldk / tc::kStageK, tc::kM);
+  CUtensorMap tmD = tc::tensor_map_3d_kblk(grho ? dphiT : phiT, N, (grho ? 3 : 1) * (ldk / tc::kStageK), tc::kM);
   switch (npsi) {
     case 16: tc::k_tc_psi_density<16><<<grid, tc::kPsiThreads, tc::kPsiSmem, st>>>(a, tmA, tmD, tmY); break;
     case 32: tc::k_tc_psi_density<32><<<grid, tc::kPsiThreads, tc::kPsiSmem, st>>>(a, tmA, tmD, tmY); break;
@@ -2269,19 +2299,34 @@ extern "C" int hqcgb_tc_orbital_density(int nao, long long N, long long ld, cons
     HQ_REQUIRE((dphi == nullptr) == (grho == nullptr), "dphi and grho go together");
     int ldk = tc_ldk(nao);
     int ncomp = dphi ? 4 : 1;
-    StreamBuf phiT_buf((size_t)ncomp * N * ldk * sizeof(float), st),
-        Yhl_buf((size_t)2 * tc_psi_max(false) * ldk * sizeof(float), st), err_buf(sizeof(int), st);
-    float *phiT = phiT_buf.as<float>(), *Yhl = Yhl_buf.as<float>();
+    StreamBuf Yhl_buf((size_t)2 * tc_psi_max(false) * ldk * sizeof(float), st), err_buf(sizeof(int), st);
+    float *Yhl = Yhl_buf.as<float>();
     int *err = err_buf.as<int>();
     HQ_CUDA(cudaMemsetAsync(err, 0, sizeof(int), st));
-    launch_transpose_phi(phi, nao, N, ld, phiT, st);
-    if (dphi)
-      for (int d = 0; d < 3; ++d)
-        launch_transpose_phi(dphi + (size_t)d * nao * ld, nao, N, ld, phiT + (size_t)(d + 1) * N * ldk,
-                             st);
     launch_psi_operand(C, occ, nao, nmo, nuse, ldk, Yhl, st);
-    launch_tc_psi_density(phiT, dphi ? phiT + (size_t)N * ldk : nullptr, Yhl, tc_psi_width(nuse), ldk,
-                          N, rho, grho, err, st, nullptr, drain);
+    // what the resident-Y form cannot take goes through a copy: grid-major
+    // for more orbitals or AOs, aligned for TMA otherwise
+    const int npsi = tc_psi_width(nuse);
+    const bool rows = tc_psi_resident(npsi, ldk), aligned = (((uintptr_t)phi | (uintptr_t)dphi) & 15) == 0;
+    const size_t field = (size_t)nao * ld * sizeof(float);
+    StreamBuf copy(rows ? (aligned ? 16 : ncomp * field) : (size_t)ncomp * N * ldk * sizeof(float), st);
+    float *phiT = copy.as<float>();
+    if (!rows) {
+      launch_transpose_phi(phi, nao, N, ld, phiT, st);
+      if (dphi)
+        for (int d = 0; d < 3; ++d)
+          launch_transpose_phi(dphi + (size_t)d * nao * ld, nao, N, ld, phiT + (size_t)(d + 1) * N * ldk,
+                               st);
+    } else if (!aligned) {
+      HQ_CUDA(cudaMemcpyAsync(phiT, phi, field, cudaMemcpyDeviceToDevice, st));
+      phi = phiT;
+      if (dphi) {
+        HQ_CUDA(cudaMemcpyAsync(phiT + (size_t)nao * ld, dphi, 3 * field, cudaMemcpyDeviceToDevice, st));
+        dphi = phiT + (size_t)nao * ld;
+      }
+    }
+    launch_tc_psi_density(phi, dphi, nao, ld, phiT, dphi ? phiT + (size_t)N * ldk : nullptr, Yhl, npsi, ldk, N, rho,
+                          grho, err, st, nullptr, drain);
     int h = 0;
     HQ_CUDA(cudaMemcpyAsync(&h, err, sizeof(int), cudaMemcpyDeviceToHost, st));
     HQ_CUDA(cudaStreamSynchronize(st));
