@@ -203,6 +203,12 @@ bool eigh_mixed_warm(int n, const double *A, const double *X0, double *V, double
 bool eigh_mixed(int n, const double *A, double *V, double *w, MixedEigWork &ws, cudaStream_t st,
                 bool wide = false, EigLevel level = EigLevel::Full);
 
+// poisson_f64.cu: dst = DFT^-1[kern DFT[src]] of a real field on an odd grid;
+// cbuf holds n n (n + 1) / 2 values, kern as launch_coulomb_table
+bool poisson_f64_supported(int n);
+void launch_poisson_f64(const double *src, double *dst, double2 *cbuf, const double *kern, int n, const double2 *tw,
+                        cudaStream_t st);
+
 // fft (FP32 transforms)
 void launch_fft3d_f32(float2 *c, int ng, int batch, const double2 *tw, bool inverse,
                       cudaStream_t st);

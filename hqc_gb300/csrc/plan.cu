@@ -650,11 +650,14 @@ static void density_matrix(Ctx &c) {
   gemm(false, true, n, n, n, 1.0, p->C, n, p->C, n, p->occ, 0.0, p->D, n, c.st);
 }
 
-static void poisson(Ctx &c, const double *src, double *dst, bool keep_spectrum = false) {
+static void poisson(Ctx &c, const double *src, double *dst) {
   hqcgb_plan *p = c.p;
+  if (poisson_f64_supported(p->ng)) {
+    launch_poisson_f64(src, dst, p->cbuf, p->coul, p->ng, p->tw, c.st);
+    return;
+  }
   launch_real_to_complex(src, nullptr, p->N, 1, p->cbuf, c.st);
   launch_fft3d(p->cbuf, p->ng, 1, p->tw, false, c.st);
-  (void)keep_spectrum;
   launch_scale_complex(p->cbuf, p->coul, p->N, 1, c.st);
   launch_fft3d(p->cbuf, p->ng, 1, p->tw, true, c.st);
   launch_complex_real(p->cbuf, p->N, 1.0, dst, c.st);
