@@ -22,7 +22,7 @@ namespace hqcgb {
 __device__ inline void hermite6(double mu, double x, double *h) {
   h[0] = 1.0;
   h[1] = -2.0 * mu * x;
-  for (int k = 1; k < 5; ++k) h[k + 1] = -2.0 * mu * x * h[k] - 2.0 * k * mu * h[k - 1];
+  for (int k = 1; k < 5; ++k) h[k + 1] = __fma_rn(h[1], h[k], -(2.0 * k * mu * h[k - 1]));
 }
 
 struct AOInfo {
@@ -59,19 +59,35 @@ __device__ inline int midx_of(int m0, int m1, int m2) {
   return 0;
 }
 
-// The general form, for any list of lattice vectors.
-// KPT: each lattice term also carries exp(-i k.t) (hqc/pbc/solver.py:257-274);
-// the real and imaginary sums are stored side by side, Q[(i,j,a,b)][4][kNq] =
-// {QS re, QT re, QS im, QT im}.
+// The general form, for any list of lattice vectors, one warp per sum.  The
+// lanes take one vector each: they drop the images beyond exp(-60), queue the
+// others in their order, and form the exponential and the Hermite products of 32
+// queued vectors in shared memory; then lane s adds the s-th of the 2 NQ sums
+// (4 NQ at a k-point) over the 32 vectors in that order, so that the sums are
+// those of one thread going through the list (the multiply-adds are written
+// out, so that no compiler choice moves them).  KPT: each lattice term also
+// carries exp(-i k.t) (hqc/pbc/solver.py:257-274); the real and imaginary sums
+// are stored side by side, Q[(i,j,a,b)][4][kNq] = {QS re, QT re, QS im, QT im}.
+// Bound by the FP64 pipe (some 200 instructions a vector kept).  With a thread a
+// sum a small molecule left most of the chip idle: H8 szv has 576 to 2,304 sums
+// of 870 vectors.  Measured, S and T of one configuration, a thread -> a warp a
+// sum: H8 szv (box 4.1 Bohr) 4.71 -> 0.21 ms, H8 dzv
+// at a k-point 4.37 -> 0.23.
 template <int NQ, bool KPT>
-__global__ void k_ovl_lattice(const double *__restrict__ xp, int n, int nprim,
-                              const double *__restrict__ alpha, const double *__restrict__ lattice,
-                              int nlat, const double *__restrict__ kpt, double *__restrict__ Q) {
-  const long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+__global__ void __launch_bounds__(128)
+    k_ovl_lattice(const double *__restrict__ xp, int n, int nprim, const double *__restrict__ alpha,
+                  const double *__restrict__ lattice, int nlat, const double *__restrict__ kpt,
+                  double *__restrict__ Q) {
+  constexpr int NH = 2 * NQ, NS = KPT ? 2 * NH : NH, ROW = NH + (KPT ? 3 : 1);  // odd rows: no bank conflicts
+  constexpr int NR = (NS + 31) / 32;
+  __shared__ double val[4][32][ROW];  // a vector's products S, T; exponential (re, im)
+  __shared__ int queue[4][64];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const long long idx = (long long)blockIdx.x * 4 + warp;
   const int np2 = nprim * nprim;
   if (idx >= (long long)n * n * np2) return;
-  // atom pairs fastest: a warp shares one primitive pair (one mu), so its
-  // lanes skip the same far lattice terms
+  // atom pairs fastest: the warps of a block share one primitive pair (one mu),
+  // so they keep about as many vectors
   const int ab = (int)(idx / ((long long)n * n)), a = ab / nprim, b = ab % nprim;
   const int ij = (int)(idx % ((long long)n * n)), i = ij / n, j = ij % n;
   double R[3];
@@ -79,58 +95,79 @@ __global__ void k_ovl_lattice(const double *__restrict__ xp, int n, int nprim,
   const double asum = alpha[a] + alpha[b];
   const double mu = alpha[a] * alpha[b] / asum;
   const double K = pow(M_PI / asum, 1.5);
-  double qs[NQ], qt[NQ], qsi[KPT ? NQ : 1], qti[KPT ? NQ : 1];
-#pragma unroll
-  for (int k = 0; k < NQ; ++k) qs[k] = qt[k] = 0.0;
-  if (KPT)
-#pragma unroll
-    for (int k = 0; k < NQ; ++k) qsi[k] = qti[k] = 0.0;
-  for (int t = 0; t < nlat; ++t) {
-    double u[3], u2 = 0;
+  int *q = queue[warp];
+  auto exponent = [&](int t, double (&u)[3]) {
+    double u2 = 0;
     for (int d = 0; d < 3; ++d) {
       u[d] = R[d] + lattice[t * 3 + d];
       u2 += u[d] * u[d];
     }
-    double e = mu * u2;
-    // exp(-60) times the largest Hermite factor (degree <= 5) is below 1e-18
-    // of every matrix element: far images add nothing in FP64
-    if (e > 60.0) continue;
-    e = K * exp(-e);
-    double ei = 0.0;
-    if (KPT) {
-      double sn, cs;
-      sincos(-(kpt[0] * lattice[t * 3] + kpt[1] * lattice[t * 3 + 1] + kpt[2] * lattice[t * 3 + 2]),
-             &sn, &cs);
-      ei = e * sn;
-      e *= cs;
-    }
-    double hx[6], hy[6], hz[6];
-    hermite6(mu, u[0], hx);
-    hermite6(mu, u[1], hy);
-    hermite6(mu, u[2], hz);
+    return mu * u2;
+  };
+  double acc[NR];
 #pragma unroll
-    for (int k = 0; k < NQ; ++k) {
-      const int m0 = kMidx[k][0], m1 = kMidx[k][1], m2 = kMidx[k][2];
-      const double hs = hx[m0] * hy[m1] * hz[m2];
-      const double ht = hx[m0 + 2] * hy[m1] * hz[m2] + hx[m0] * hy[m1 + 2] * hz[m2] +
-                        hx[m0] * hy[m1] * hz[m2 + 2];
-      qs[k] += e * hs;
-      qt[k] += e * ht;
+  for (int r = 0; r < NR; ++r) acc[r] = 0.0;
+  auto add = [&](int m) {  // the first m <= 32 queued vectors
+    if (lane < m) {
+      double *row = val[warp][lane];
+      const int t = q[lane];
+      double u[3];
+      const double e0 = exponent(t, u);
+      double e = K * exp(-e0);
       if (KPT) {
-        qsi[k] += ei * hs;
-        qti[k] += ei * ht;
+        double sn, cs;
+        const double *tv = lattice + t * 3;
+        sincos(-__fma_rn(kpt[2], tv[2], __fma_rn(kpt[0], tv[0], kpt[1] * tv[1])), &sn, &cs);
+        row[NH + 1] = e * sn;
+        e *= cs;
+      }
+      row[NH] = e;
+      double hx[6], hy[6], hz[6];
+      hermite6(mu, u[0], hx);
+      hermite6(mu, u[1], hy);
+      hermite6(mu, u[2], hz);
+#pragma unroll
+      for (int k = 0; k < NQ; ++k) {
+        const int m0 = midx(k, 0), m1 = midx(k, 1), m2 = midx(k, 2);
+        row[k] = hx[m0] * hy[m1] * hz[m2];
+        row[NQ + k] = __fma_rn(hx[m0] * hy[m1], hz[m2 + 2],
+                               __fma_rn(hx[m0 + 2] * hy[m1], hz[m2], hx[m0] * hy[m1 + 2] * hz[m2]));
       }
     }
+    __syncwarp();
+    for (int v = 0; v < m; ++v) {
+#pragma unroll
+      for (int r = 0; r < NR; ++r) {
+        const int s = lane + 32 * r;
+        if (s < NS) acc[r] = fma(val[warp][v][NH + s / NH], val[warp][v][s % NH], acc[r]);
+      }
+    }
+    __syncwarp();
+  };
+  int have = 0;
+  for (int t0 = 0; t0 < nlat; t0 += 32) {
+    const int t = t0 + lane;
+    double u[3];
+    // exp(-60) times the largest Hermite factor (degree <= 5) is below 1e-18
+    // of every matrix element: far images add nothing in FP64
+    const bool keep = t < nlat && !(exponent(t, u) > 60.0);
+    const unsigned mask = __ballot_sync(~0u, keep);
+    if (keep) q[have + __popc(mask & ((1u << lane) - 1u))] = t;
+    have += __popc(mask);
+    __syncwarp();
+    if (have >= 32) {
+      add(32);
+      have -= 32;
+      if (lane < have) q[lane] = q[32 + lane];
+      __syncwarp();
+    }
   }
+  if (have) add(have);
   double *out = Q + (((long long)i * n + j) * np2 + ab) * ((KPT ? 4 : 2) * kNq);
 #pragma unroll
-  for (int k = 0; k < NQ; ++k) {
-    out[k] = qs[k];
-    out[kNq + k] = qt[k];
-    if (KPT) {
-      out[2 * kNq + k] = qsi[k];
-      out[3 * kNq + k] = qti[k];
-    }
+  for (int r = 0; r < NR; ++r) {
+    const int s = lane + 32 * r;
+    if (s < NS) out[s / NQ * kNq + s % NQ] = acc[r];
   }
 }
 
@@ -471,10 +508,10 @@ void launch_overlap_kinetic(const double *xp, int n, int nb, int nprim, const do
   else if (rows.tmax >= 0)
     k_ovl_rows<10, double><<<blocks, 32, 0, st>>>(xp, n, nprim, alpha, rows, nullptr, Q);
   else if (gpart)
-    k_ovl_lattice<20, false><<<ceil_div(terms, 128), 128, 0, st>>>(xp, n, nprim, alpha, lattice, nlat,
+    k_ovl_lattice<20, false><<<ceil_div(terms, 4), 128, 0, st>>>(xp, n, nprim, alpha, lattice, nlat,
                                                                    nullptr, Q);
   else
-    k_ovl_lattice<10, false><<<ceil_div(terms, 128), 128, 0, st>>>(xp, n, nprim, alpha, lattice, nlat,
+    k_ovl_lattice<10, false><<<ceil_div(terms, 4), 128, 0, st>>>(xp, n, nprim, alpha, lattice, nlat,
                                                                    nullptr, Q);
   HQ_LAUNCH_CHECK();
   const long long total = (long long)n * n * nb * nb;
@@ -501,10 +538,10 @@ void launch_overlap_kinetic_kpt(const double *xp, int n, int nb, int nprim, cons
   else if (rows.tmax >= 0)
     k_ovl_rows<10, double2><<<blocks, 32, 0, st>>>(xp, n, nprim, alpha, rows, kpt, Q);
   else if (gpart)
-    k_ovl_lattice<20, true><<<ceil_div(terms, 128), 128, 0, st>>>(xp, n, nprim, alpha, lattice, nlat,
+    k_ovl_lattice<20, true><<<ceil_div(terms, 4), 128, 0, st>>>(xp, n, nprim, alpha, lattice, nlat,
                                                                   kpt, Q);
   else
-    k_ovl_lattice<10, true><<<ceil_div(terms, 128), 128, 0, st>>>(xp, n, nprim, alpha, lattice, nlat,
+    k_ovl_lattice<10, true><<<ceil_div(terms, 4), 128, 0, st>>>(xp, n, nprim, alpha, lattice, nlat,
                                                                   kpt, Q);
   HQ_LAUNCH_CHECK();
   const long long total = (long long)n * n * nb * nb;
