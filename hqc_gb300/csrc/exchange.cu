@@ -141,7 +141,7 @@ __global__ void __launch_bounds__(256, exx_min_blocks<R>()) k_exx_plane(PlaneArg
   __syncthreads();
   // z transform of the packed lines, then unpacked into C[y][kz], kz < nh:
   // A[k] = (Z[k] + conj Z[n-k]) / 2 (line 2 pr), B[k] = (Z[k] - conj Z[n-k]) / 2i
-  R2 *Zt = dft_axis0<R, R2>(B0, B1, B0, n, npair, a.n1, w);
+  R2 *Zt = dft_axis0<R, R2>(B0, B1, n, npair, a.n1, w);
   R2 *Cb = (Zt == B0) ? B1 : B0;
   for (int i = threadIdx.x; i < npair * nh; i += blockDim.x) {
     const int pr = i / nh, kz = i - pr * nh;
@@ -156,7 +156,7 @@ __global__ void __launch_bounds__(256, exx_min_blocks<R>()) k_exx_plane(PlaneArg
   }
   __syncthreads();
   R2 *Ct = (Cb == B0) ? B1 : B0;
-  const R2 *res = dft_axis0<R, R2>(Cb, Ct, Cb, n, nh, a.n1, w);
+  const R2 *res = dft_axis0<R, R2>(Cb, Ct, n, nh, a.n1, w);
   R2 *T = reinterpret_cast<R2 *>(a.T) + (((long long)jl * a.rows + r) * n + x) * (long long)n * nh;
   for (int i = threadIdx.x; i < n * nh; i += blockDim.x) T[i] = res[i];
 }
@@ -203,7 +203,7 @@ __global__ void __launch_bounds__(256, OUT == 2 ? 1 : exx_min_blocks<R>()) k_exx
   };
   if (OUT != 2) {
     load_line(r, B0);
-    const R2 *res = dft_axis0<R, R2>(B0, B1, B0, n, nh, a.n1, w);
+    const R2 *res = dft_axis0<R, R2>(B0, B1, n, nh, a.n1, w);
     const long long K0 = (long long)jl * 2 * n * plane;
     for (int i = threadIdx.x; i < n * nh; i += blockDim.x) {
       const int kx = i / nh, kz = i - kx * nh;
@@ -228,12 +228,12 @@ __global__ void __launch_bounds__(256, OUT == 2 ? 1 : exx_min_blocks<R>()) k_exx
     const int p = r;
     __shared__ double red[3][8];
     load_line(p, B0);
-    const R2 *xh = dft_axis0<R, R2>(B0, B1, B0, n, nh, a.n1, w);  // in B0 or B1
+    const R2 *xh = dft_axis0<R, R2>(B0, B1, n, nh, a.n1, w);  // in B0 or B1
     R2 *spare = (xh == B0) ? B1 : B0;
     double acc[3] = {0, 0, 0};
     for (int c = 0; c < 3; ++c) {
       load_line(a.nao * (1 + c) + p, B2);
-      const R2 *dh = dft_axis0<R, R2>(B2, spare, B2, n, nh, a.n1, w);
+      const R2 *dh = dft_axis0<R, R2>(B2, spare, n, nh, a.n1, w);
       for (int i = threadIdx.x; i < n * nh; i += blockDim.x) {
         const int kx = i / nh, kz = i - kx * nh;
         const double s = (double)wsq[(long long)kx * n * nh + kz];

@@ -209,6 +209,18 @@ bool poisson_f64_supported(int n);
 void launch_poisson_f64(const double *src, double *dst, double2 *cbuf, const double *kern, int n, const double2 *tw,
                         cudaStream_t st);
 
+// exchange_kpt.cu: FP64 grid contractions of a k-point plan (odd grids).
+// W[j][p] = sqrt(f_j) sqcoul DFT[phi_p conj(psi_j)] for g <= kKxGroup orbitals;
+// M (+)= alpha sum over `sets` and N points of A_p conj(B_q), rows N apart,
+// sets sA / sB apart, herm where the result is Hermitian (P: zgram_scratch).
+constexpr int kKxGroup = 16;
+int kx_group(int nao, long long N);
+void launch_kx_pairs(const double2 *phi, const double2 *psi, const double *f, int g, const double *sqcoul, int n,
+                     int nao, const double2 *tw, double2 *W, cudaStream_t st);
+size_t zgram_scratch(int n, int sets, long long N);
+void launch_zgram(int n, long long N, int sets, const double2 *A, long long sA, const double2 *B, long long sB,
+                  bool herm, double alpha, bool accumulate, double2 *P, double2 *M, cudaStream_t st);
+
 // fft (FP32 transforms)
 void launch_fft3d_f32(float2 *c, int ng, int batch, const double2 *tw, bool inverse,
                       cudaStream_t st);

@@ -47,6 +47,12 @@ static constexpr double kMadelungK = 0.22578495;  // solver.py:404, 510
 // exx_occ_threshold): each adds f_i times a bounded matrix to K, below FP64
 // rounding of the sum; with Fermi smearing most virtual orbitals are such.
 static constexpr double kExxOccFloor = 1e-14;
+// AOs from which an FP64 plan takes the tiled contractions and folded transforms
+// (H8 dzv at 33^3, 16 AOs, two k-points of Hartree-Fock: 237 -> 71 ms).  Fewer
+// rows leave a 16 x 16 tile mostly padding, and four-atom Hartree-Fock under
+// strong smearing often runs to the iteration limit without converging, where
+// a result is the rounding's: those keep the library's sums.
+static constexpr int kTiledNao = 16;
 
 // Factor table F[A][d][i][a][s] (complex): s = 3 l + k, k = value, first and
 // second derivative of u^l exp(-alpha u^2), each lattice term times the
@@ -454,6 +460,10 @@ struct hqcgb_kplan {
   double *xp = nullptr, *kpt = nullptr;
   double2 *F1d = nullptr, *phi = nullptr, *dphi = nullptr, *ph = nullptr;
   // grid work: operand / pair densities, their potentials, conjugated orbitals
+  // FP64 plans: exchange, quadratures and Poisson solve by exchange_kpt.cu and
+  // poisson_f64.cu instead of complex passes and library contractions
+  bool tiled = false;
+  double2 *zpart = nullptr;  // parts of their contractions
   double2 *Z = nullptr, *W = nullptr, *Psi = nullptr, *dPsi = nullptr, *cbuf = nullptr;
   // matrices (complex, row-major nao x nao)
   double2 *S = nullptr, *T = nullptr, *V = nullptr, *H = nullptr, *St = nullptr, *vorth = nullptr,
@@ -583,7 +593,10 @@ static void kcreate(const hqcgb_params &P, hqcgb_kplan *p) {
   p->mixed = P.precision == HQCGB_PREC_MIXED;
   if (!p->mixed) {  // FP64 operand, pair-density and orbital grids (the mixed path keeps FP32 ones)
     p->Z = p->alloc<double2>((size_t)nao * N);
-    if (p->hf) p->W = p->alloc<double2>((size_t)nao * N);
+    p->tiled = nao >= kTiledNao && p->ng % 2 == 1;
+    p->xg = p->tiled ? kx_group(nao, N) : 1;
+    if (p->hf) p->W = p->alloc<double2>((size_t)p->xg * nao * N);
+    if (p->tiled) p->zpart = p->alloc<double2>(zgram_scratch(nao, p->hf ? p->xg : 1, N));
     p->Psi = p->alloc<double2>((size_t)nao * N);
   }
   if (p->gga) p->dPsi = p->alloc<double2>((size_t)3 * nao * N);
@@ -717,8 +730,22 @@ static void kdensity_matrix(KCtx &c) {
   zgemm('N', 'C', n, n, n, kOne, p->t1, n, p->C, n, kZero, p->D, n, c.st);
 }
 
+// out = scale A Phibar^H over the grid (FP64 plans); herm: the result is Hermitian
+static void kcontract(KCtx &c, const double2 *A, double scale, bool herm, double2 *out) {
+  hqcgb_kplan *p = c.p;
+  const int n = p->nao;
+  if (p->tiled)
+    launch_zgram(n, p->N, 1, A, 0, p->phi, 0, herm, scale, false, p->zpart, out, c.st);
+  else
+    zgemm('N', 'C', n, n, (int)p->N, make_double2(scale, 0.0), A, (int)p->N, p->phi, (int)p->N, kZero, out, n, c.st);
+}
+
 static void kpoisson_real(KCtx &c, const double *src, double *dst) {
   hqcgb_kplan *p = c.p;
+  if (p->tiled) {
+    launch_poisson_f64(src, dst, p->cbuf, p->coul, p->ng, p->tw, c.st);
+    return;
+  }
   launch_real_to_complex(src, nullptr, p->N, 1, p->cbuf, c.st);
   launch_fft3d(p->cbuf, p->ng, 1, p->tw, false, c.st);
   launch_scale_complex(p->cbuf, p->coul, p->N, 1, c.st);
@@ -822,10 +849,10 @@ static void kquadrature(KCtx &c, const double *w, const double *u, double2 *out)
                                                                   u ? 0.5 : 1.0, p->dV, p->Z);
   HQ_LAUNCH_CHECK();
   if (u) {
-    zgemm('N', 'C', n, n, (int)N, kOne, p->Z, (int)N, p->phi, (int)N, kZero, p->t1, n, c.st);
+    kcontract(c, p->Z, 1.0, false, p->t1);
     zcomb(n, 1.0, p->t1, 1.0, p->t1, true, out, c.st);
   } else {
-    zgemm('N', 'C', n, n, (int)N, kOne, p->Z, (int)N, p->phi, (int)N, kZero, out, n, c.st);
+    kcontract(c, p->Z, 1.0, true, out);
   }
 }
 
@@ -840,9 +867,19 @@ static void kexchange(KCtx &c) {
   const long long N = p->N;
   HQ_STAGE(ST_EXCHANGE, c.st);
   HQ_CUDA(cudaMemsetAsync(p->K, 0, sizeof(double2) * n * n, c.st));
+  const double thr = std::max(p->P.exx_occ_threshold, kExxOccFloor);
   for (int i = 0; i < p->nuse; ++i) {
     const double f = p->h_occ[i];
-    if (!(f > std::max(p->P.exx_occ_threshold, kExxOccFloor))) continue;
+    if (!(f > thr)) continue;
+    if (p->tiled) {  // the run of orbitals that begins here
+      int g = 1;
+      while (g < p->xg && i + g < p->nuse && p->h_occ[i + g] > thr) ++g;
+      launch_kx_pairs(p->phi, p->Psi + (long long)i * N, p->h_occ.data() + i, g, p->sqcoul, p->ng, n, p->tw, p->W,
+                      c.st);
+      launch_zgram(n, N, g, p->W, n * N, p->W, n * N, true, p->dV, true, p->zpart, p->K, c.st);
+      i += g - 1;
+      continue;
+    }
     k_pair_kpt<<<ceil_div((long long)n * N, 256), 256, 0, c.st>>>(p->phi, p->Psi + (long long)i * N, n,
                                                                     N, p->W);
     HQ_LAUNCH_CHECK();
@@ -961,7 +998,7 @@ static void kgeometry(KCtx &c, const double *xp_dev, const double *kpt_host) {
     k_zoperand<<<ceil_div((long long)n * N, 256), 256, 0, c.st>>>(p->phi, nullptr, p->vloc, nullptr, n,
                                                                     N, p->dV, 0.0, p->Z);
     HQ_LAUNCH_CHECK();
-    zgemm('N', 'C', n, n, (int)N, kOne, p->Z, (int)N, p->phi, (int)N, kZero, p->V, n, c.st);
+    kcontract(c, p->Z, 1.0, true, p->V);
   }
   zcomb(n, 1.0, p->T, 1.0, p->V, false, p->H, c.st);
   if (p->hf && p->mixed) {
@@ -969,8 +1006,7 @@ static void kgeometry(KCtx &c, const double *xp_dev, const double *kpt_host) {
     HQ_LAUNCH_CHECK();
     kx_quad(c, 1, p->St);
   } else if (p->hf) {
-    zgemm('N', 'C', n, n, (int)N, make_double2(p->dV, 0.0), p->phi, (int)N, p->phi, (int)N, kZero, p->St,
-          n, c.st);
+    kcontract(c, p->phi, p->dV, true, p->St);
   }
   // S^{-1/2} as U w^{-1/2} (solver.py:795-796)
   HQ_CUDA(cudaMemsetAsync(p->ibad, 0, sizeof(int), c.st));

@@ -9,7 +9,7 @@
 // output a thread took six FP64 instructions a term and both halves, these
 // take four a pair of outputs and one half.  Five launches of columns in
 // chunks, so that every pass fills the SMs.  Measured, one
-// potential: 65^3 0.70 -> 0.14 ms, 41^3 (a prime, direct sums) 0.57 -> 0.11,
+// potential: 65^3 0.70 -> 0.12 ms, 41^3 (a prime, direct sums) 0.57 -> 0.11,
 // 49^3 0.28 -> 0.09.
 #include <algorithm>
 
@@ -47,7 +47,7 @@ __global__ void __launch_bounds__(kPsThreads) k_ps_z(PsArgs a) {
     B0[z * cols + c] = make_double2(line[0], 2 * pr + 1 < n ? line[n] : 0.0);
   }
   __syncthreads();
-  const double2 *Z = dft_axis0<double, double2>(B0, B1, B0, n, cols, a.n1, w);
+  const double2 *Z = dft_axis0<double, double2>(B0, B1, n, cols, a.n1, w);
   // A[k] = (Z[k] + conj Z[n-k]) / 2 of the first line, B[k] = (Z[k] - conj Z[n-k]) / 2i of the second
   for (int i = threadIdx.x; i < nh * cols; i += kPsThreads) {
     const int c = i / nh, kz = i - c * nh, id = first + c, x = id / npair, pr = id - x * npair;
@@ -73,7 +73,7 @@ __global__ void __launch_bounds__(kPsThreads) k_ps_y(PsArgs a) {
     B0[i] = INV ? conj2(v) : v;
   }
   __syncthreads();
-  const double2 *R = dft_axis0<double, double2>(B0, B1, B0, n, cols, a.n1, w);
+  const double2 *R = dft_axis0<double, double2>(B0, B1, n, cols, a.n1, w);
   for (int i = threadIdx.x; i < n * cols; i += kPsThreads) {
     const int y = i / cols, c = i - y * cols;
     base[(long long)y * nh + c] = INV ? conj2(R[i]) : R[i];
@@ -93,7 +93,7 @@ __global__ void __launch_bounds__(kPsThreads) k_ps_x(PsArgs a) {
     B0[i] = base[(long long)x * n * nh + c];
   }
   __syncthreads();
-  double2 *R = dft_axis0<double, double2>(B0, B1, B0, n, cols, a.n1, w);
+  double2 *R = dft_axis0<double, double2>(B0, B1, n, cols, a.n1, w);
   for (int i = threadIdx.x; i < n * cols; i += kPsThreads) {
     const int kx = i / cols, c = i - kx * cols;
     const double f = a.kern[((long long)kx * n + ky) * n + k0 + c];
@@ -101,7 +101,7 @@ __global__ void __launch_bounds__(kPsThreads) k_ps_x(PsArgs a) {
   }
   __syncthreads();
   double2 *spare = R == B0 ? B1 : B0;
-  const double2 *S = dft_axis0<double, double2>(R, spare, R, n, cols, a.n1, w);
+  const double2 *S = dft_axis0<double, double2>(R, spare, n, cols, a.n1, w);
   for (int i = threadIdx.x; i < n * cols; i += kPsThreads) {
     const int x = i / cols, c = i - x * cols;
     base[(long long)x * n * nh + c] = conj2(S[i]);
@@ -125,7 +125,7 @@ __global__ void __launch_bounds__(kPsThreads) k_ps_z_inverse(PsArgs a) {
     if (kz) B0[(n - kz) * cols + c] = make_double2(A.x + B.y, A.y - B.x);
   }
   __syncthreads();
-  const double2 *Z = dft_axis0<double, double2>(B0, B1, B0, n, cols, a.n1, w);
+  const double2 *Z = dft_axis0<double, double2>(B0, B1, n, cols, a.n1, w);
   for (int i = threadIdx.x; i < n * cols; i += kPsThreads) {
     const int c = i / n, z = i - c * n, id = first + c, x = id / npair, pr = id - x * npair;
     double *line = a.dst + ((long long)x * n + 2 * pr) * n + z;
