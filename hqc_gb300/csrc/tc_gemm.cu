@@ -1321,6 +1321,203 @@ __global__ void __launch_bounds__(kQtThreads, 1)
 }
 
 // ---------------------------------------------------------------------------
+// The same for at most 64 AOs (one tile, mostly padding in the form above).  Only
+// the tile's nb rows (nb a multiple of 16) are loaded and kept, a Gram matrix
+// (A = B: the exchange) loads them once; the MMA's M = 128 rows of A run on into
+// the bytes that follow a piece, and the accumulator rows they give are never
+// read.  So a stage is 4 to 32 KB instead of 64, a ring holds up to 12 of them and two
+// CTAs share an SM, and the compensated sums of a row fit in its thread's registers:
+// with a drain every stage (the exchange) the three TMEM round trips a stage were
+// what bounded it.  Every sum and its order are as above: the same bits.  Bound now by
+// the MMAs, twelve a stage at some 128 cycles whatever their N (four accumulators
+// and twice the drain warps gave nothing).  Measured, 28 AOs, Gram matrix of 9
+// orbitals at 49^3 (1.06 M points): 340 + 90 (sum of the parts) -> 160 + 10 us.
+// ---------------------------------------------------------------------------
+constexpr int kQnMaxAo = 64, kQnRing = 12;
+constexpr int kQnMmaWarp = 2, kQnTmaWarp = 3, kQnThreads = 128;
+constexpr size_t kQnSmemMax = 110 * 1024;  // two CTAs an SM
+
+struct QnArgs {
+  int nb, same, ring, blocked;
+  long long N;
+  int kchunk, drain;
+  double *partial;  // [parts][nb][nb]
+  int *err;
+};
+
+struct QnPipe {
+  uint64_t full[kQnRing], empty[kQnRing], acc_full[2], acc_empty[2];
+  uint32_t tmem_base;
+};
+
+template <int NB>  // accumulator columns: nb <= NB
+__global__ void __launch_bounds__(kQnThreads, 2)
+    k_tc_quad_narrow(QnArgs a, const __grid_constant__ CUtensorMap mAh, const __grid_constant__ CUtensorMap mAl,
+                     const __grid_constant__ CUtensorMap mBh, const __grid_constant__ CUtensorMap mBl) {
+  extern __shared__ __align__(1024) char smraw[];
+  char *sm = (char *)(((uintptr_t)smraw + 1023) & ~(uintptr_t)1023);
+  __shared__ QnPipe P;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int nb = a.nb, drainers = (nb + 31) / 32;
+  const uint32_t piece = (uint32_t)nb * 128u, slot_bytes = piece * (a.same ? 2u : 4u);
+  const long long k0 = (long long)blockIdx.x * a.kchunk, k1 = min(k0 + (long long)a.kchunk, a.N);
+  const int nstages = (int)((k1 - k0 + kStageK - 1) / kStageK), nsub = (nstages + a.drain - 1) / a.drain;
+  if (tid == 0) {
+    for (int b = 0; b < a.ring; ++b) {
+      mbar_init(&P.full[b], 1);
+      mbar_init(&P.empty[b], 1);
+    }
+    for (int b = 0; b < 2; ++b) {
+      mbar_init(&P.acc_full[b], 1);
+      mbar_init(&P.acc_empty[b], drainers * 32);
+    }
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  if (warp == kQnMmaWarp) tmem_alloc(&P.tmem_base, 2 * NB);
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+
+  bool ok = true;
+  if (warp == kQnTmaWarp) {
+    if (lane == 0) {
+      int slot = 0, phase = 1;
+      for (int st = 0; st < nstages; ++st) {
+        if (st >= a.ring && !mbar_wait(&P.empty[slot], (unsigned)phase, a.err, 36)) break;
+        const int x = (int)(k0 + (long long)st * kStageK);
+        const uint32_t base = smem_u32(sm) + (uint32_t)slot * slot_bytes;
+        mbar_expect_tx(&P.full[slot], slot_bytes);
+        auto load = [&](uint32_t dst, const CUtensorMap *m) {
+          if (a.blocked) tma_load_3d(dst, m, 0, 0, x / kStageK, &P.full[slot]);
+          else tma_load_2d(dst, m, x, 0, &P.full[slot]);
+        };
+        load(base, &mAh);
+        load(base + piece, &mAl);
+        if (!a.same) {
+          load(base + 2u * piece, &mBh);
+          load(base + 3u * piece, &mBl);
+        }
+        if (++slot == a.ring) {
+          slot = 0;
+          phase ^= 1;
+        }
+      }
+    }
+  } else if (warp == kQnMmaWarp) {
+    if (lane == 0) {
+      const uint32_t idesc = idesc_tf32(kM, nb);
+      int stage = 0, slot = 0, phase = 0;
+      for (int j = 0; j < nsub; ++j) {
+        const int ab = j & 1, ause = j >> 1;
+        if (ok && ause > 0 && !mbar_wait(&P.acc_empty[ab], (unsigned)((ause - 1) & 1), a.err, 37)) ok = false;
+        tc_fence_after();
+        const uint32_t tmem_d = P.tmem_base + (uint32_t)(ab * NB);
+        const int s_end = min(nstages, (j + 1) * a.drain);
+        bool first = true;
+        for (; stage < s_end; ++stage) {
+          if (ok && !mbar_wait(&P.full[slot], (unsigned)phase, a.err, 38)) ok = false;
+          tc_fence_after();
+          if (ok) {
+            const uint32_t Ah = smem_u32(sm) + (uint32_t)slot * slot_bytes, Al = Ah + piece;
+            const uint64_t dAh = sdesc(Ah), dAl = sdesc(Al);
+            const uint64_t dBh = a.same ? dAh : sdesc(Ah + 2u * piece), dBl = a.same ? dAl : sdesc(Ah + 3u * piece);
+#pragma unroll
+            for (int ks = 0; ks < kStageK / 8; ++ks) {
+              const uint64_t o = 2u * (uint32_t)ks;
+              mma_tf32(tmem_d, dAl + o, dBh + o, idesc, (first && ks == 0) ? 0 : 1);
+              mma_tf32(tmem_d, dAh + o, dBl + o, idesc, 1);
+              mma_tf32(tmem_d, dAh + o, dBh + o, idesc, 1);
+            }
+          }
+          first = false;
+          mma_commit(&P.empty[slot]);
+          if (++slot == a.ring) {
+            slot = 0;
+            phase ^= 1;
+          }
+        }
+        mma_commit(&P.acc_full[ab]);
+      }
+    }
+  } else if (warp < drainers) {
+    // thread = TMEM lane (output row); its compensated sums in registers
+    const uint32_t lane_off = (uint32_t)(warp * 32) << 16;
+    float sv[NB], cv[NB];
+#pragma unroll
+    for (int i = 0; i < NB; ++i) sv[i] = cv[i] = 0.f;
+    for (int j = 0; j < nsub; ++j) {
+      const int b = j & 1, use = j >> 1;
+      const bool got = ok && mbar_wait(&P.acc_full[b], (unsigned)(use & 1), a.err, 39);
+      if (!got) ok = false;
+      tc_fence_after();
+      if (got) {
+        uint32_t va[NB];
+#pragma unroll
+        for (int c = 0; c < NB; c += 16)
+          if (c < nb) tmem_ld16_nowait(P.tmem_base + lane_off + b * NB + c, va + c);
+        tmem_wait_ld();
+        if (j == 0) {
+#pragma unroll
+          for (int i = 0; i < NB; ++i) sv[i] = i < nb ? __uint_as_float(va[i]) : 0.f;
+        } else {
+#pragma unroll
+          for (int c = 0; c < NB; c += 16)
+            if (c < nb)
+#pragma unroll
+              for (int i = c; i < c + 16; ++i) two_sum_add(sv[i], cv[i], __uint_as_float(va[i]));
+        }
+      }
+      tc_fence_before();
+      mbar_arrive(&P.acc_empty[b]);
+    }
+    const int row = warp * 32 + lane;
+    if (ok && row < nb) {
+      double *out = a.partial + ((long long)blockIdx.x * nb + row) * nb;
+#pragma unroll
+      for (int i = 0; i < NB; ++i)
+        if (i < nb) out[i] = (double)sv[i] + (double)cv[i];
+    }
+  }
+  tc_fence_before();
+  __syncthreads();
+  if (warp == kQnMmaWarp) {
+    tc_fence_after();
+    tmem_dealloc(P.tmem_base, 2 * NB);
+  }
+}
+
+// Sums of the parts into part 0 in the order of k_tc_quad_sum_parts (four partial
+// sums, one a quarter of the block); 64 elements a block.
+__global__ void __launch_bounds__(256) k_qn_sum(double *__restrict__ P, int nparts, int nb2) {
+  __shared__ double sh[4][64];
+  const int q = threadIdx.x >> 6, e = threadIdx.x & 63, idx = blockIdx.x * 64 + e;
+  const double *src = P + idx;
+  double s = 0;
+  if (idx < nb2) {
+    const int n4 = nparts & ~3;
+#pragma unroll 8
+    for (int k = q; k < n4; k += 4) s += src[(long long)k * nb2];
+    if (q == 0)
+      for (int k = n4; k < nparts; ++k) s += src[(long long)k * nb2];
+  }
+  sh[q][e] = s;
+  __syncthreads();
+  if (q == 0 && idx < nb2) P[idx] = (sh[0][e] + sh[1][e]) + (sh[2][e] + sh[3][e]);
+}
+
+// M from the sums, as k_tc_quad_reduce
+__global__ void k_qn_reduce(const double *__restrict__ P, int nb, int nao, int sym, int add_transpose, double scale,
+                            double *__restrict__ M) {
+  const int idx = blockIdx.x * blockDim.x + threadIdx.x;
+  if (idx >= nao * nao) return;
+  const int p = idx / nao, q = idx - p * nao;
+  const double a = P[p * nb + q], b = P[q * nb + p];
+  double v = (sym && !add_transpose) ? 0.5 * (a + b) : a;
+  if (add_transpose) v += b;
+  M[idx] = scale * v;
+}
+
+// ---------------------------------------------------------------------------
 // Persistent quadrature for n_ao = 128 nfull + last with last <= 16 (e.g.
 // 270 = 2 x 128 + 14) or no partial block: grid (tiles, groups).  The CTAs
 // of group g share one contiguous K slice (1/groups of the grid points) and
@@ -2045,6 +2242,39 @@ void launch_tc_quad_split(const float *Ahl, const float *Bhl, int nao, long long
   HQ_REQUIRE(kchunk % tc::kStageK == 0, "K chunk must be a multiple of 32");
   HQ_REQUIRE(ld % 32 == 0 && ld >= N, "pre-split operands need a row stride that is a multiple of 32");
   HQ_REQUIRE(N <= (1LL << 31) - 64, "grid too large for 32-bit TMA coordinates");
+  if (nao <= tc::kQnMaxAo) {
+    tc::QnArgs q;
+    q.nb = (nao + 15) / 16 * 16;
+    q.same = Ahl == Bhl ? 1 : 0;
+    const size_t slot = (size_t)q.nb * 128 * (q.same ? 2 : 4), past = (size_t)(tc::kM - q.nb) * 128 + 1024;
+    q.ring = (int)std::min<size_t>(tc::kQnRing, (tc::kQnSmemMax - past) / slot);
+    q.blocked = blocked ? 1 : 0;
+    q.N = N;
+    q.kchunk = kchunk;
+    q.drain = drain;
+    q.partial = partial;
+    q.err = err;
+    auto map = [&](const float *b) {
+      return blocked ? tc::tensor_map_3d_kblk(b, nao, ld / tc::kStageK, q.nb)
+                     : tc::tensor_map_2d_ext(b, ld, N, nao, q.nb);
+    };
+    const size_t lo = (size_t)nao * ld, smem = q.ring * slot + past;
+    const CUtensorMap mAh = map(Ahl), mAl = map(Ahl + lo), mBh = map(Bhl), mBl = map(Bhl + lo);
+    const int nparts = (int)ceil_div(N, (long long)kchunk);
+    auto go = [&](auto kernel) {
+      ensure_dyn_smem((const void *)kernel, smem);
+      kernel<<<nparts, tc::kQnThreads, smem, st>>>(q, mAh, mAl, mBh, mBl);
+      HQ_LAUNCH_CHECK();
+    };
+    if (q.nb <= 32) go(tc::k_tc_quad_narrow<32>);
+    else go(tc::k_tc_quad_narrow<64>);
+    tc::k_qn_sum<<<ceil_div(q.nb * q.nb, 64), 256, 0, st>>>(partial, nparts, q.nb * q.nb);
+    HQ_LAUNCH_CHECK();
+    tc::k_qn_reduce<<<ceil_div(nao * nao, 256), 256, 0, st>>>(partial, q.nb, nao, sym ? 1 : 0, add_transpose ? 1 : 0,
+                                                             scale, M);
+    HQ_LAUNCH_CHECK();
+    return;
+  }
   const QuadTilePlan plan = plan_quad_tiles(nao, sym, blocked);  // the persistent form reads K-blocked pieces
   const int nblk = plan.nblk;
   const long long rows = nao;
