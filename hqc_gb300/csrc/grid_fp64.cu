@@ -160,6 +160,61 @@ void launch_density(const double *phi, const double *dphi, const double *D, int 
 }
 
 // ---------------------------------------------------------------------------
+// S~ = dV phi phi^T of a mixed Hartree-Fock plan, in FP64: chunks of 2048 points
+// in sequence, then the chunks in sequence.  8 x 8 tiles of the lower triangle, one
+// output a thread: the FP64 pipe bounds it, and few AOs in larger tiles leave most
+// SMs idle (28 AOs at 49^3: 664 us with 32 x 32 tiles, 163 with 8 x 8; the digit form
+// of the FP64 plans takes 76, with operands and tables for this one sum a geometry).
+// ---------------------------------------------------------------------------
+constexpr int kGramChunk = 2048, kGramT = 8;
+
+__global__ void __launch_bounds__(kGramT * kGramT) k_gram_part(const double *__restrict__ A, int nao, long long N,
+                                                               double *__restrict__ P) {
+  __shared__ double As[kGramT][33], Bs[kGramT][33];
+  int pt = (int)((sqrtf(8.f * blockIdx.x + 1.f) - 1.f) * 0.5f);
+  while (pt * (pt + 1) / 2 > (int)blockIdx.x) --pt;
+  while ((pt + 1) * (pt + 2) / 2 <= (int)blockIdx.x) ++pt;
+  const int p0 = pt * kGramT, q0 = ((int)blockIdx.x - pt * (pt + 1) / 2) * kGramT;
+  const int tid = threadIdx.x, p = tid / kGramT, q = tid % kGramT, tx = tid & 31;
+  const long long k0 = (long long)blockIdx.y * kGramChunk, k1 = min(k0 + kGramChunk, N);
+  double acc = 0;
+  for (long long kb = k0; kb < k1; kb += 32) {
+    const long long k = kb + tx;
+#pragma unroll
+    for (int r = tid >> 5; r < kGramT; r += kGramT * kGramT / 32) {
+      As[r][tx] = k < k1 && p0 + r < nao ? A[(long long)(p0 + r) * N + k] : 0.0;
+      Bs[r][tx] = k < k1 && q0 + r < nao ? A[(long long)(q0 + r) * N + k] : 0.0;
+    }
+    __syncthreads();
+#pragma unroll
+    for (int kk = 0; kk < 32; ++kk) acc = fma(As[p][kk], Bs[q][kk], acc);
+    __syncthreads();
+  }
+  if (p0 + p < nao && q0 + q < nao) P[((long long)blockIdx.y * nao + p0 + p) * nao + q0 + q] = acc;
+}
+
+__global__ void k_gram_sum(const double *__restrict__ P, int nchunk, int nao, double scale, double *__restrict__ M) {
+  const int idx = blockIdx.x * blockDim.x + threadIdx.x;
+  if (idx >= nao * nao) return;
+  const int i = idx / nao, j = idx % nao, p = max(i, j), q = min(i, j);
+  double s = 0;
+#pragma unroll 8
+  for (int c = 0; c < nchunk; ++c) s += P[((long long)c * nao + p) * nao + q];
+  M[idx] = scale * s;
+}
+
+size_t gram_scratch_doubles(int nao, long long N) { return (size_t)ceil_div(N, kGramChunk) * nao * nao; }
+
+void launch_gram(const double *A, int nao, long long N, double scale, double *P, double *M, cudaStream_t st) {
+  HQ_STAGE(ST_QUAD, st);
+  const int nt = ceil_div(nao, kGramT), nchunk = ceil_div(N, kGramChunk);
+  k_gram_part<<<dim3(nt * (nt + 1) / 2, nchunk), kGramT * kGramT, 0, st>>>(A, nao, N, P);
+  HQ_LAUNCH_CHECK();
+  k_gram_sum<<<ceil_div(nao * nao, 256), 256, 0, st>>>(P, nchunk, nao, scale, M);
+  HQ_LAUNCH_CHECK();
+}
+
+// ---------------------------------------------------------------------------
 // pointwise: exchange-correlation on the grid.
 //   in : rho, grho (GGA), vh (Hartree potential)
 //   out: w = dV (vh + v_rho) (quadrature weight), u = 2 v_sigma grad rho (GGA)

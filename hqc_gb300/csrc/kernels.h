@@ -203,6 +203,10 @@ bool eigh_mixed_warm(int n, const double *A, const double *X0, double *V, double
 bool eigh_mixed(int n, const double *A, double *V, double *w, MixedEigWork &ws, cudaStream_t st,
                 bool wide = false, EigLevel level = EigLevel::Full);
 
+// grid_fp64.cu: M = scale A A^T over rows of N points, P: gram_scratch_doubles
+size_t gram_scratch_doubles(int nao, long long N);
+void launch_gram(const double *A, int nao, long long N, double scale, double *P, double *M, cudaStream_t st);
+
 // poisson_f64.cu: dst = DFT^-1[kern DFT[src]] of a real field on an odd grid;
 // cbuf holds n n (n + 1) / 2 values, kern as launch_coulomb_table
 bool poisson_f64_supported(int n);

@@ -214,6 +214,7 @@ struct hqcgb_plan {
   float2 *cbuf32 = nullptr;
   int *tc_err = nullptr;
   Quad64 q64{};                // FP64 quadratures
+  double *stpart = nullptr;    // chunks of S~ (mixed Hartree-Fock)
   Density64 d64{};             // FP64 density from the orbitals
   int nuse_64 = 0;             // orbitals it runs over
   MixedEigWork mew{};
@@ -483,7 +484,8 @@ static void create(const hqcgb_params *in, hqcgb_plan *p) {
   p->cbuf_batch = (p->hf && !p->exx_fused) ? nao : 1;
   if (p->hf && !p->exx_fused) p->W = p->alloc<double>((size_t)nao * N);
   p->cbuf = p->alloc<double2>((size_t)p->cbuf_batch * N);
-  if (!p->mixed || p->hf) {
+  if (p->mixed && p->hf) p->stpart = p->alloc<double>(gram_scratch_doubles(nao, N));
+  if (!p->mixed || (p->hf && !p->exx_fused)) {
     // FP64 quadratures: Fock, V, S~ and the Gram matrix of the FP64 exchange
     const long long gK = p->exx_fused && !p->mixed ? (long long)p->exx_g * exx_pair_len(p->ng) : 0;
     const long long most = std::max(N, gK), tabN = quad64_table(N);
@@ -946,7 +948,8 @@ static void geometry(Ctx &c, const double *xp_dev) {
     quad64_weighted(p->q64, p->phi, p->vloc, N, p->dV, p->V, c.st);
   }
   axpby(n, 1.0, p->T, 1.0, p->V, false, p->H, c.st);
-  if (p->hf) quad64_weighted(p->q64, p->phi, nullptr, N, p->dV, p->St, c.st);
+  if (p->hf && p->mixed) launch_gram(p->phi, n, N, p->dV, p->stpart, p->St, c.st);
+  else if (p->hf) quad64_weighted(p->q64, p->phi, nullptr, N, p->dV, p->St, c.st);
   // S^{-1/2} as U w^{-1/2} (solver.py:729-730)
   HQ_CUDA(cudaMemsetAsync(p->ibad, 0, sizeof(int), c.st));
   eigh(c, p->S, p->c1, p->ws, true);
