@@ -78,18 +78,24 @@ struct PlaneArgs {
   const void *psi;           // psi~ of the group's first orbital, rows ldpsi apart (R)
   long long ldpsi;
   void *T;                   // [g][rows][n][n][nh] complex R
+  int g, per;                // orbitals of the group, orbitals a block
 };
 
-// grid (n x-planes, rows, orbitals of the group)
-// FP32: four CTAs of 256 threads per SM (64 registers); FP64 runs one
+// grid (n x-planes, rows, ceil(g / per)).  Several orbitals a block share the row's
+// field: its primitives' products cost about as much as the transforms (28 rows,
+// 10 orbitals at 49^3, FP32: 320 -> 212 us).
+// CTAs of 256 threads per SM: FP32 four (64 registers; the gradient's columns three:
+// 957 -> 500 us for 28 rows of 4 orbitals at 49^3, where one block an SM hid no
+// latency), FP64 two (H8 szv at 41^3: 7.3 -> 6.65 ms a run)
 template <typename R>
-constexpr int exx_min_blocks() { return sizeof(R) == 4 ? 4 : 1; }
+constexpr int exx_min_blocks() { return sizeof(R) == 4 ? 4 : 2; }
 
 template <typename R>
 __global__ void __launch_bounds__(256, exx_min_blocks<R>()) k_exx_plane(PlaneArgs a) {
   using R2 = typename C2<R>::T;
   extern __shared__ __align__(16) unsigned char smraw[];
-  const int n = a.n, nh = a.nh, x = blockIdx.x, r = blockIdx.y, jl = blockIdx.z;
+  const int n = a.n, nh = a.nh, x = blockIdx.x, r = blockIdx.y;
+  const int jl0 = blockIdx.z * a.per, jl1 = min(jl0 + a.per, a.g);
   const size_t bufc = (size_t)n * (n + 1) / 2 + 1;  // complex slots of one plane buffer (>= n^2 reals)
   R2 *w = reinterpret_cast<R2 *>(smraw);
   R2 *B0 = w + n;                  // plane buffers: the packed pair lines, the
@@ -97,23 +103,28 @@ __global__ void __launch_bounds__(256, exx_min_blocks<R>()) k_exx_plane(PlaneArg
   R *fyz = reinterpret_cast<R *>(B1 + bufc);  // [2][nprim][n]: y and z factors
   load_twiddles(w, a.tw, n);
   const long long plane = (long long)x * n * n;
-  const R *psi = reinterpret_cast<const R *>(a.psi) + (long long)jl * a.ldpsi + plane;
-  const long long nn = (long long)n * n;
+  const int nn = n * n;
   // The pair plane goes straight into the packed layout of the z transform:
   // complex column pr of Z[z][pr] holds the real y-lines 2 pr (real part) and
   // 2 pr + 1 (imaginary part); the last column of an odd n has no partner.
   const int npair = (n + 1) / 2;
-  R *Zr = reinterpret_cast<R *>(B0);  // Z[z][pr] as reals: [z][pr][2]
-  auto put = [&](int i, R v) {
-    const int y = i / n, z = i - y * n;
-    Zr[2 * (z * npair + (y >> 1)) + (y & 1)] = v;
+  const int sy = (int)blockDim.x / n, sz = (int)blockDim.x - sy * n;  // a step of blockDim.x points
+  const int yf = (int)threadIdx.x / n, zf = (int)threadIdx.x - yf * n;
+  // each(f): f(i, y, z, slot of the packed layout) for the thread's points i = y n + z
+  auto each = [&](auto f) {
+    int y = yf, z = zf;
+    for (int i = threadIdx.x; i < nn; i += blockDim.x) {
+      f(i, y, z, 2 * (z * npair + (y >> 1)) + (y & 1));
+      y += sy;
+      z += sz;
+      if (z >= n) {
+        z -= n;
+        ++y;
+      }
+    }
   };
-  if (n & 1)
-    for (int z = threadIdx.x; z < n; z += blockDim.x) Zr[2 * (z * npair + npair - 1) + 1] = 0;
-  if (r < a.xrows) {
-    const double *Xr = a.X + (long long)r * a.ldx + plane;
-    for (int i = threadIdx.x; i < nn; i += blockDim.x) put(i, (R)Xr[i] * psi[i]);
-  } else {
+  R fx[8];
+  if (r >= a.xrows) {
     // Fock mode: row r is phi_p, p = r (c = -1: the value); gradient mode:
     // row nao (1 + c) + p is d_c phi_p
     const int rr = r - a.xrows;
@@ -127,38 +138,49 @@ __global__ void __launch_bounds__(256, exx_min_blocks<R>()) k_exx_plane(PlaneArg
       const int ax = i / (a.nprim * n), rem = i - ax * a.nprim * n, pr = rem / n, t = rem - pr * n;
       fyz[i] = F[((((long long)A * 3 + 1 + ax) * n + t) * a.nprim + pr) * 6 + e[1 + ax]];
     }
-    __syncthreads();
-    R fx[8];
     for (int pr = 0; pr < a.nprim; ++pr)
       fx[pr] = (R)a.coef[k * a.nprim + pr] * F[((((long long)A * 3 + 0) * n + x) * a.nprim + pr) * 6 + e[0]];
-    for (int i = threadIdx.x; i < nn; i += blockDim.x) {
-      const int y = i / n, z = i - y * n;
-      R v = 0;
-      for (int pr = 0; pr < a.nprim; ++pr) v += fx[pr] * fyz[pr * n + y] * fyz[(a.nprim + pr) * n + z];
-      put(i, v * psi[i]);
+    __syncthreads();
+  }
+  const double *Xr = a.X + (long long)r * a.ldx + plane;  // read where r < xrows
+  auto field = [&](int i, int y, int z) {
+    if (r < a.xrows) return (R)Xr[i];
+    R v = 0;
+    for (int pr = 0; pr < a.nprim; ++pr) v += fx[pr] * fyz[pr * n + y] * fyz[(a.nprim + pr) * n + z];
+    return v;
+  };
+  R *ao = fyz + 2 * a.nprim * n;  // the row's field on the plane, packed (several orbitals a block)
+  if (a.per > 1) each([&](int i, int y, int z, int slot) { ao[slot] = field(i, y, z); });
+  for (int jl = jl0; jl < jl1; ++jl) {
+    const R *psi = reinterpret_cast<const R *>(a.psi) + (long long)jl * a.ldpsi + plane;
+    R *Zr = reinterpret_cast<R *>(B0);  // Z[z][pr] as reals: [z][pr][2]
+    if (n & 1)
+      for (int z = threadIdx.x; z < n; z += blockDim.x) Zr[2 * (z * npair + npair - 1) + 1] = 0;
+    if (a.per > 1) each([&](int i, int, int, int slot) { Zr[slot] = ao[slot] * psi[i]; });
+    else each([&](int i, int y, int z, int slot) { Zr[slot] = field(i, y, z) * psi[i]; });
+    __syncthreads();
+    // z transform of the packed lines, then unpacked into C[y][kz], kz < nh:
+    // A[k] = (Z[k] + conj Z[n-k]) / 2 (line 2 pr), B[k] = (Z[k] - conj Z[n-k]) / 2i
+    R2 *Zt = dft_axis0<R, R2>(B0, B1, n, npair, a.n1, w);
+    R2 *Cb = (Zt == B0) ? B1 : B0;
+    for (int i = threadIdx.x; i < npair * nh; i += blockDim.x) {
+      const int pr = i / nh, kz = i - pr * nh;
+      const R2 zk = Zt[kz * npair + pr], zm = Zt[(kz == 0 ? 0 : n - kz) * npair + pr];
+      R2 u, v;
+      u.x = (R)0.5 * (zk.x + zm.x);
+      u.y = (R)0.5 * (zk.y - zm.y);
+      v.x = (R)0.5 * (zk.y + zm.y);
+      v.y = (R)0.5 * (zm.x - zk.x);
+      Cb[(2 * pr) * nh + kz] = u;
+      if (2 * pr + 1 < n) Cb[(2 * pr + 1) * nh + kz] = v;
     }
+    __syncthreads();
+    R2 *Ct = (Cb == B0) ? B1 : B0;
+    const R2 *res = dft_axis0<R, R2>(Cb, Ct, n, nh, a.n1, w);
+    R2 *T = reinterpret_cast<R2 *>(a.T) + (((long long)jl * a.rows + r) * n + x) * (long long)n * nh;
+    for (int i = threadIdx.x; i < n * nh; i += blockDim.x) T[i] = res[i];
+    if (jl + 1 < jl1) __syncthreads();  // the next pair overwrites res
   }
-  __syncthreads();
-  // z transform of the packed lines, then unpacked into C[y][kz], kz < nh:
-  // A[k] = (Z[k] + conj Z[n-k]) / 2 (line 2 pr), B[k] = (Z[k] - conj Z[n-k]) / 2i
-  R2 *Zt = dft_axis0<R, R2>(B0, B1, n, npair, a.n1, w);
-  R2 *Cb = (Zt == B0) ? B1 : B0;
-  for (int i = threadIdx.x; i < npair * nh; i += blockDim.x) {
-    const int pr = i / nh, kz = i - pr * nh;
-    const R2 zk = Zt[kz * npair + pr], zm = Zt[(kz == 0 ? 0 : n - kz) * npair + pr];
-    R2 u, v;
-    u.x = (R)0.5 * (zk.x + zm.x);
-    u.y = (R)0.5 * (zk.y - zm.y);
-    v.x = (R)0.5 * (zk.y + zm.y);
-    v.y = (R)0.5 * (zm.x - zk.x);
-    Cb[(2 * pr) * nh + kz] = u;
-    if (2 * pr + 1 < n) Cb[(2 * pr + 1) * nh + kz] = v;
-  }
-  __syncthreads();
-  R2 *Ct = (Cb == B0) ? B1 : B0;
-  const R2 *res = dft_axis0<R, R2>(Cb, Ct, n, nh, a.n1, w);
-  R2 *T = reinterpret_cast<R2 *>(a.T) + (((long long)jl * a.rows + r) * n + x) * (long long)n * nh;
-  for (int i = threadIdx.x; i < n * nh; i += blockDim.x) T[i] = res[i];
 }
 
 struct ColumnArgs {
@@ -182,7 +204,7 @@ __device__ inline uint32_t tf32_rna_x(float x) {
 // OUT 0: FP64 Q;  OUT 1: TF32 hi/lo Q;  OUT 2: gradient dot products.
 // grid (n ky-lines, AOs (OUT 2) or rows, orbitals of the group)
 template <typename R, int OUT>
-__global__ void __launch_bounds__(256, OUT == 2 ? 1 : exx_min_blocks<R>()) k_exx_column(ColumnArgs a) {
+__global__ void __launch_bounds__(256, OUT == 2 && sizeof(R) == 4 ? 3 : exx_min_blocks<R>()) k_exx_column(ColumnArgs a) {
   using R2 = typename C2<R>::T;
   extern __shared__ __align__(16) unsigned char smraw[];
   const int n = a.n, nh = a.nh, ky = blockIdx.x, r = blockIdx.y, jl = blockIdx.z;
@@ -383,9 +405,20 @@ void launch_exx_plane(const ExxGeom &G, const R *F1d, const double *X, long long
   a.psi = psi;
   a.ldpsi = ldpsi;
   a.T = T;
-  const size_t smem = plane_smem<R>(G.n, G.nprim);
+  // The shared field takes n (n + 1) reals, where that leaves four (FP64: two)
+  // blocks an SM; as many blocks as orbitals allow above four waves.
+  size_t smem = plane_smem<R>(G.n, G.nprim);
+  const size_t field = sizeof(R) * ((size_t)G.n * (G.n + 1) + 2);
+  const int blocks = sizeof(R) == 4 ? 4 : 2;
+  a.g = g;
+  a.per = 1;
+  if (g > 1 && blocks * (smem + field + 1024) <= 228 * 1024) {
+    const int split = std::min(g, std::max(1, ceil_div(152 * blocks * 4, (long long)G.n * a.rows)));
+    a.per = ceil_div(g, split);
+    if (a.per > 1) smem += field;
+  }
   ensure_dyn_smem((const void *)exx::k_exx_plane<R>, smem);
-  exx::k_exx_plane<R><<<dim3(G.n, a.rows, g), 256, smem, st>>>(a);
+  exx::k_exx_plane<R><<<dim3(G.n, a.rows, ceil_div(g, a.per)), 256, smem, st>>>(a);
   HQ_LAUNCH_CHECK();
 }
 
