@@ -1,4 +1,7 @@
-// Periodic Poisson solver on the odd real-space grid (FP64 path).
+// Complex 3D transforms on the odd real-space grid: the local potential and its
+// force term, the FP32 Poisson solve of the mixed plans, the k-point plans' FP32
+// pairs and, below 16 AOs, their FP64 ones (the FP64 Hartree potential and the
+// larger k-point exchange have their own: poisson_f64.cu, exchange_kpt.cu).
 //
 // The reference forms pair densities in G space with 1D FFTs and contracts
 // them with V(G) = 4 pi / (Omega G^2), G = 0 dropped (hqc/pbc/solver.py:

@@ -250,11 +250,11 @@ void launch_tc_quad_split(const float *Ahl, const float *Bhl, int nao, long long
                           int *err, cudaStream_t st, int drain, int kchunk = 0, bool blocked = false);
 void launch_split_operand(const float *phi, const float *dphi, const float *w, const float *u, int nao,
                           long long N, long long ldi, long long ldo, float a, float b, float *out,
-                          cudaStream_t st);
+                          cudaStream_t st, float *plain = nullptr);
 void launch_tc_quadrature(const float *phi, const float *dphi, const float *phihl, const float *w,
                           const float *u, float dV, int nao, long long N, long long ld, bool gga,
                           double scale, double *partial, double *M, int *err, cudaStream_t st, int drain,
-                          float *zhl);
+                          float *zhl, float *split_phi = nullptr);
 size_t tc_density_partial_doubles(int nao, long long ld, bool gga);
 int tc_ldk(int nao);
 void launch_transpose_phi(const float *phi, int nao, long long N, long long ld, float *phiT,

@@ -26,7 +26,9 @@
 //   k_tc_quad_tma /   TMA loads of operands split once by the pass that forms
 //   k_tc_quad_persist them (k_split_operand), one MMA thread, four or eight
 //                     drain warps; FP64 partial tiles per K chunk (tile-list
-//                     form) or per K slice of a persistent CTA group.
+//                     form) or per K slice of a persistent CTA group;
+//   k_tc_quad_narrow  the same for at most 64 AOs: the rows that exist, sums in
+//                     registers, two CTAs an SM.
 // Shared memory holds every operand in the UMMA canonical K-major
 // 128-byte-swizzled layout.  Every mbarrier wait has a time limit: on expiry
 // the kernel records an error code in *err, stops issuing work, waits
@@ -1882,19 +1884,26 @@ __global__ void __launch_bounds__(256) k_quad_corner(const float *__restrict__ A
 // [ldo / 32][nao][32] per piece, with zeros in [N, ldo), so that the
 // quadrature's 128-row x 32-point TMA boxes are contiguous 16 KB runs.
 // Grid (column blocks of 1024, rows); 4 columns per thread (ldi a multiple of
-// 4, ldo of 32, 16-byte aligned rows).
+// 4, ldo of 32, 16-byte aligned rows).  PLAIN: the pieces of phi itself as well, for
+// a caller that has none yet: phi is read once for both (HBM-bound: 270 x 81^3 PBE,
+// both operands in two passes 0.80 ms, in one 0.71).
+template <bool PLAIN>
 __global__ void __launch_bounds__(256)
     k_split_operand(const float *__restrict__ phi, const float *__restrict__ dphi,
                     const float *__restrict__ w, const float *__restrict__ u, int nao, long long N,
                     long long ldi, long long ldo, float a, float b, float *__restrict__ hi,
-                    float *__restrict__ lo) {
+                    float *__restrict__ lo, float *__restrict__ plain_hi, float *__restrict__ plain_lo) {
   const int p = blockIdx.y;
   const long long g = ((long long)blockIdx.x * blockDim.x + threadIdx.x) * 4;
   if (g >= ldo) return;
   const long long j = (long long)p * ldi + g, NN = (long long)nao * ldi;
-  float z[4] = {0.f, 0.f, 0.f, 0.f};
+  float z[4] = {0.f, 0.f, 0.f, 0.f}, x[4] = {0.f, 0.f, 0.f, 0.f};
   if (g + 3 < N) {
     const float4 f = *reinterpret_cast<const float4 *>(phi + j);
+    x[0] = f.x;
+    x[1] = f.y;
+    x[2] = f.z;
+    x[3] = f.w;
     float4 wv = w ? *reinterpret_cast<const float4 *>(w + g) : make_float4(1.f, 1.f, 1.f, 1.f);
     z[0] = a * wv.x * f.x;
     z[1] = a * wv.y * f.y;
@@ -1914,6 +1923,7 @@ __global__ void __launch_bounds__(256)
   } else {
     for (int e = 0; e < 4; ++e) {
       if (g + e >= N) break;
+      x[e] = phi[j + e];
       float v = (w ? a * w[g + e] : a) * phi[j + e];
       if (u)
         for (int d = 0; d < 3; ++d) v += b * u[d * ldi + g + e] * dphi[d * NN + j + e];
@@ -1928,6 +1938,14 @@ __global__ void __launch_bounds__(256)
   const long long o = ((g >> 5) * nao + p) * 32 + (g & 31);
   *reinterpret_cast<float4 *>(hi + o) = h;
   *reinterpret_cast<float4 *>(lo + o) = l;
+  if (PLAIN) {
+    split2(x[0], h.x, l.x);
+    split2(x[1], h.y, l.y);
+    split2(x[2], h.z, l.z);
+    split2(x[3], h.w, l.w);
+    *reinterpret_cast<float4 *>(plain_hi + o) = h;
+    *reinterpret_cast<float4 *>(plain_lo + o) = l;
+  }
 }
 
 // Yhl[0][k][p], Yhl[1][k][p]: TF32 hi/lo pieces of C[p][k] sqrt(occ[k]) for
@@ -2344,37 +2362,44 @@ void launch_tc_quad_split(const float *Ahl, const float *Bhl, int nao, long long
   HQ_LAUNCH_CHECK();
 }
 
-// hi/lo pieces of a w phi + b u . grad phi into out [2][nao][ldo]
+// hi/lo pieces of a w phi + b u . grad phi into out [2][nao][ldo], and those of phi
+// into plain where given
 void launch_split_operand(const float *phi, const float *dphi, const float *w, const float *u, int nao,
                           long long N, long long ldi, long long ldo, float a, float b, float *out,
-                          cudaStream_t st) {
+                          cudaStream_t st, float *plain) {
   HQ_STAGE(ST_SPLIT, st);
   HQ_REQUIRE(ldi % 4 == 0 && ldo % 32 == 0 && ldo >= N && ldi >= N, "split operand: bad row strides");
   dim3 grid(ceil_div(ldo, 1024), nao);
-  tc::k_split_operand<<<grid, 256, 0, st>>>(phi, dphi, w, u, nao, N, ldi, ldo, a, b, out,
-                                             out + (size_t)nao * ldo);
+  const size_t lo = (size_t)nao * ldo;
+  if (plain)
+    tc::k_split_operand<true><<<grid, 256, 0, st>>>(phi, dphi, w, u, nao, N, ldi, ldo, a, b, out, out + lo, plain,
+                                                    plain + lo);
+  else
+    tc::k_split_operand<false><<<grid, 256, 0, st>>>(phi, dphi, w, u, nao, N, ldi, ldo, a, b, out, out + lo, nullptr,
+                                                     nullptr);
   HQ_LAUNCH_CHECK();
 }
 
 // Quadrature of the Fock build from the pre-split phi (phihl [2][nao][ld]):
 // LDA  M = (w phi) phi^T (symmetric);  GGA  M = Z phi^T + phi Z^T with
-// Z = 0.5 w phi + dV u . grad phi.  zhl [2][nao][ld] receives the split operand.
+// Z = 0.5 w phi + dV u . grad phi.  zhl [2][nao][ld] receives the split operand;
+// split_phi: phihl, where its pieces are still to be formed (in the same pass).
 void launch_tc_quadrature(const float *phi, const float *dphi, const float *phihl, const float *w,
                           const float *u, float dV, int nao, long long N, long long ld, bool gga,
                           double scale, double *partial, double *M, int *err, cudaStream_t st, int drain,
-                          float *zhl) {
-  HQ_REQUIRE(zhl && phihl, "quadrature needs the split operand buffers");
+                          float *zhl, float *split_phi) {
+  HQ_REQUIRE(zhl && phihl && (!split_phi || split_phi == phihl), "quadrature needs the split operand buffers");
   // K chunk: a tuned multiple of the default (the partial tiles are sized
   // for the default, so longer chunks always fit)
   long long kc = tune_get("quad_kchunk", tc_quad_chunk());
   if (kc < tc_quad_chunk() || kc % tc_quad_chunk() != 0 || kc > (1 << 20)) kc = tc_quad_chunk();
   if (!gga) {
-    launch_split_operand(phi, nullptr, w, nullptr, nao, N, ld, ld, 1.f, 0.f, zhl, st);
+    launch_split_operand(phi, nullptr, w, nullptr, nao, N, ld, ld, 1.f, 0.f, zhl, st, split_phi);
     launch_tc_quad_split(zhl, phihl, nao, N, ld, true, false, scale, partial, M, err, st, drain, (int)kc, true);
     return;
   }
   HQ_REQUIRE(dphi && u, "GGA quadrature needs dphi and u");
-  launch_split_operand(phi, dphi, w, u, nao, N, ld, ld, 0.5f, dV, zhl, st);
+  launch_split_operand(phi, dphi, w, u, nao, N, ld, ld, 0.5f, dV, zhl, st, split_phi);
   launch_tc_quad_split(zhl, phihl, nao, N, ld, false, true, scale, partial, M, err, st, drain, (int)kc, true);
 }
 
@@ -2441,8 +2466,7 @@ extern "C" int hqcgb_tc_quadrature_gga(int nao, long long N, long long ld, const
     int *err = err_buf.as<int>();
     HQ_CUDA(cudaMemsetAsync(err, 0, sizeof(int), st));
     float *phl = hl, *zhl = hl + 2 * (size_t)nao * ld;
-    launch_split_operand(phi, nullptr, nullptr, nullptr, nao, N, ld, ld, 1.f, 0.f, phl, st);
-    launch_tc_quadrature(phi, dphi, phl, w, u, dV, nao, N, ld, true, 1.0, part, M, err, st, drain, zhl);
+    launch_tc_quadrature(phi, dphi, phl, w, u, dV, nao, N, ld, true, 1.0, part, M, err, st, drain, zhl, phl);
     int h = 0;
     HQ_CUDA(cudaMemcpyAsync(&h, err, sizeof(int), cudaMemcpyDeviceToHost, st));
     HQ_CUDA(cudaStreamSynchronize(st));
@@ -2469,8 +2493,7 @@ extern "C" int hqcgb_tc_quadrature(int nao, long long N, long long ld, const flo
     int *err = err_buf.as<int>();
     HQ_CUDA(cudaMemsetAsync(err, 0, sizeof(int), st));
     float *phl = hl, *zhl = hl + 2 * (size_t)nao * ldo;
-    launch_split_operand(phi, nullptr, nullptr, nullptr, nao, N, ld, ldo, 1.f, 0.f, phl, st);
-    launch_split_operand(phi, nullptr, w, nullptr, nao, N, ld, ldo, 1.f, 0.f, zhl, st);
+    launch_split_operand(phi, nullptr, w, nullptr, nao, N, ld, ldo, 1.f, 0.f, zhl, st, phl);
     launch_tc_quad_split(zhl, phl, nao, N, ldo, true, false, 1.0, part, M, err, st, drain, 0, true);
     int h = 0;
     HQ_CUDA(cudaMemcpyAsync(&h, err, sizeof(int), cudaMemcpyDeviceToHost, st));
