@@ -151,8 +151,8 @@ CONFIG = {"workload": "H54 bcc rs=1.31 gth-dzvp PBE 81^3 Gamma, SCF tol 1e-7 Ry 
 def psi_density_roofline(hbm_gbs, src, reps=5):
     """The orbital-density kernel (the dominant grid kernel: tcgen05 3xTF32,
     HBM-bound) timed alone with CUDA events on its own stream at the H54
-    shapes: algorithmic bytes = the grid-major AO values and gradients it
-    streams once (4 x N x 288 fp32) + Y^T + rho and grad rho (4 x N fp64)."""
+    shapes: algorithmic bytes = the AO values and gradients it streams once
+    (4 x N x n_ao fp32) + Y^T + rho and grad rho (4 x N fp64)."""
     import torch
     from hqc_gb300 import _lib
     nao, N, nocc, ldk = 270, 531441, 27, 288
@@ -175,12 +175,12 @@ def psi_density_roofline(hbm_gbs, src, reps=5):
     cnt, tot = _lib.stage_stats()["psi_density"]
     _lib.profile(0)
     avg_s = tot / cnt / 1000.0
-    algo = 4 * N * ldk * 4 + 2 * 32 * ldk * 4 + 4 * N * 8
+    algo = 4 * N * nao * 4 + 2 * 32 * ldk * 4 + 4 * N * 8
     achieved = algo / avg_s / 1e9
     del phi, dphi
     torch.cuda.empty_cache()
     return {"bound": "hbm", "achieved": achieved, "peak": hbm_gbs, "unit": "GB/s",
-            "frac": achieved / hbm_gbs, "traffic": 2449091000 + 19750144,
+            "frac": achieved / hbm_gbs, "traffic": 2300000000 + 19430000,
             "kernel": "k_tc_psi_density_r<32> (orbital-form density + gradient, resident Y, H54 shapes)",
             "algorithmic_bytes": algo, "avg_ms": avg_s * 1e3, "launches": cnt,
             "peak_source": f"{src} (MEASURED_PEAKS.json hbm_gbs, burst)" if src == "measured" else src,
