@@ -705,7 +705,7 @@ def exchange_roofline(hbm_gbs, src, reps=5):
     achieved = algo / avg_s / 1e9
     return {"bound": "hbm", "achieved": achieved, "peak": hbm_gbs, "unit": "GB/s",
             "frac": achieved / hbm_gbs, "traffic": None,
-            "kernel": "k_exx_plane<float> + k_exx_column<float,1> + k_tc_quad_tma (Gram) + reduce "
+            "kernel": "k_exx_plane<float> + k_exx_column<float,1> + Gram matrix (tcgen05) + reduce "
                       "(HF exchange of one Fock build, H32 dzv 65^3)",
             "algorithmic_bytes": algo, "pairs": int(pairs), "avg_ms": avg_s * 1e3, "launches": reps,
             "peak_source": f"{src} (MEASURED_PEAKS.json hbm_gbs, burst)" if src == "measured" else src}
