@@ -304,24 +304,28 @@ __global__ void __launch_bounds__(32)
     for (int k = lane; k < n; k += 32) x[k] = 1.f + 0.37f * __sinf(0.7f * (float)k + 1.3f * (float)j);
     __syncwarp();
     for (int it = 0; it < 3; ++it) {
-      // L y = P x
-      float x0 = x[0];
-      unsigned word = 0;
-      for (int k = 0; k < n - 1; ++k) {
-        if ((k & 31) == 0) word = swap[k >> 5];
-        float x1 = x[k + 1];
-        if ((word >> (k & 31)) & 1) {
-          const float t = x0;
-          x0 = x1;
-          x1 = t;
+      // L y = P x, by the first lane alone: it stores x[k] and reads x[k + 1]
+      if (lane == 0) {
+        float y = x[0];
+        unsigned word = 0;
+        for (int k = 0; k < n - 1; ++k) {
+          if ((k & 31) == 0) word = swap[k >> 5];
+          float x1 = x[k + 1];
+          if ((word >> (k & 31)) & 1) {
+            const float t = y;
+            y = x1;
+            x1 = t;
+          }
+          x1 -= lm[k] * y;
+          x[k] = y;
+          y = x1;
         }
-        x1 -= lm[k] * x0;
-        if (lane == 0) x[k] = x0;
-        x0 = x1;
+        x[n - 1] = y;
       }
       __syncwarp();
       // U z = y
-      float z1 = x0 / u1[n - 1], z2 = 0.f;
+      float z1 = x[n - 1] / u1[n - 1], z2 = 0.f;
+      __syncwarp();
       if (lane == 0) x[n - 1] = z1;
       if (n > 1) {
         z2 = z1;

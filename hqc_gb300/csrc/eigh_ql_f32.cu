@@ -9,8 +9,8 @@
 //     column and the product A v through distributed shared memory, two cluster
 //     barriers a step;
 //  2. k_ql_rotations (one warp): the QL iteration on d and e alone, its Givens
-//     rotations written down sweep by sweep (the search for a small off-diagonal
-//     element over 32 lanes);
+//     rotations written down sweep by sweep by one lane (the search for a small
+//     off-diagonal element over all 32);
 //  3. k_ql_apply: the rotations on the eigenvector matrix, a thread per row;
 //  4. k_ql_back: the reflectors, a warp per eigenvector;
 //  5. k_ql_store: ascending order.
@@ -216,44 +216,40 @@ __global__ void __launch_bounds__(32)
         fail = 1;
         break;
       }
-      // one sweep; every lane follows the chain, the first one stores
-      float g = (d[l + 1] - d[l]) / (2.f * e[l]);
-      float r = e_hypot(g, 1.f);
-      g = d[m] - d[l] + e[l] / (g + e_copysign(r, g));
-      float s = 1.f, c = 1.f, pp = 0.f;
-      int i, nrot = 0;
-      bool early = false;
-      float ei = e[m - 1], di = d[m - 1], di1 = d[m];
-      for (i = m - 1; i >= l; --i) {
-        const float en = i > l ? e[i - 1] : 0.f, dn = i > l ? d[i - 1] : 0.f;
-        const float f = s * ei, b = c * ei;
-        r = e_hypot(f, g);
-        if (lane == 0) e[i + 1] = r;
-        if (r == 0.f) {
-          if (lane == 0) {
+      // one sweep by the first lane alone: it reads d and e two elements ahead of
+      // where it stores them, which no other lane may do unordered
+      int nrot = 0;
+      if (lane == 0) {
+        float g = (d[l + 1] - d[l]) / (2.f * e[l]);
+        float r = e_hypot(g, 1.f);
+        g = d[m] - d[l] + e[l] / (g + e_copysign(r, g));
+        float s = 1.f, c = 1.f, pp = 0.f;
+        bool early = false;
+        float ei = e[m - 1], di = d[m - 1], di1 = d[m];
+        for (int i = m - 1; i >= l; --i) {
+          const float en = i > l ? e[i - 1] : 0.f, dn = i > l ? d[i - 1] : 0.f;
+          const float f = s * ei, b = c * ei;
+          r = e_hypot(f, g);
+          e[i + 1] = r;
+          if (r == 0.f) {
             d[i + 1] = di1 - pp;
             e[m] = 0.f;
+            early = true;
+            break;
           }
-          early = true;
-          break;
-        }
-        s = f / r;
-        c = g / r;
-        g = di1 - pp;
-        r = __fmaf_rn(2.f * c, b, __fmul_rn(di - g, s));
-        pp = s * r;
-        if (lane == 0) {
+          s = f / r;
+          c = g / r;
+          g = di1 - pp;
+          r = __fmaf_rn(2.f * c, b, __fmul_rn(di - g, s));
+          pp = s * r;
           d[i + 1] = g + pp;
           rot[pos + nrot] = make_float2(c, s);
+          g = c * r - b;
+          ++nrot;
+          di1 = di;
+          di = dn;
+          ei = en;
         }
-        g = c * r - b;
-        ++nrot;
-        di1 = di;
-        di = dn;
-        ei = en;
-      }
-      __syncwarp();
-      if (lane == 0) {
         if (!early) {
           d[l] = di1 - pp;
           e[l] = g;
@@ -261,11 +257,12 @@ __global__ void __launch_bounds__(32)
         }
         sweeps[ns] = QlSweep{m, pos, nrot};
       }
-      pos += nrot;
+      __syncwarp();  // d and e are read by all lanes again
+      pos += __shfl_sync(0xffffffffu, nrot, 0);
       ++ns;
-      __syncwarp();
     }
   }
+  __syncwarp();
   for (int i = lane; i < n; i += 32) dout[i] = d[i];
   if (lane == 0) {
     info[0] = ns;
