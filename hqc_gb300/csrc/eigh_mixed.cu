@@ -561,7 +561,8 @@ extern "C" int hqcgb_eigh_mixed(int n, const double *A, double *w, double *V, vo
     ws.emax = d + 6 * nn;
     float *f = reinterpret_cast<float *>(d + f64);
     ws.A32 = f; ws.V32 = f + nn; ws.work32 = f + 2 * nn; ws.w32 = f + 3 * nn;
-    ws.f32scr = f + 3 * nn + 2 * n + 64;
+    // 16-byte aligned for either FP32 solver's scratch (3 nn + 2 n is odd for odd n)
+    ws.f32scr = f + (3 * nn + 2 * (size_t)n + 3) / 4 * 4;
     ws.status = reinterpret_cast<int *>(f + f32);
     ws.iwork = ws.status + 64;
     HQ_CUDA(cudaMemsetAsync(ws.status, 0, sizeof(int), st));

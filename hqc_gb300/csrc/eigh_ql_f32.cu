@@ -379,6 +379,7 @@ size_t eigh_ql_f32_scratch_floats(int n) {
 // A (n x n) -> w ascending, V columns; Zt: n x n scratch; status < 0 when a limit was hit.
 void eigh_ql_f32(int n, const float *A, float *V, float *w, float *Zt, float *scr, int *status, cudaStream_t st) {
   HQ_STAGE(ST_JACOBI, st);
+  HQ_REQUIRE((uintptr_t)scr % sizeof(float2) == 0, "QL scratch must be 8-byte aligned");
   float2 *rot = reinterpret_cast<float2 *>(scr);
   float *hv = scr + 2 * (size_t)kQlRot * n * n, *dg = hv + (size_t)n * n, *eg = dg + n, *taug = eg + n, *dout = taug + n;
   QlSweep *sweeps = reinterpret_cast<QlSweep *>(dout + n);
