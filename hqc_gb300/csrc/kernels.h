@@ -1,6 +1,7 @@
 // Host-side launchers of the hqcgb kernels (internal header).
 #pragma once
 #include <cuda_runtime.h>
+#include <vector>
 
 namespace hqcgb {
 
@@ -20,26 +21,29 @@ void launch_sum_partials(const double *part, int nblk, int stride, int nout, dou
                          double *out, bool accumulate, cudaStream_t st);
 
 // quad_f64.cu: FP64 quadratures on the tensor cores (digits of 7 bits).
-// Workspace of one plan: digits, exponents and scales of the weighted operand
-// (A), of the AOs (B) and, for a second operand of quad64_pair, X; the tables
-// of block maxima of the AOs and their gradients, of the weights, and of other
-// operands; FP64 partial tiles; the tensor-core error word.
+// Workspace of one plan: digits and exponents of the weighted operand (A), of the
+// AOs (B) and, for a second operand of quad64_pair, X; the bricks of its grid;
+// FP64 partial tiles; the tensor-core error word.
 struct Quad64 {
-  int n = 0;
+  int n = 0, ng = 0, stages = 0;
   char *A = nullptr, *B = nullptr, *X = nullptr;
   int *eA = nullptr, *eB = nullptr, *eX = nullptr, *err = nullptr;
-  double *sA = nullptr, *sB = nullptr, *sX = nullptr, *part = nullptr;
-  float *tab = nullptr, *wtab = nullptr, *xtab = nullptr;
+  int *first = nullptr;  // quad64_first on the device; stages = its last
+  double *part = nullptr;
 };
-size_t quad64_operand_bytes(int n, long long N);
-long long quad64_table(long long N);  // entries of a maxima table's row
+std::vector<int> quad64_first(int ng);
+// bytes and exponents of an operand: a field of the grid, or rows of K values
+size_t quad64_grid_bytes(int n, int ng);
+size_t quad64_linear_bytes(int n, long long K);
+size_t quad64_grid_exponents(int n, int ng);
+size_t quad64_linear_exponents(int n, long long K);
 size_t quad64_partial_doubles(int n);
-// AOs (and gradients) of a geometry: maxima, exponents and digits (B)
-void quad64_basis(const Quad64 &q, const double *phi, const double *dphi, long long N, cudaStream_t st);
+// AOs of a geometry: exponents and digits (B)
+void quad64_basis(const Quad64 &q, const double *phi, long long N, cudaStream_t st);
 // M = scale sum_g phi_p w phi_q (w NULL: 1), both after quad64_basis
 void quad64_weighted(const Quad64 &q, const double *phi, const double *w, long long N, double scale, double *M,
                      cudaStream_t st);
-// M = Z phi^T + phi Z^T, Z = 0.5 w phi + dV u . dphi (after quad64_basis with dphi)
+// M = Z phi^T + phi Z^T, Z = 0.5 w phi + dV u . dphi (after quad64_basis)
 void quad64_gga(const Quad64 &q, const double *phi, const double *dphi, const double *w, const double *u, double dV,
                 long long N, double *M, cudaStream_t st);
 // M (+)= Q Q^T

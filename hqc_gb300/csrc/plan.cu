@@ -488,18 +488,23 @@ static void create(const hqcgb_params *in, hqcgb_plan *p) {
   if (!p->mixed || (p->hf && !p->exx_fused)) {
     // FP64 quadratures: Fock, V, S~ and the Gram matrix of the FP64 exchange
     const long long gK = p->exx_fused && !p->mixed ? (long long)p->exx_g * exx_pair_len(p->ng) : 0;
-    const long long most = std::max(N, gK), tabN = quad64_table(N);
     const bool legacy = p->hf && !p->exx_fused;
+    const size_t field = quad64_grid_bytes(nao, p->ng), fexp = quad64_grid_exponents(nao, p->ng);
     Quad64 &q = p->q64;
     q.n = nao;
-    q.B = p->alloc<char>(quad64_operand_bytes(nao, N));
-    if (!p->mixed || legacy) q.A = p->alloc<char>(quad64_operand_bytes(nao, most));
-    if (legacy) q.X = p->alloc<char>(quad64_operand_bytes(nao, N));
-    for (int **e : {&q.eA, &q.eB, &q.eX}) *e = p->alloc<int>(nao);
-    for (double **sc : {&q.sA, &q.sB, &q.sX}) *sc = p->alloc<double>(nao);
-    q.tab = p->alloc<float>((size_t)(p->gga && !p->mixed ? 4 : 1) * nao * tabN);
-    q.wtab = p->alloc<float>(4 * tabN);
-    if (p->hf) q.xtab = p->alloc<float>((size_t)nao * quad64_table(most));
+    q.ng = p->ng;
+    const std::vector<int> first = quad64_first(p->ng);
+    q.stages = first.back();
+    q.first = p->alloc<int>(first.size());
+    upload(q.first, first.data(), first.size() * sizeof(int));
+    q.B = p->alloc<char>(field);
+    q.eB = p->alloc<int>(fexp);
+    q.A = p->alloc<char>(std::max(field, quad64_linear_bytes(nao, gK)));
+    q.eA = p->alloc<int>(std::max(fexp, quad64_linear_exponents(nao, gK)));
+    if (legacy) {
+      q.X = p->alloc<char>(field);
+      q.eX = p->alloc<int>(fexp);
+    }
     q.part = p->alloc<double>(quad64_partial_doubles(nao));
     if (!p->tc_err) {
       p->tc_err = p->alloc<int>(1);
@@ -921,7 +926,7 @@ static void geometry(Ctx &c, const double *xp_dev) {
     launch_phi(p->F1d, p->coef, p->ao_l, p->ao_cart, p->nb, p->nprim, n, p->ng, p->phi, p->dphi,
                c.st);
   if (p->d64.n) density64_basis(p->d64, p->phi, p->gga ? p->dphi : nullptr, N, c.st);
-  if (p->q64.n) quad64_basis(p->q64, p->phi, p->gga && !p->mixed ? p->dphi : nullptr, N, c.st);
+  if (p->q64.n) quad64_basis(p->q64, p->phi, N, c.st);
   if (p->mixed) {
     launch_to_float((long long)p->n * 3 * p->ng * P.n_prim * 6, p->F1d, p->F1d32, c.st);
     launch_phi32(p->F1d32, p->coef, p->ao_l, p->ao_cart, p->nb, p->nprim, n, p->ng, p->ld, p->phi32,

@@ -8,27 +8,39 @@
 // matrix multiplication by using fast routines of matrix multiplication and
 // its applications", Numer. Algorithms 59 (2012) 95-118):
 //   x = 2^e sum_s d_s 128^-(s + 1),  s = 0..7, d_s integers in [-64, 64],
-// with one power of two e for a row, |x| <= 2^(e - 1): 56 bits below the row's
-// largest element, where FP64 keeps 53.  A product of digits is at most 2^12,
-// so 512 points of the at most 8 products s + t = d fit FP32's 24 bits and the
-// sums P_d (kind::f16, FP32 accumulators in TMEM, one per d = 0..7) are exact;
-// the 36 products with s + t <= 7 are formed, the others are below 2^-56 of
-// the row maxima's product.  The drains add the P_d to integers of 64 bits, so
-// a CTA's share of the sum has one rounding, and the result's error is that of
-// the digits: a rounding of 2^-57 of a row's maximum a point, which averages
-// out, against the rounding of every FP64 product and partial sum before.
+// with one power of two e for a row and a block of points, |x| <= 2^(e - 1): 56
+// bits below the largest element of the row in that block, where FP64 keeps 53 of
+// each.  The blocks are bricks of the grid, at most 8 points a side (512
+// consecutive ones where the operand is no grid field): within a brick an AO
+// changes little, so an element of M made of two AOs' tails keeps the relative
+// accuracy of an FP64 sum, which one power of two for a whole row would cost it.
+// Error over the sum of the absolute terms, FP64 sums / a power of two a row / a
+// brick, emulated, dzvp, box 9.75 Bohr, 49^3: elements of 1e-2 of the largest and
+// more 3e-16 / 2e-16 / 3e-16, of 1e-6 to 1e-4 4e-16 / 1e-12 / 6e-16, of 1e-8 to 1e-6
+// 4e-16 / 3e-11 / 8e-16.
 //
-// Operands are stored by blocks of 32 points, [block][row block][pair][row]
-// [128 bytes]: a 128-byte row holds 32 points of two digits, already in the
-// K-major SW128 pattern that the MMA reads, so plain bulk copies fill the
-// ring.  One CTA an SM: a persistent share of the points for one 128 x 64
-// destination tile, a copy thread, an MMA thread and eight drain warps.
+// A product of digits is at most 2^12, so the points of a block and the at most 8
+// products s + t = d fit FP32's 24 bits and the sums P_d (kind::f16, FP32
+// accumulators in TMEM, one per d = 0..7) are exact; the 36 products with
+// s + t <= 7 are formed, the others are below 2^-56 of the maxima's product.  The
+// drains add a block's P_d to an integer of 64 bits, round it once and add it to
+// the tile's FP64 sums.
+//
+// Operands are stored by stages of 32 points, [stage][pair][row][128 bytes]: a
+// 128-byte row holds 32 points of two digits, already in the K-major SW128 pattern
+// that the MMA reads, so plain bulk copies fill the ring.  One CTA an SM: a
+// persistent share of the stages for one 128 x 64 destination tile, a copy thread,
+// an MMA warp and eight drain warps.  The MMA warp stays together and one elected lane
+// issues: with a branch on the lane number the descriptors of every MMA go through
+// ordinary registers (193 -> 146 us at 64 AOs, 65^3).  The digit pass takes a brick a block and a
+// row a warp, whose maximum gives the exponent of the values it holds.
 //
 // Bounds.  One 32-point stage is 72 MMAs of 128 x 64 x 16: the kernel is bound
 // by the tensor pipe, at 36 products a term.  Measured, digits
 // of the weighted operand and sums included, FP64 pipe -> this: 64 AOs and 65^3
-// points 2.24 -> 0.24 ms, 70 AOs and 49^3 points with the gradient term 2.21 ->
-// 0.31 ms, 8 AOs and 41^3 points 0.57 -> 0.12 ms.
+// points 2.24 -> 0.29 ms, 70 AOs and 49^3 points with the gradient term 2.21 ->
+// 0.30 ms, 8 AOs and 41^3 points 0.57 -> 0.07 ms (with a power of two a row 0.24,
+// 0.32 and 0.08).
 #include <algorithm>
 #include <cmath>
 
@@ -40,7 +52,8 @@ namespace hqcgb {
 using namespace tc;
 
 constexpr int kQfK = 32;                                // points per stage
-constexpr int kQfChain = 16;                            // stages per TMEM sum (512 points)
+constexpr int kQfSide = 8;                              // most points a side of a brick
+constexpr int kQfBlk = 512;                             // most points of a block: what FP32 adds exactly
 constexpr int kQfM = 128, kQfN = 64;
 constexpr int kQfRing = 2;
 constexpr uint32_t kQfPairA = kQfM * 128, kQfPairB = kQfN * 128;
@@ -50,15 +63,33 @@ constexpr size_t kQfSmem = kQfRing * kQfStage + 1024;   // + alignment to the sw
 constexpr int kQfDrainWarps = 8;
 constexpr int kQfThreads = (kQfDrainWarps + 2) * 32;
 constexpr int kQfMaxTiles = (kMaxNao / kQfM) * (kMaxNao / kQfN);
-constexpr int kQfBlk = 512;                             // points per entry of the maxima tables
+constexpr int kQfBad = 1 << 20;                         // exponent of a block with a value that is not finite
 static_assert(kQfSmem <= 227 * 1024, "FP64 quadrature ring above 227 KB");
+static_assert(kQfSide * kQfSide * kQfSide <= kQfBlk, "a brick is one block");
 
-int quad64_rows(int n) { return n <= 128 ? (n + 7) / 8 * 8 : 128; }
-int quad64_row_blocks(int n) { return n <= 128 ? 1 : ceil_div(n, 128); }
-size_t quad64_operand_bytes(int n, long long N) {
-  return (size_t)ceil_div(N, kQfK) * quad64_row_blocks(n) * quad64_rows(n) * 128 * kQfPairs;
+static int quad64_rows(int n) { return (n + 7) / 8 * 8; }  // the swizzle's period
+static size_t stage_bytes(int n) { return (size_t)quad64_rows(n) * 128 * kQfPairs; }
+static int quad64_parts(int ng) { return ceil_div(ng, kQfSide); }
+static long long quad64_linear_blocks(long long K) { return (K + kQfBlk - 1) / kQfBlk; }
+
+// Bricks: an axis is cut into `parts` nearly equal pieces; first[b] = the first
+// stage of brick b (x slowest), first[bricks] = all stages.
+std::vector<int> quad64_first(int ng) {
+  const int m = quad64_parts(ng);
+  std::vector<int> first(1, 0);
+  auto len = [&](int k) { return ng * (k + 1) / m - ng * k / m; };
+  for (int x = 0; x < m; ++x)
+    for (int y = 0; y < m; ++y)
+      for (int z = 0; z < m; ++z) first.push_back(first.back() + ceil_div(len(x) * len(y) * len(z), kQfK));
+  return first;
 }
-long long quad64_table(long long N) { return ceil_div(N, kQfBlk); }
+size_t quad64_grid_bytes(int n, int ng) { return (size_t)quad64_first(ng).back() * stage_bytes(n); }
+size_t quad64_linear_bytes(int n, long long K) { return (size_t)ceil_div(K, kQfK) * stage_bytes(n); }
+size_t quad64_grid_exponents(int n, int ng) {
+  const size_t m = quad64_parts(ng);
+  return m * m * m * quad64_rows(n);
+}
+size_t quad64_linear_exponents(int n, long long K) { return (size_t)quad64_linear_blocks(K) * quad64_rows(n); }
 
 static int quad64_tiles(int n, bool sym, unsigned char (*t)[2] = nullptr) {
   int cnt = 0;
@@ -81,106 +112,147 @@ size_t quad64_partial_doubles(int n) {
   return most;
 }
 
-// tab[row][block] = max |X[row][g]| over the block's points, rounded up to
-// FP32; NaN and infinity compare above every number by their bits.
-__global__ void __launch_bounds__(128)
-    k_qf_maxima(const double *__restrict__ X, long long N, float *__restrict__ tab) {
-  __shared__ unsigned s[4];
-  const long long g0 = (long long)blockIdx.x * kQfBlk;
-  const double *row = X + (long long)blockIdx.y * N;
-  unsigned v = 0;
-  for (int i = threadIdx.x; i < kQfBlk; i += 128)
-    if (g0 + i < N) v = max(v, __float_as_uint(__double2float_ru(fabs(row[g0 + i]))));
-  v = __reduce_max_sync(0xffffffffu, v);
-  if ((threadIdx.x & 31) == 0) s[threadIdx.x >> 5] = v;
-  __syncthreads();
-  if (threadIdx.x == 0)
-    tab[(long long)blockIdx.y * gridDim.x + blockIdx.x] =
-        __uint_as_float(max(max(s[0], s[1]), max(s[2], s[3])));
+// A form of the operand: values X (MODE 0), w X (1) or 0.5 w X + dV u . dX (2)
+// at the points of a grid in bricks (first) or in their order (first null).
+struct QfSource {
+  const double *X, *dX, *w, *u;
+  double dV;
+  int n, rows, ng, parts;
+  long long N;
+  const int *first;
+  int *e;      // [block][rows]
+  char *out;
+};
+
+constexpr int kQfFormRows = 8;                                // rows a block works on, a warp each
+constexpr int kQfChunk = 9, kQfRowLd = kQfBlk / 8 * kQfChunk + 4;  // doubles from a chunk of 8 points, a row to the
+                                                                   // next: no bank conflicts in either phase
+static size_t form_smem(int mode) {
+  return sizeof(double) * (kQfFormRows * kQfRowLd + (mode == 0 ? 0 : mode == 1 ? 1 : 4) * kQfBlk) + sizeof(int) * kQfBlk;
 }
 
-// Exponent and scale of every row: the largest |X| (w NULL), |w X| or, with
-// dtab and u, |0.5 w X + dV sum_c u_c dX_c| that the tables allow.  A row that
-// is not finite gets a NaN scale.
-__global__ void __launch_bounds__(128)
-    k_qf_exponents(const float *__restrict__ tab, const float *__restrict__ dtab, int n, int nb,
-                   const float *__restrict__ w, const float *__restrict__ u, float dV, int *__restrict__ e,
-                   double *__restrict__ scale) {
-  __shared__ unsigned s[4];
-  const int p = blockIdx.x;
-  unsigned v = 0;
-  for (int b = threadIdx.x; b < nb; b += 128) {
-    float m = tab[(long long)p * nb + b];
-    if (w) m = __fmul_ru(m, w[b]);
-    if (dtab) {
-      m *= 0.5f;
-      for (int c = 0; c < 3; ++c)
-        m = __fmaf_ru(__fmul_ru(dV, u[c * nb + b]), dtab[((long long)c * n + p) * nb + b], m);
-    }
-    v = max(v, __float_as_uint(m) & 0x7fffffffu);
-  }
-  v = __reduce_max_sync(0xffffffffu, v);
-  if ((threadIdx.x & 31) == 0) s[threadIdx.x >> 5] = v;
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    const float m = __uint_as_float(max(max(s[0], s[1]), max(s[2], s[3])));
-    int k = 0;
-    if (m > 0.f && m < INFINITY) frexpf(m, &k);  // m < 2^k
-    e[p] = k + 1;
-    scale[p] = m < INFINITY ? scalbn(1.0, k + 1) : NAN;
-  }
-}
-
-// Digits of X (MODE 0), w X (1) or 0.5 w X + dV u.dX (2) into the operand
-// layout; blockIdx.x = block of 32 points, a warp takes 8 rows x 4 chunks of
-// 8 points.  Points beyond N become zeros; rows beyond n are left alone (they
-// only reach destination rows and columns that nothing reads).
+// Grid (blocks of points, row groups).  A warp loads a row, neighbouring lanes
+// neighbouring points, and its maximum gives the exponent; then the warps take a
+// stage of all eight rows in turn, eight points of a row a lane, so that what they
+// store is 1 KB in one piece.  Points beyond a block's last become zeros; rows beyond
+// n are left alone (they only reach destination rows and columns that nothing reads).
 template <int MODE>
-__global__ void __launch_bounds__(256)
-    k_qf_digits(const double *__restrict__ X, const double *__restrict__ dX, const double *__restrict__ w,
-                const double *__restrict__ u, double dV, int n, long long N, int rb, int rbn,
-                const int *__restrict__ e, char *__restrict__ out) {
-  const int lane = threadIdx.x & 31, c = lane & 3;
-  const long long kb = blockIdx.x, g0 = kb * kQfK + c * 8;
-  const int cnt = (int)min(8LL, max(0LL, N - g0));
-  double wv[MODE ? 8 : 1], uv[MODE == 2 ? 24 : 1];
-  if (MODE)
-#pragma unroll
-    for (int i = 0; i < 8; ++i) wv[i] = i < cnt ? w[g0 + i] * (MODE == 2 ? 0.5 : 1.0) : 0.0;
-  if (MODE == 2)
-#pragma unroll
-    for (int d = 0; d < 3; ++d)
-#pragma unroll
-      for (int i = 0; i < 8; ++i) uv[d * 8 + i] = i < cnt ? dV * u[(long long)d * N + g0 + i] : 0.0;
-  for (int p = (threadIdx.x >> 5) * 8 + (lane >> 2); p < n; p += 64) {
-    const int ep = e[p];
-    QfPack pack;
-#pragma unroll
-    for (int i = 0; i < 8; ++i) {
-      double x = 0.0;
-      if (i < cnt) {
-        const long long at = (long long)p * N + g0 + i;
-        x = X[at];
-        if (MODE) x *= wv[i];
+__global__ void __launch_bounds__(kQfFormRows * 32) k_qf_digits(const QfSource a) {
+  extern __shared__ __align__(16) double s_x[];  // [rows][kQfRowLd]
+  double *s_w = s_x + kQfFormRows * kQfRowLd, *s_u = s_w + kQfBlk;
+  int *s_off = reinterpret_cast<int *>(s_w + (MODE == 0 ? 0 : MODE == 1 ? 1 : 4) * kQfBlk);  // the block's points
+  __shared__ int s_e[kQfFormRows];
+  const int b = blockIdx.x, tid = threadIdx.x;
+  int cnt, stage0;
+  long long base = 0;
+  int x0 = 0, y0 = 0, z0 = 0, sy = 1, sz = 1;
+  if (a.first) {
+    const int bz = b % a.parts, by = b / a.parts % a.parts, bx = b / (a.parts * a.parts);
+    auto cut = [&](int k) { return a.ng * k / a.parts; };
+    x0 = cut(bx);
+    y0 = cut(by);
+    z0 = cut(bz);
+    sy = cut(by + 1) - y0;
+    sz = cut(bz + 1) - z0;
+    cnt = (cut(bx + 1) - x0) * sy * sz;
+    stage0 = a.first[b];
+  } else {
+    base = (long long)b * kQfBlk;
+    cnt = (int)min((long long)kQfBlk, a.N - base);
+    stage0 = b * (kQfBlk / kQfK);
+  }
+  const int stages = (cnt + kQfK - 1) / kQfK, pts = stages * kQfK;
+  for (int k = tid; k < pts; k += kQfFormRows * 32) {
+    const int r = min(k, cnt - 1);  // beyond the last point: the last once more, times zero below
+    int off = r;
+    if (a.first) {
+      const int x = r / (sy * sz), q = r - x * (sy * sz), y = q / sz;
+      off = ((x0 + x) * a.ng + y0 + y) * a.ng + z0 + q - y * sz;
+    }
+    s_off[k] = off;
+    if (MODE) s_w[k] = k < cnt ? a.w[base + off] * (MODE == 2 ? 0.5 : 1.0) : 0.0;
+    if (MODE == 2)
+      for (int d = 0; d < 3; ++d) s_u[d * kQfBlk + k] = k < cnt ? a.dV * a.u[(long long)d * a.N + base + off] : 0.0;
+  }
+  __syncthreads();
+  const int lane = tid & 31, warp = tid >> 5;
+  for (int p0 = blockIdx.y * kQfFormRows; p0 < a.n; p0 += gridDim.y * kQfFormRows) {
+    const int p = p0 + warp;
+    if (p < a.n) {
+      const double *X = a.X + (long long)p * a.N + base;
+      const double *dX = MODE == 2 ? a.dX + (long long)p * a.N + base : nullptr;
+      unsigned top = 0;
+#pragma unroll 4
+      for (int k = lane; k < pts; k += 32) {
+        const int off = s_off[k];
+        double x = X[off];
+        if (MODE) x *= s_w[k];
+        else if (k >= cnt) x = 0.0;
         if (MODE == 2)
 #pragma unroll
-          for (int d = 0; d < 3; ++d) x += uv[d * 8 + i] * dX[(long long)d * n * N + at];
+          for (int d = 0; d < 3; ++d) x += s_u[d * kQfBlk + k] * dX[(long long)d * a.n * a.N + off];
+        s_x[warp * kQfRowLd + (k >> 3) * kQfChunk + (k & 7)] = x;
+        top = max(top, (unsigned)__double2hiint(x) & 0x7fffffffu);
       }
-      pack.put(i, x, ep);
+      top = __reduce_max_sync(0xffffffffu, top);
+      const int ex = (int)(top >> 20);  // every |x| < 2^(ex - 1022)
+      const int e = ex == 0x7ff ? kQfBad : ex - 1021;
+      if (lane == 0) {
+        s_e[warp] = e;
+        a.e[(long long)b * a.rows + p] = e;
+      }
     }
-    char *row = out + ((kb * rbn + p / rb) * kQfPairs * (long long)rb + p % rb) * 128;
-    const int r = p % rb;
-    pack.store(row, (long long)rb * 128, c, r);
+    __syncthreads();
+    const int r = lane >> 2, c = lane & 3;
+    if (p0 + r < a.n) {
+      const int e = s_e[r];
+      for (int st = warp; st < stages; st += kQfFormRows) {
+        const double *x = s_x + r * kQfRowLd + (st * 4 + c) * kQfChunk;
+        QfPack pack;
+#pragma unroll
+        for (int i = 0; i < 8; ++i) pack.put(i, x[i], e);
+        char *row = a.out + ((long long)(stage0 + st) * kQfPairs * a.rows + p0 + r) * 128;
+        pack.store(row, (long long)a.rows * 128, c, r);  // p0 is a multiple of 8
+      }
+    }
+    __syncthreads();
   }
 }
 
 struct QfArgs {
   const char *A, *B;
-  double *part;  // [group][tile][128][64]
+  const int *eA, *eB;  // [block][rows]
+  const int *first;    // first stage of every block, or null: 16 stages a block
+  double *part;        // [group][tile][128][64]
   int *err;
-  long long stages;
-  int n, rb, rbn, groups, tiles;
+  int stages, blocks, n, rows, groups, tiles;
   unsigned char tile[kQfMaxTiles][2];  // 128-row block of A, 64-row block of B
+};
+
+// The chains of group g's share of the stages, in order: stages [s, e) of block b.
+struct QfChains {
+  const QfArgs &a;
+  int s, e, end, b;
+  __device__ __forceinline__ int first(int k) const { return a.first ? a.first[k] : min(k * (kQfBlk / kQfK), a.stages); }
+  __device__ __forceinline__ QfChains(const QfArgs &a_, int g) : a(a_) {
+    s = e = (int)((long long)a.stages * g / a.groups);
+    end = (int)((long long)a.stages * (g + 1) / a.groups);
+    b = s / (kQfBlk / kQfK);  // a block is at most 16 stages
+    if (a.first)
+      for (int hi = a.blocks; hi - b > 1;) {
+        const int mid = (b + hi) / 2;
+        if (a.first[mid] <= s) b = mid;
+        else hi = mid;
+      }
+    --b;
+  }
+  __device__ __forceinline__ bool next() {
+    s = e;
+    if (s >= end) return false;
+    ++b;
+    e = min(end, first(b + 1));
+    return true;
+  }
 };
 
 struct QfPipe {
@@ -195,9 +267,6 @@ __global__ void __launch_bounds__(kQfThreads, 1) k_qf_gemm(const __grid_constant
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int tile = blockIdx.x, g = blockIdx.y;
   const int mt = a.tile[tile][0], ct = a.tile[tile][1];
-  const long long s0 = a.stages * g / a.groups;
-  const int nst = (int)(a.stages * (g + 1) / a.groups - s0);
-  const int nchain = (nst + kQfChain - 1) / kQfChain;
   const int rows_b = min(kQfN, a.n - ct * kQfN);            // columns that are read
   const int nn = (rows_b + 15) / 16 * 16;                   // MMA N
   if (tid == 0) {
@@ -214,45 +283,50 @@ __global__ void __launch_bounds__(kQfThreads, 1) k_qf_gemm(const __grid_constant
   __syncthreads();
   tc_fence_after();
 
+  const uint32_t tmem = P.tmem_base;
   bool ok = true;
   if (warp == kQfDrainWarps + 1) {
     if (lane == 0) {
-      // rows of A's block and of B's, in steps of 8 (the swizzle's period), within the stored block
-      const int brow = ct * kQfN, bblk = brow / a.rb, boff = brow % a.rb;
-      const uint32_t na = (uint32_t)min(a.rb, (a.n - mt * kQfM + 7) / 8 * 8) * 128u;
-      const uint32_t nb = (uint32_t)min(a.rb - boff, (rows_b + 7) / 8 * 8) * 128u;
-      const long long pair = (long long)a.rb * 128, blk = kQfPairs * pair;
-      for (int st = 0; st < nst; ++st) {
-        const int slot = st % kQfRing, use = st / kQfRing;
-        if (use > 0 && !mbar_wait(&P.empty[slot], (unsigned)((use - 1) & 1), a.err, 61)) {
-          ok = false;
-          break;
+      const uint32_t na = (uint32_t)min(kQfM, a.rows - mt * kQfM) * 128u;
+      const uint32_t nb = (uint32_t)min(kQfN, a.rows - ct * kQfN) * 128u;
+      const long long pair = (long long)a.rows * 128;
+      int it = 0;
+      for (QfChains c(a, g); ok && c.next();)
+        for (int s = c.s; s < c.e; ++s, ++it) {
+          const int slot = it % kQfRing, use = it / kQfRing;
+          if (use > 0 && !mbar_wait(&P.empty[slot], (unsigned)((use - 1) & 1), a.err, 61)) {
+            ok = false;
+            break;
+          }
+          mbar_expect_tx(&P.full[slot], kQfPairs * (na + nb));
+          const uint32_t dst = smem_u32(sm + slot * kQfStage);
+          const char *srcA = a.A + s * kQfPairs * pair + (long long)mt * kQfM * 128;
+          const char *srcB = a.B + s * kQfPairs * pair + (long long)ct * kQfN * 128;
+          for (int q = 0; q < kQfPairs; ++q) {
+            bulk_copy(dst + q * kQfPairA, srcA + q * pair, na, &P.full[slot]);
+            bulk_copy(dst + kQfOffB + q * kQfPairB, srcB + q * pair, nb, &P.full[slot]);
+          }
         }
-        mbar_expect_tx(&P.full[slot], kQfPairs * (na + nb));
-        const uint32_t dst = smem_u32(sm + slot * kQfStage);
-        const char *srcA = a.A + ((s0 + st) * a.rbn + mt) * blk;
-        const char *srcB = a.B + ((s0 + st) * a.rbn + bblk) * blk + (long long)boff * 128;
-        for (int q = 0; q < kQfPairs; ++q) {
-          bulk_copy(dst + q * kQfPairA, srcA + q * pair, na, &P.full[slot]);
-          bulk_copy(dst + kQfOffB + q * kQfPairB, srcB + q * pair, nb, &P.full[slot]);
-        }
-      }
     }
   } else if (warp == kQfDrainWarps) {
-    if (lane == 0) {
+    {
       // kind::f16, D = F32, A = B = BF16, both K-major
       const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(nn >> 3) << 17) |
                              ((uint32_t)(kQfM >> 4) << 24);
-      for (int j = 0, st = 0; j < nchain && ok; ++j) {
+      QfChains c(a, g);
+      for (int j = 0, it = 0; ok && c.next(); ++j) {
         if (j > 0 && !mbar_wait(&P.acc_empty, (unsigned)((j - 1) & 1), a.err, 64)) ok = false;
+        ok = __all_sync(0xffffffffu, ok);
         tc_fence_after();
-        const int end = min(nst, (j + 1) * kQfChain);
+        const int end = it + c.e - c.s;
         bool first = true;
-        for (; st < end && ok; ++st) {
-          const int slot = st % kQfRing, use = st / kQfRing;
+        for (; it < end && ok; ++it) {
+          const int slot = it % kQfRing, use = it / kQfRing;
           if (!mbar_wait(&P.full[slot], (unsigned)(use & 1), a.err, 62)) ok = false;
+          ok = __all_sync(0xffffffffu, ok);
           tc_fence_after();
-          if (ok) {
+          const bool el = elect();
+          if (ok && el) {
             const uint64_t dA = sdesc(smem_u32(sm + slot * kQfStage)), dB = dA + (kQfOffB >> 4);
 #pragma unroll 1
             for (int ks = 0; ks < kQfK / 16; ++ks) {
@@ -262,69 +336,88 @@ __global__ void __launch_bounds__(kQfThreads, 1) k_qf_gemm(const __grid_constant
                 const uint64_t da = dA + (uint32_t)((s >> 1) * (kQfPairA >> 4) + (s & 1) * 4 + 2 * ks);
 #pragma unroll
                 for (int t = 0; t < kQfDigits - s; ++t)
-                  mma_bf16(P.tmem_base + (s + t) * kQfN, da,
+                  mma_bf16(tmem + (s + t) * kQfN, da,
                            dB + (uint32_t)((t >> 1) * (kQfPairB >> 4) + (t & 1) * 4 + 2 * ks), idesc,
                            !(first && ks == 0 && s == 0));
               }
             }
-            first = false;
           }
-          mma_commit(&P.empty[slot]);
+          first = false;
+          if (el) mma_commit(&P.empty[slot]);
         }
-        mma_commit(&P.acc_full);
+        if (elect()) mma_commit(&P.acc_full);
       }
     }
   } else {
     // warp w owns TMEM lanes 32 (w % 4) .. and columns 32 (w / 4) .. + 31 of every P_d
-    const int c0 = (warp >> 2) * 32;
-    const uint32_t base = P.tmem_base + ((uint32_t)((warp & 3) * 32) << 16) + c0;
-    long long hi[32], lo[32];  // sum_d P_d 128^(3 - d), d < 4, and the same of d - 4
+    const int c0 = (warp >> 2) * 32, row = (warp & 3) * 32 + lane;
+    const uint32_t base = tmem + ((uint32_t)((warp & 3) * 32) << 16) + c0;
+    const int ra = min(mt * kQfM + row, a.n - 1), rb = min(ct * kQfN + c0 + lane, a.n - 1);
+    double acc[32];
 #pragma unroll
-    for (int i = 0; i < 32; ++i) hi[i] = lo[i] = 0;
-    for (int j = 0; j < nchain; ++j) {
-      if (ok && !mbar_wait(&P.acc_full, (unsigned)(j & 1), a.err, 63)) ok = false;
+    for (int i = 0; i < 32; ++i) acc[i] = 0.0;
+    QfChains c(a, g);
+    for (int j = 0; c.next(); ++j) {
+      const int ea = a.eA[(long long)c.b * a.rows + ra], eb = a.eB[(long long)c.b * a.rows + rb];
+      if (!mbar_wait(&P.acc_full, (unsigned)(j & 1), a.err, 63)) ok = false;
+      // a warp's lanes stay together: the loads below and the shuffles are the warp's
+      ok = __all_sync(0xffffffffu, ok);
+      if (!ok) break;
       tc_fence_after();
-      if (ok) {
+      // sum_d P_d 128^(5 - d) / 2, 63 bits before the one rounding; 2^(eA + eB - 53) of it is the block's sum
+      long long x[32];
 #pragma unroll
-        for (int q = 0; q < 8; ++q) {
-          uint32_t v[kQfDigits][4];
+      for (int q = 0; q < 8; ++q) {
+        uint32_t v[kQfDigits][4];
 #pragma unroll
-          for (int d = 0; d < kQfDigits; ++d) tmem_ld4_nowait(base + d * kQfN + q * 4, v[d]);
-          tmem_wait_ld();
+        for (int d = 0; d < kQfDigits; ++d) tmem_ld4_nowait(base + d * kQfN + q * 4, v[d]);
+        tmem_wait_ld();
 #pragma unroll
-          for (int i = 0; i < 4; ++i)
+        for (int i = 0; i < 4; ++i) {
+          long long hi = 0, lo = 0;
 #pragma unroll
-            for (int d = 0; d < 4; ++d) {
-              hi[q * 4 + i] += (long long)__float2int_rn(__uint_as_float(v[d][i])) * (1 << (7 * (3 - d)));
-              lo[q * 4 + i] += (long long)__float2int_rn(__uint_as_float(v[d + 4][i])) * (1 << (7 * (3 - d)));
-            }
+          for (int d = 0; d < 4; ++d) {
+            hi += (long long)__float2int_rn(__uint_as_float(v[d][i])) * (1 << (7 * (3 - d)));
+            lo += (long long)__float2int_rn(__uint_as_float(v[d + 4][i])) * (1 << (7 * (3 - d)));
+          }
+          x[q * 4 + i] = (hi << 18) + (lo >> 10);
         }
       }
       tc_fence_before();
       mbar_arrive(&P.acc_empty);
+      // the conversions stay behind the arrival: they run beside the next block's MMAs
+#pragma unroll
+      for (int i = 0; i < 32; ++i) asm volatile("" : "+l"(x[i]));
+#pragma unroll
+      for (int i = 0; i < 32; ++i) {
+        const int ei = ea + __shfl_sync(0xffffffffu, eb, i);
+        const double y = (double)x[i];
+        const int h = __double2hiint(y), ey = ((h >> 20) & 0x7ff) + ei - 53;
+        if (ei >= kQfBad / 2) acc[i] = NAN;
+        else if (ey >= 0x7ff) acc[i] += h < 0 ? -INFINITY : INFINITY;
+        else if (x[i] != 0 && ey > 0) acc[i] += __hiloint2double(h + (ei - 53) * (1 << 20), __double2loint(y));
+      }
     }
-    const int row = (warp & 3) * 32 + lane;
     if (ok && mt * kQfM + row < a.n) {
       double *out = a.part + (((long long)g * a.tiles + tile) * kQfM + row) * kQfN + c0;
 #pragma unroll
       for (int i = 0; i < 32; ++i)
-        if (c0 + i < rows_b) out[i] = fma((double)lo[i], 0x1p-28, (double)hi[i]);
+        if (c0 + i < rows_b) out[i] = acc[i];
     }
   }
   tc_fence_before();
   __syncthreads();
   if (warp == kQfDrainWarps) {
     tc_fence_after();
-    tmem_dealloc(P.tmem_base, kQfDigits * kQfN);
+    tmem_dealloc(tmem, kQfDigits * kQfN);
   }
 }
 
-// M (+)= scale 2^(eA + eB) 2^-35 sum over groups; sym: (p, q) from the upper
-// triangle; tr: M_pq = v_pq + v_qp.  A block takes 32 columns of a row, eight
-// threads a value.
+// M (+)= scale sum over groups; sym: (p, q) from the upper triangle; tr: M_pq =
+// v_pq + v_qp.  A block takes 32 columns of a row, eight threads a value.
 __global__ void __launch_bounds__(256)
-    k_qf_reduce(const __grid_constant__ QfArgs a, int sym, int tr, double scale, const double *__restrict__ sA,
-                const double *__restrict__ sB, int accumulate, double *__restrict__ M) {
+    k_qf_reduce(const __grid_constant__ QfArgs a, int sym, int tr, double scale, int accumulate,
+                double *__restrict__ M) {
   __shared__ double sh[8][33];
   const int p = blockIdx.y, q = blockIdx.x * 32 + (threadIdx.x & 31), part = threadIdx.x >> 5;
   auto value = [&](int r, int c) {
@@ -334,7 +427,7 @@ __global__ void __launch_bounds__(256)
     const double *src = a.part + ((long long)t * kQfM + r % kQfM) * kQfN + c % kQfN;
     double s = 0;
     for (int g = part; g < a.groups; g += 8) s += src[(long long)g * a.tiles * kQfM * kQfN];
-    return s * sA[r] * sB[c];
+    return s;
   };
   double s = 0;
   if (q < a.n) {
@@ -345,104 +438,96 @@ __global__ void __launch_bounds__(256)
   __syncthreads();
   if (part == 0 && q < a.n) {
     for (int k = 1; k < 8; ++k) s += sh[k][threadIdx.x];
-    s *= 0x1p-35 * scale;
+    s *= scale;
     double *m = M + (long long)p * a.n + q;
     *m = accumulate ? *m + s : s;
   }
 }
 
-static void maxima(const double *X, int rows, long long N, float *tab, cudaStream_t st) {
-  k_qf_maxima<<<dim3((unsigned)quad64_table(N), rows), 128, 0, st>>>(X, N, tab);
-  HQ_LAUNCH_CHECK();
+// Digits of an operand; ng > 0: a field of that grid, in bricks.
+struct QfForm {
+  int mode = 0;
+  const double *X = nullptr, *dX = nullptr, *w = nullptr, *u = nullptr;
+  double dV = 0.0;
+};
+static int blocks_of(const Quad64 &q, long long N, bool grid) {
+  return grid ? (int)quad64_grid_exponents(q.n, q.ng) / quad64_rows(q.n) : (int)quad64_linear_blocks(N);
+}
+static void form(const Quad64 &q, const QfForm &f, long long N, bool grid, int *e, char *out, cudaStream_t st) {
+  QfSource a{f.X, f.dX, f.w, f.u, f.dV, q.n, quad64_rows(q.n), q.ng, quad64_parts(q.ng), N, grid ? q.first : nullptr,
+             e, out};
+  const int blocks = blocks_of(q, N, grid), groups = ceil_div(q.n, kQfFormRows);
+  // few bricks: the rows over several blocks, until there are eight blocks an SM
+  const dim3 g(blocks, std::max(1, std::min(groups, ceil_div(8 * 152, blocks))));
+  const size_t smem = form_smem(f.mode);
+  auto go = [&](auto kernel) {
+    ensure_dyn_smem((const void *)kernel, smem);
+    kernel<<<g, kQfFormRows * 32, smem, st>>>(a);
+    HQ_LAUNCH_CHECK();
+  };
+  if (f.mode == 0) go(k_qf_digits<0>);
+  else if (f.mode == 1) go(k_qf_digits<1>);
+  else go(k_qf_digits<2>);
 }
 
-static void product(const Quad64 &q, const char *A, const char *B, const double *sA, const double *sB, long long N,
+static void product(const Quad64 &q, const char *A, const char *B, const int *eA, const int *eB, long long N, bool grid,
                     bool sym, bool tr, double scale, bool accumulate, double *M, cudaStream_t st) {
   QfArgs a{};
   a.A = A;
   a.B = B;
+  a.eA = eA;
+  a.eB = eB;
+  a.first = grid ? q.first : nullptr;
   a.part = q.part;
   a.err = q.err;
-  a.stages = ceil_div(N, kQfK);
+  a.blocks = blocks_of(q, N, grid);
+  a.stages = grid ? q.stages : ceil_div(N, kQfK);
   a.n = q.n;
-  a.rb = quad64_rows(q.n);
-  a.rbn = quad64_row_blocks(q.n);
+  a.rows = quad64_rows(q.n);
   a.tiles = quad64_tiles(q.n, sym, a.tile);
   a.groups = quad64_groups(q.n, sym);
   ensure_dyn_smem((const void *)k_qf_gemm, kQfSmem);
   k_qf_gemm<<<dim3(a.tiles, a.groups), kQfThreads, kQfSmem, st>>>(a);
   HQ_LAUNCH_CHECK();
-  k_qf_reduce<<<dim3(ceil_div(q.n, 32), q.n), 256, 0, st>>>(a, sym, tr, scale, sA, sB, accumulate, M);
+  k_qf_reduce<<<dim3(ceil_div(q.n, 32), q.n), 256, 0, st>>>(a, sym, tr, scale, accumulate, M);
   HQ_LAUNCH_CHECK();
 }
 
-void quad64_basis(const Quad64 &q, const double *phi, const double *dphi, long long N, cudaStream_t st) {
+void quad64_basis(const Quad64 &q, const double *phi, long long N, cudaStream_t st) {
   HQ_STAGE(ST_SPLIT, st);
-  const int nb = (int)quad64_table(N), rb = quad64_rows(q.n), rbn = quad64_row_blocks(q.n);
-  maxima(phi, q.n, N, q.tab, st);
-  if (dphi) maxima(dphi, 3 * q.n, N, q.tab + (size_t)q.n * nb, st);
-  k_qf_exponents<<<q.n, 128, 0, st>>>(q.tab, nullptr, q.n, nb, nullptr, nullptr, 0.f, q.eB, q.sB);
-  HQ_LAUNCH_CHECK();
-  k_qf_digits<0><<<ceil_div(N, kQfK), 256, 0, st>>>(phi, nullptr, nullptr, nullptr, 0.0, q.n, N, rb, rbn, q.eB, q.B);
-  HQ_LAUNCH_CHECK();
+  form(q, QfForm{0, phi}, N, true, q.eB, q.B, st);
 }
 
 void quad64_weighted(const Quad64 &q, const double *phi, const double *w, long long N, double scale, double *M,
                      cudaStream_t st) {
   HQ_STAGE(ST_QUAD, st);
   if (!w) {
-    product(q, q.B, q.B, q.sB, q.sB, N, true, false, scale, false, M, st);
+    product(q, q.B, q.B, q.eB, q.eB, N, true, true, false, scale, false, M, st);
     return;
   }
-  const int nb = (int)quad64_table(N), rb = quad64_rows(q.n), rbn = quad64_row_blocks(q.n);
-  maxima(w, 1, N, q.wtab, st);
-  k_qf_exponents<<<q.n, 128, 0, st>>>(q.tab, nullptr, q.n, nb, q.wtab, nullptr, 0.f, q.eA, q.sA);
-  HQ_LAUNCH_CHECK();
-  k_qf_digits<1><<<ceil_div(N, kQfK), 256, 0, st>>>(phi, nullptr, w, nullptr, 0.0, q.n, N, rb, rbn, q.eA, q.A);
-  HQ_LAUNCH_CHECK();
-  product(q, q.A, q.B, q.sA, q.sB, N, true, false, scale, false, M, st);
+  form(q, QfForm{1, phi, nullptr, w}, N, true, q.eA, q.A, st);
+  product(q, q.A, q.B, q.eA, q.eB, N, true, true, false, scale, false, M, st);
 }
 
 void quad64_gga(const Quad64 &q, const double *phi, const double *dphi, const double *w, const double *u, double dV,
                 long long N, double *M, cudaStream_t st) {
   HQ_STAGE(ST_QUAD, st);
-  const int nb = (int)quad64_table(N), rb = quad64_rows(q.n), rbn = quad64_row_blocks(q.n);
-  maxima(w, 1, N, q.wtab, st);
-  maxima(u, 3, N, q.wtab + nb, st);
-  k_qf_exponents<<<q.n, 128, 0, st>>>(q.tab, q.tab + (size_t)q.n * nb, q.n, nb, q.wtab, q.wtab + nb,
-                                      std::nextafter((float)dV, INFINITY), q.eA, q.sA);
-  HQ_LAUNCH_CHECK();
-  k_qf_digits<2><<<ceil_div(N, kQfK), 256, 0, st>>>(phi, dphi, w, u, dV, q.n, N, rb, rbn, q.eA, q.A);
-  HQ_LAUNCH_CHECK();
-  product(q, q.A, q.B, q.sA, q.sB, N, false, true, 1.0, false, M, st);
+  form(q, QfForm{2, phi, dphi, w, u, dV}, N, true, q.eA, q.A, st);
+  product(q, q.A, q.B, q.eA, q.eB, N, true, false, true, 1.0, false, M, st);
 }
 
 void quad64_gram(const Quad64 &q, const double *Q, long long N, bool accumulate, double *M, cudaStream_t st) {
   HQ_STAGE(ST_QUAD, st);
-  const int nb = (int)quad64_table(N), rb = quad64_rows(q.n), rbn = quad64_row_blocks(q.n);
-  maxima(Q, q.n, N, q.xtab, st);
-  k_qf_exponents<<<q.n, 128, 0, st>>>(q.xtab, nullptr, q.n, nb, nullptr, nullptr, 0.f, q.eA, q.sA);
-  HQ_LAUNCH_CHECK();
-  k_qf_digits<0><<<ceil_div(N, kQfK), 256, 0, st>>>(Q, nullptr, nullptr, nullptr, 0.0, q.n, N, rb, rbn, q.eA, q.A);
-  HQ_LAUNCH_CHECK();
-  product(q, q.A, q.A, q.sA, q.sA, N, true, false, 1.0, accumulate, M, st);
+  form(q, QfForm{0, Q}, N, false, q.eA, q.A, st);
+  product(q, q.A, q.A, q.eA, q.eA, N, false, true, false, 1.0, accumulate, M, st);
 }
 
 void quad64_pair(const Quad64 &q, const double *phi, const double *w, const double *Y, long long N, double scale,
                  bool accumulate, double *M, cudaStream_t st) {
   HQ_STAGE(ST_QUAD, st);
-  const int nb = (int)quad64_table(N), rb = quad64_rows(q.n), rbn = quad64_row_blocks(q.n);
-  maxima(w, 1, N, q.wtab, st);
-  k_qf_exponents<<<q.n, 128, 0, st>>>(q.tab, nullptr, q.n, nb, q.wtab, nullptr, 0.f, q.eA, q.sA);
-  HQ_LAUNCH_CHECK();
-  k_qf_digits<1><<<ceil_div(N, kQfK), 256, 0, st>>>(phi, nullptr, w, nullptr, 0.0, q.n, N, rb, rbn, q.eA, q.A);
-  HQ_LAUNCH_CHECK();
-  maxima(Y, q.n, N, q.xtab, st);
-  k_qf_exponents<<<q.n, 128, 0, st>>>(q.xtab, nullptr, q.n, nb, nullptr, nullptr, 0.f, q.eX, q.sX);
-  HQ_LAUNCH_CHECK();
-  k_qf_digits<0><<<ceil_div(N, kQfK), 256, 0, st>>>(Y, nullptr, nullptr, nullptr, 0.0, q.n, N, rb, rbn, q.eX, q.X);
-  HQ_LAUNCH_CHECK();
-  product(q, q.A, q.X, q.sA, q.sX, N, false, false, scale, accumulate, M, st);
+  form(q, QfForm{1, phi, nullptr, w}, N, true, q.eA, q.A, st);
+  form(q, QfForm{0, Y}, N, true, q.eX, q.X, st);
+  product(q, q.A, q.X, q.eA, q.eX, N, true, false, false, scale, accumulate, M, st);
 }
 
 }  // namespace hqcgb

@@ -63,6 +63,13 @@ __device__ inline uint64_t sdesc(uint32_t saddr) {
   return d;
 }
 
+// One lane of a whole warp, the same at every call.
+__device__ __forceinline__ bool elect() {
+  uint32_t r;
+  asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(r));
+  return r != 0;
+}
+
 __device__ inline void mma_commit(uint64_t *bar) {
   asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];"
                ::"r"(smem_u32(bar)) : "memory");
