@@ -12,6 +12,8 @@
 // Layout: phi^T (and the gradient's three fields) by tiles of 128 points,
 // [field][tile][block of 32 AOs][pair][128 rows][128 bytes], a stage's 64 KB in
 // one piece; Y^T by 64 orbitals, [column block][block of 32 AOs][pair][64][128].
+// Digits of all tiles are kept for a geometry where the plan affords it, otherwise
+// formed for a range of tiles at a time (the same bits: points are independent).
 // Persistent CTAs, one an SM, take tiles in turn: a copy thread, an MMA thread,
 // eight drain warps.  Bound by the drains: conversion of the TMEM sums and the
 // FP64 squares.  Measured, against the sum over D on the FP64 pipe: 64 AOs, up to 64
@@ -38,17 +40,16 @@ constexpr int kDfMaxAo = 512;  // one TMEM sum holds 512 terms exactly
 
 int density64_max_ao() { return kDfMaxAo; }
 static int df_blocks(int nao) { return ceil_div(nao, kDfK); }
-size_t density64_field_bytes(int nao, long long N) {
-  return (size_t)ceil_div(N, kDfM) * df_blocks(nao) * kDfStage / (kDfPairA + kDfPairB) * kDfPairA;
-}
+int density64_tiles(long long N) { return ceil_div(N, kDfM); }
+int density64_min_tiles(long long N) { return std::min(152, density64_tiles(N)); }
+size_t density64_tile_bytes(int nao, int fields) { return (size_t)fields * df_blocks(nao) * kQfPairs * kDfPairA; }
 size_t density64_orbital_bytes(int nao) {
   return (size_t)ceil_div(nao, kDfN) * df_blocks(nao) * kQfPairs * kDfPairB;
 }
 
-// Exponent and scale of every grid point: the largest |phi_p(g)|.
+// Scale of every grid point, the power of two 2^e above the largest |phi_p(g)|.
 __global__ void __launch_bounds__(256)
-    k_df_points(const double *__restrict__ phi, int nao, long long N, int *__restrict__ e,
-                double *__restrict__ scale) {
+    k_df_points(const double *__restrict__ phi, int nao, long long N, double *__restrict__ scale) {
   const long long g = (long long)blockIdx.x * 256 + threadIdx.x;
   if (g >= N) return;
   unsigned v = 0;
@@ -56,24 +57,26 @@ __global__ void __launch_bounds__(256)
   const float m = __uint_as_float(v);
   int k = 0;
   if (m > 0.f && m < INFINITY) frexpf(m, &k);
-  e[g] = k + 1;
   scale[g] = m < INFINITY ? scalbn(1.0, k + 1) : NAN;
 }
 
-// Digits of phi^T: a block takes a tile of 128 points, a warp 32 of them and
-// every other chunk of 8 AOs (reads along the points).  Zeros beyond N and nao.
+// Digits of phi^T (blockIdx.y > 0: of a gradient's field): a block takes a tile of
+// 128 points, a warp 32 of them and every other chunk of 8 AOs (reads along the
+// points).  Zeros beyond N and nao.
 __global__ void __launch_bounds__(256)
-    k_df_digits(const double *__restrict__ phi, int nao, long long N, int nkb, const int *__restrict__ e,
-                char *__restrict__ out) {
-  const int warp = threadIdx.x >> 5, r = (warp & 3) * 32 + (threadIdx.x & 31);
-  const long long g = (long long)blockIdx.x * kDfM + r;
-  const int eg = g < N ? e[g] : 0;
+    k_df_digits(const double *__restrict__ phi, const double *__restrict__ dphi, int nao, long long N, int nkb, int tile0,
+                const double *__restrict__ scale, char *__restrict__ out) {
+  const int warp = threadIdx.x >> 5, r = (warp & 3) * 32 + (threadIdx.x & 31), f = blockIdx.y;
+  const double *X = f == 0 ? phi : dphi + (long long)(f - 1) * nao * N;
+  const long long g = (long long)(tile0 + blockIdx.x) * kDfM + r;
+  const int eg = g < N ? ((__double2hiint(scale[f * N + g]) >> 20) & 0x7ff) - 1023 : 0;
+  out += (long long)f * gridDim.x * nkb * kQfPairs * kDfPairA;
   for (int ch = warp >> 2; ch < nkb * 4; ch += 2) {
     QfPack pack;
 #pragma unroll
     for (int i = 0; i < 8; ++i) {
       const int p = ch * 8 + i;
-      pack.put(i, g < N && p < nao ? phi[(long long)p * N + g] : 0.0, eg);
+      pack.put(i, g < N && p < nao ? X[(long long)p * N + g] : 0.0, eg);
     }
     char *row = out + (((long long)blockIdx.x * nkb + (ch >> 2)) * kQfPairs * kDfM + r) * 128;
     pack.store(row, kDfPairA, ch & 3, r);
@@ -125,7 +128,8 @@ struct DfArgs {
   int *err;
   long long N;
   size_t field;  // bytes of a field's digits
-  int nkb, nuse, tiles, cols, bufs;  // cols: TMEM columns of one P_d
+  int tile0, tiles;  // the tiles of A
+  int nkb, nuse, cols, bufs;  // cols: TMEM columns of one P_d
 };
 
 struct DfPipe {
@@ -226,7 +230,7 @@ __global__ void __launch_bounds__(kDfThreads, 1) k_df_density(const DfArgs a) {
     const uint32_t base = P.tmem_base + ((uint32_t)((warp & 3) * 32) << 16) + half * hc;
     int chain = 0;
     for (int tile = blockIdx.x; tile < a.tiles; tile += gridDim.x) {
-      const long long g = (long long)tile * kDfM + row;
+      const long long g = (long long)(a.tile0 + tile) * kDfM + row;
       double acc[FIELDS];
 #pragma unroll
       for (int f = 0; f < FIELDS; ++f) acc[f] = 0.0;
@@ -303,22 +307,26 @@ __global__ void __launch_bounds__(kDfThreads, 1) k_df_density(const DfArgs a) {
   }
 }
 
-void density64_basis(const Density64 &d, const double *phi, const double *dphi, long long N, cudaStream_t st) {
-  HQ_STAGE(ST_SPLIT, st);
-  const int nkb = df_blocks(d.n);
-  for (int f = 0; f < (dphi ? 4 : 1); ++f) {
-    const double *X = f == 0 ? phi : dphi + (long long)(f - 1) * d.n * N;
-    k_df_points<<<ceil_div(N, 256), 256, 0, st>>>(X, d.n, N, d.e, d.sA + f * N);
-    HQ_LAUNCH_CHECK();
-    k_df_digits<<<ceil_div(N, kDfM), 256, 0, st>>>(X, d.n, N, nkb, d.e, d.A + f * density64_field_bytes(d.n, N));
-    HQ_LAUNCH_CHECK();
-  }
+static void form(const Density64 &d, const double *phi, const double *dphi, long long N, int tile0, int tiles,
+                 cudaStream_t st) {
+  k_df_digits<<<dim3(tiles, dphi ? 4 : 1), 256, 0, st>>>(phi, dphi, d.n, N, df_blocks(d.n), tile0, d.sA, d.A);
+  HQ_LAUNCH_CHECK();
 }
 
-void density64(const Density64 &d, const double *C, const double *occ, int nuse, bool gga, long long N, double *rho,
-               double *grho, double *psi, cudaStream_t st) {
+void density64_basis(const Density64 &d, const double *phi, const double *dphi, long long N, cudaStream_t st) {
+  HQ_STAGE(ST_SPLIT, st);
+  for (int f = 0; f < (dphi ? 4 : 1); ++f) {
+    k_df_points<<<ceil_div(N, 256), 256, 0, st>>>(f == 0 ? phi : dphi + (long long)(f - 1) * d.n * N, d.n, N,
+                                                  d.sA + f * N);
+    HQ_LAUNCH_CHECK();
+  }
+  if (d.keep) form(d, phi, dphi, N, 0, density64_tiles(N), st);
+}
+
+void density64(const Density64 &d, const double *phi, const double *dphi, const double *C, const double *occ, int nuse,
+               long long N, double *rho, double *grho, double *psi, cudaStream_t st) {
   HQ_STAGE(ST_DENSITY, st);
-  const int nkb = df_blocks(d.n);
+  const int nkb = df_blocks(d.n), tiles = density64_tiles(N), ranges = ceil_div(tiles, d.cap);
   k_df_orbitals<<<nuse, 128, 0, st>>>(C, occ, d.n, nkb, d.eY, d.B);
   HQ_LAUNCH_CHECK();
   DfArgs a{};
@@ -331,20 +339,24 @@ void density64(const Density64 &d, const double *C, const double *occ, int nuse,
   a.psi = psi;
   a.err = d.err;
   a.N = N;
-  a.field = density64_field_bytes(d.n, N);
   a.nkb = nkb;
   a.nuse = nuse;
-  a.tiles = ceil_div(N, kDfM);
   a.cols = (std::min(nuse, kDfN) + 15) / 16 * 16;
   a.bufs = kQfDigits * a.cols * 2 <= 512 ? 2 : 1;
-  const int grid = std::min(152, a.tiles);
-  auto go = [&](auto kernel) {
-    ensure_dyn_smem((const void *)kernel, kDfSmem);
-    kernel<<<grid, kDfThreads, kDfSmem, st>>>(a);
-    HQ_LAUNCH_CHECK();
-  };
-  if (gga) go(k_df_density<4>);
-  else go(k_df_density<1>);
+  for (int k = 0; k < ranges; ++k) {
+    a.tile0 = (int)((long long)tiles * k / ranges);
+    a.tiles = (int)((long long)tiles * (k + 1) / ranges) - a.tile0;
+    a.field = density64_tile_bytes(d.n, 1) * a.tiles;
+    if (!d.keep) form(d, phi, dphi, N, a.tile0, a.tiles, st);
+    const int grid = std::min(152, a.tiles);
+    auto go = [&](auto kernel) {
+      ensure_dyn_smem((const void *)kernel, kDfSmem);
+      kernel<<<grid, kDfThreads, kDfSmem, st>>>(a);
+      HQ_LAUNCH_CHECK();
+    };
+    if (dphi) go(k_df_density<4>);
+    else go(k_df_density<1>);
+  }
 }
 
 }  // namespace hqcgb

@@ -21,24 +21,28 @@ void launch_sum_partials(const double *part, int nblk, int stride, int nout, dou
                          double *out, bool accumulate, cudaStream_t st);
 
 // quad_f64.cu: FP64 quadratures on the tensor cores (digits of 7 bits).
-// Workspace of one plan: digits and exponents of the weighted operand (A), of the
-// AOs (B) and, for a second operand of quad64_pair, X; the bricks of its grid;
-// FP64 partial tiles; the tensor-core error word.
+// Workspace of one plan: digits and exponents of a segment of either operand (A, X)
+// and, where the plan keeps them for a geometry, of the AOs (B, else null: they are
+// formed in X for every product); the bricks of its grid; FP64 partial tiles; the
+// tensor-core error word.
 struct Quad64 {
   int n = 0, ng = 0, stages = 0;
   char *A = nullptr, *B = nullptr, *X = nullptr;
   int *eA = nullptr, *eB = nullptr, *eX = nullptr, *err = nullptr;
+  size_t exponents = 0;  // that eA and eX hold; A and X hold the same segment
   int *first = nullptr;  // quad64_first on the device; stages = its last
   double *part = nullptr;
 };
 std::vector<int> quad64_first(int ng);
-// bytes and exponents of an operand: a field of the grid, or rows of K values
-size_t quad64_grid_bytes(int n, int ng);
-size_t quad64_linear_bytes(int n, long long K);
-size_t quad64_grid_exponents(int n, int ng);
-size_t quad64_linear_exponents(int n, long long K);
+// digits (bytes) and exponents of a whole operand and of its largest segment: a
+// field of the grid, or rows of K values
+struct Quad64Sizes {
+  size_t bytes, exponents, seg_bytes, seg_exponents;
+};
+Quad64Sizes quad64_grid_sizes(int n, int ng);
+Quad64Sizes quad64_linear_sizes(int n, long long K);
 size_t quad64_partial_doubles(int n);
-// AOs of a geometry: exponents and digits (B)
+// AOs of a geometry: exponents and digits (B), where kept
 void quad64_basis(const Quad64 &q, const double *phi, long long N, cudaStream_t st);
 // M = scale sum_g phi_p w phi_q (w NULL: 1), both after quad64_basis
 void quad64_weighted(const Quad64 &q, const double *phi, const double *w, long long N, double scale, double *M,
@@ -53,22 +57,27 @@ void quad64_pair(const Quad64 &q, const double *phi, const double *w, const doub
                  bool accumulate, double *M, cudaStream_t st);
 
 // density_f64.cu: FP64 density from the orbitals on the tensor cores, up to
-// density64_max_ao() AOs.  A: digits of phi^T (and of the gradient's fields),
-// sA [fields][N], e [N] scratch; B, eY: digits and exponents of Y^T.
+// density64_max_ao() AOs.  A: digits of phi^T (and of the gradient's fields) for
+// `cap` tiles of points: all of them where the plan keeps them for a geometry (keep),
+// otherwise formed range by range of tiles for every density; sA [fields][N];
+// B, eY: digits and exponents of Y^T.
 struct Density64 {
-  int n = 0;
+  int n = 0, cap = 0;
+  bool keep = false;
   char *A = nullptr, *B = nullptr;
   double *sA = nullptr;
-  int *e = nullptr, *eY = nullptr, *err = nullptr;
+  int *eY = nullptr, *err = nullptr;
 };
 int density64_max_ao();
-size_t density64_field_bytes(int nao, long long N);
+int density64_tiles(long long N);
+int density64_min_tiles(long long N);  // fewer in a range would leave SMs idle
+size_t density64_tile_bytes(int nao, int fields);
 size_t density64_orbital_bytes(int nao);
 void density64_basis(const Density64 &d, const double *phi, const double *dphi, long long N, cudaStream_t st);
-// rho (and grad rho) of the first nuse orbitals (nuse >= 1); psi not null:
-// sqrt(f_k) psi_k into psi [nuse][N]
-void density64(const Density64 &d, const double *C, const double *occ, int nuse, bool gga, long long N, double *rho,
-               double *grho, double *psi, cudaStream_t st);
+// rho (and grad rho, dphi not null) of the first nuse orbitals (nuse >= 1) after
+// density64_basis with the same AOs; psi not null: sqrt(f_k) psi_k into psi [nuse][N]
+void density64(const Density64 &d, const double *phi, const double *dphi, const double *C, const double *occ, int nuse,
+               long long N, double *rho, double *grho, double *psi, cudaStream_t st);
 
 // fft_fp64.cu
 void launch_fft3d(double2 *c, int ng, int batch, const double2 *tw, bool inverse, cudaStream_t st);

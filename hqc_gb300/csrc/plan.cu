@@ -217,6 +217,7 @@ struct hqcgb_plan {
   double *stpart = nullptr;    // chunks of S~ (mixed Hartree-Fock)
   Density64 d64{};             // FP64 density from the orbitals
   int nuse_64 = 0;             // orbitals it runs over
+  long long kept_digits = 0;   // bytes of digits kept for a geometry
   MixedEigWork mew{};
   bool eig_wide = false;       // FP64 path: this geometry's Fock matrices need the FP32 QL sweep
   // exact exchange in the occupied-pair form (exchange.cu); R = double on
@@ -288,7 +289,17 @@ static double occ_shift(const hqcgb_plan *p) {
   return -P.smearing_sigma * x;
 }
 
-static void create(const hqcgb_params *in, hqcgb_plan *p) {
+// Digits of the AOs (quad_f64.cu, density_f64.cu: 16 bytes a value and operand) that
+// plans keep for a geometry instead of forming them for every density and
+// quadrature.  A bound for a plan and its batch workers together, because kept digits
+// would take twice what the AOs themselves do (H54 dzvp PBE 81^3 with forces: 8 GB
+// without, 24 with), and batches or grids that fit the device would not any more.
+// What does not fit is formed piece by piece in a scratch a few per cent of the plan's
+// size.  Kept / formed every time: H32 dzv LDA 65^3 (570 MB) 34 / 41 ms a run, H14
+// dzvp PBE 49^3 with forces (860 MB) 38 / 50.
+static constexpr long long kKeptDigits = 1LL << 30;
+
+static void create(const hqcgb_params *in, hqcgb_plan *p, long long digit_budget) {
   const hqcgb_params &P = *in;
   HQ_REQUIRE(P.n_atoms >= 1, "n_atoms must be >= 1");
   HQ_REQUIRE(P.n_grid >= 3 && P.n_grid <= kMaxGrid, "n_grid out of range");
@@ -488,40 +499,54 @@ static void create(const hqcgb_params *in, hqcgb_plan *p) {
   if (!p->mixed || (p->hf && !p->exx_fused)) {
     // FP64 quadratures: Fock, V, S~ and the Gram matrix of the FP64 exchange
     const long long gK = p->exx_fused && !p->mixed ? (long long)p->exx_g * exx_pair_len(p->ng) : 0;
+    const Quad64Sizes field = quad64_grid_sizes(nao, p->ng), gram = quad64_linear_sizes(nao, gK);
     const bool legacy = p->hf && !p->exx_fused;
-    const size_t field = quad64_grid_bytes(nao, p->ng), fexp = quad64_grid_exponents(nao, p->ng);
     Quad64 &q = p->q64;
+    Density64 &d = p->d64;
     q.n = nao;
     q.ng = p->ng;
     const std::vector<int> first = quad64_first(p->ng);
     q.stages = first.back();
     q.first = p->alloc<int>(first.size());
     upload(q.first, first.data(), first.size() * sizeof(int));
-    q.B = p->alloc<char>(field);
-    q.eB = p->alloc<int>(fexp);
-    q.A = p->alloc<char>(std::max(field, quad64_linear_bytes(nao, gK)));
-    q.eA = p->alloc<int>(std::max(fexp, quad64_linear_exponents(nao, gK)));
-    if (legacy) {
-      q.X = p->alloc<char>(field);
-      q.eX = p->alloc<int>(fexp);
+    const size_t seg = std::max(field.seg_bytes, gram.seg_bytes);
+    const int fields = p->gga ? 4 : 1, tiles = density64_tiles(N);
+    if (!p->mixed && nao <= density64_max_ao()) d.n = nao;
+    const size_t tile = d.n ? density64_tile_bytes(nao, fields) : 0;
+    const size_t all = field.bytes + tile * tiles;
+    const bool keep = !p->mixed && (long long)all <= digit_budget;
+    const bool second = !keep || legacy;
+    if (keep) {
+      p->kept_digits = (long long)all;
+      q.B = p->alloc<char>(field.bytes);
+      q.eB = p->alloc<int>(field.exponents);
+      q.A = p->alloc<char>(seg * (second ? 2 : 1));
+      d.cap = tiles;
+      d.keep = true;
+      if (d.n) d.A = p->alloc<char>(tile * tiles);
+    } else {
+      // one scratch: a density and a quadrature follow one another on the plan's stream
+      const size_t want = std::max(2 * seg, tile * density64_min_tiles(N));
+      q.A = p->alloc<char>(want);
+      d.A = q.A;
+      if (tile) d.cap = (int)std::min<size_t>(tiles, want / tile);
     }
+    if (second) q.X = q.A + seg;
+    q.exponents = std::max(field.seg_exponents, gram.seg_exponents);
+    q.eA = p->alloc<int>(q.exponents);
+    if (second) q.eX = p->alloc<int>(q.exponents);
     q.part = p->alloc<double>(quad64_partial_doubles(nao));
     if (!p->tc_err) {
       p->tc_err = p->alloc<int>(1);
       HQ_CUDA(cudaMemset(p->tc_err, 0, sizeof(int)));
     }
     q.err = p->tc_err;
-  }
-  if (!p->mixed && nao <= density64_max_ao()) {
-    const int fields = p->gga ? 4 : 1;
-    Density64 &d = p->d64;
-    d.n = nao;
-    d.A = p->alloc<char>(fields * density64_field_bytes(nao, N));
-    d.B = p->alloc<char>(density64_orbital_bytes(nao));
-    d.sA = p->alloc<double>(fields * N);
-    d.e = p->alloc<int>(N);
-    d.eY = p->alloc<int>(nao);
-    d.err = p->tc_err;
+    if (d.n) {
+      d.B = p->alloc<char>(density64_orbital_bytes(nao));
+      d.sA = p->alloc<double>(fields * N);
+      d.eY = p->alloc<int>(nao);
+      d.err = p->tc_err;
+    }
   }
   p->xpart = p->alloc<double>((size_t)2 * xc_blocks(N));
   if (P.want_forces) {
@@ -857,7 +882,8 @@ static double fock(Ctx &c) {
   } else {
   if (p->d64.n) {
     double *psi = p->exx_fused ? static_cast<double *>(p->exx_psi) : nullptr;  // the exchange takes them
-    density64(p->d64, p->C, p->occ, p->nuse_64, p->gga, N, p->rho, p->gga ? p->grho : nullptr, psi, c.st);
+    density64(p->d64, p->phi, p->gga ? p->dphi : nullptr, p->C, p->occ, p->nuse_64, N, p->rho,
+              p->gga ? p->grho : nullptr, psi, c.st);
     p->exx_psi_ready = psi != nullptr;
   } else {
     launch_density(p->phi, p->gga ? p->dphi : nullptr, p->D, n, N, p->rho, p->gga ? p->grho : nullptr,
@@ -1203,18 +1229,21 @@ static hqcgb_params params_of(const hqcgb_plan *p) {
 }
 
 static void ensure_workers(hqcgb_plan *p, int k) {
+  long long left = kKeptDigits - p->kept_digits;
+  for (const hqcgb_plan *w : p->workers) left -= w->kept_digits;
   while ((int)p->workers.size() < k) {
     hqcgb_params q = params_of(p);
     cudaStream_t s;
     HQ_CUDA(cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking));
     hqcgb_plan *w = new hqcgb_plan();
     try {
-      create(&q, w);
+      create(&q, w, left);
     } catch (...) {  // nothing of a failed clone outlives this call
       delete w;
       cudaStreamDestroy(s);
       throw;
     }
+    left -= w->kept_digits;
     p->workers.push_back(w);
     p->wstreams.push_back(s);
   }
@@ -1392,9 +1421,11 @@ static hqcgb_plan *batch_plan(hqcgb_batch *b, int t, int n_atoms, int n_grid, do
   q.lat1d = l1.data();
   q.n_lattice = (int)lat.size() / 3;
   q.lattice = lat.data();
+  long long left = kKeptDigits / b->workers;  // each worker's share: their threads create plans at the same time
+  for (const auto &kv : b->plans[t]) left -= kv.second->kept_digits;
   hqcgb_plan *p = new hqcgb_plan();
   try {
-    create(&q, p);
+    create(&q, p, left);
   } catch (...) {
     delete p;
     throw;
@@ -1496,7 +1527,7 @@ int hqcgb_plan_create(const hqcgb_params *params, hqcgb_plan **plan) {
     HQ_REQUIRE(params && plan, "null argument");
     hqcgb_plan *p = new hqcgb_plan();
     try {
-      create(params, p);
+      create(params, p, kKeptDigits);
     } catch (...) {
       delete p;
       throw;

@@ -63,6 +63,7 @@ constexpr size_t kQfSmem = kQfRing * kQfStage + 1024;   // + alignment to the sw
 constexpr int kQfDrainWarps = 8;
 constexpr int kQfThreads = (kQfDrainWarps + 2) * 32;
 constexpr int kQfMaxTiles = (kMaxNao / kQfM) * (kMaxNao / kQfN);
+constexpr long long kQfSegment = 160LL << 20;           // bytes of an operand's digits formed at a time
 constexpr int kQfBad = 1 << 20;                         // exponent of a block with a value that is not finite
 static_assert(kQfSmem <= 227 * 1024, "FP64 quadrature ring above 227 KB");
 static_assert(kQfSide * kQfSide * kQfSide <= kQfBlk, "a brick is one block");
@@ -83,13 +84,41 @@ std::vector<int> quad64_first(int ng) {
       for (int z = 0; z < m; ++z) first.push_back(first.back() + ceil_div(len(x) * len(y) * len(z), kQfK));
   return first;
 }
-size_t quad64_grid_bytes(int n, int ng) { return (size_t)quad64_first(ng).back() * stage_bytes(n); }
-size_t quad64_linear_bytes(int n, long long K) { return (size_t)ceil_div(K, kQfK) * stage_bytes(n); }
-size_t quad64_grid_exponents(int n, int ng) {
-  const size_t m = quad64_parts(ng);
-  return m * m * m * quad64_rows(n);
+// Operands are formed and multiplied in segments of whole blocks, so that a plan's
+// memory does not grow with its digits: a grid in equal segments of kQfSegment to
+// twice that, rows of any length in segments of kQfSegment and a rest (a buffer for
+// the longest then holds the shorter ones').  A segment more costs two launches and
+// their tails (quadratures of an H32 dzv run at 65^3, 23 of them: one segment 6.3 ms,
+// three 7.9, nine 13.4 with the AOs' digits formed too).
+struct Segments {
+  int blocks, count, size;  // size 0: equal ones
+  int begin(int k) const { return size ? std::min(blocks, k * size) : (int)((long long)blocks * k / count); }
+};
+static Segments grid_segments(int n, int ng, int stages) {
+  const int m = quad64_parts(ng);
+  return {m * m * m, (int)std::max(1LL, (long long)stages * (long long)stage_bytes(n) / kQfSegment), 0};
 }
-size_t quad64_linear_exponents(int n, long long K) { return (size_t)quad64_linear_blocks(K) * quad64_rows(n); }
+static Segments linear_segments(int n, long long K) {
+  const int blocks = (int)quad64_linear_blocks(K);
+  const int size = (int)std::max<long long>(1, kQfSegment / (long long)(stage_bytes(n) * (kQfBlk / kQfK)));
+  return {blocks, std::max(1, ceil_div(blocks, size)), size};
+}
+Quad64Sizes quad64_grid_sizes(int n, int ng) {
+  const std::vector<int> first = quad64_first(ng);
+  const Segments sg = grid_segments(n, ng, first.back());
+  int stages = 0, most = 0;
+  for (int k = 0; k < sg.count; ++k) {
+    stages = std::max(stages, first[sg.begin(k + 1)] - first[sg.begin(k)]);
+    most = std::max(most, sg.begin(k + 1) - sg.begin(k));
+  }
+  const size_t rows = quad64_rows(n);
+  return {first.back() * stage_bytes(n), sg.blocks * rows, stages * stage_bytes(n), most * rows};
+}
+Quad64Sizes quad64_linear_sizes(int n, long long K) {
+  const Segments sg = linear_segments(n, K);
+  const size_t rows = quad64_rows(n), stage = stage_bytes(n) * (kQfBlk / kQfK), most = std::min(sg.blocks, sg.size);
+  return {sg.blocks * stage, sg.blocks * rows, most * stage, most * rows};
+}
 
 static int quad64_tiles(int n, bool sym, unsigned char (*t)[2] = nullptr) {
   int cnt = 0;
@@ -120,6 +149,7 @@ struct QfSource {
   int n, rows, ng, parts;
   long long N;
   const int *first;
+  int b0;      // the block that the output starts with
   int *e;      // [block][rows]
   char *out;
 };
@@ -142,7 +172,7 @@ __global__ void __launch_bounds__(kQfFormRows * 32) k_qf_digits(const QfSource a
   double *s_w = s_x + kQfFormRows * kQfRowLd, *s_u = s_w + kQfBlk;
   int *s_off = reinterpret_cast<int *>(s_w + (MODE == 0 ? 0 : MODE == 1 ? 1 : 4) * kQfBlk);  // the block's points
   __shared__ int s_e[kQfFormRows];
-  const int b = blockIdx.x, tid = threadIdx.x;
+  const int b = a.b0 + blockIdx.x, tid = threadIdx.x;
   int cnt, stage0;
   long long base = 0;
   int x0 = 0, y0 = 0, z0 = 0, sy = 1, sz = 1;
@@ -155,11 +185,11 @@ __global__ void __launch_bounds__(kQfFormRows * 32) k_qf_digits(const QfSource a
     sy = cut(by + 1) - y0;
     sz = cut(bz + 1) - z0;
     cnt = (cut(bx + 1) - x0) * sy * sz;
-    stage0 = a.first[b];
+    stage0 = a.first[b] - a.first[a.b0];
   } else {
     base = (long long)b * kQfBlk;
     cnt = (int)min((long long)kQfBlk, a.N - base);
-    stage0 = b * (kQfBlk / kQfK);
+    stage0 = blockIdx.x * (kQfBlk / kQfK);
   }
   const int stages = (cnt + kQfK - 1) / kQfK, pts = stages * kQfK;
   for (int k = tid; k < pts; k += kQfFormRows * 32) {
@@ -199,7 +229,7 @@ __global__ void __launch_bounds__(kQfFormRows * 32) k_qf_digits(const QfSource a
       const int e = ex == 0x7ff ? kQfBad : ex - 1021;
       if (lane == 0) {
         s_e[warp] = e;
-        a.e[(long long)b * a.rows + p] = e;
+        a.e[(long long)blockIdx.x * a.rows + p] = e;
       }
     }
     __syncthreads();
@@ -222,26 +252,32 @@ __global__ void __launch_bounds__(kQfFormRows * 32) k_qf_digits(const QfSource a
 struct QfArgs {
   const char *A, *B;
   const int *eA, *eB;  // [block][rows]
-  const int *first;    // first stage of every block, or null: 16 stages a block
+  const int *first;    // first stage of every block, or null: 16 stages a block, `stages` in all
   double *part;        // [group][tile][128][64]
   int *err;
-  int stages, blocks, n, rows, groups, tiles;
+  int stages, b0, b1;  // the segment's blocks
+  int wholeA, wholeB;  // the operand holds all blocks, not the segment's alone
+  int add;             // to the sums of the segments before
+  int n, rows, groups, tiles;
   unsigned char tile[kQfMaxTiles][2];  // 128-row block of A, 64-row block of B
 };
 
-// The chains of group g's share of the stages, in order: stages [s, e) of block b.
+// The chains of group g's share of the segment's stages, in order: stages [s, e) of
+// block b, s and e counted from the segment's first stage.
 struct QfChains {
   const QfArgs &a;
-  int s, e, end, b;
+  int s, e, end, b, base;
   __device__ __forceinline__ int first(int k) const { return a.first ? a.first[k] : min(k * (kQfBlk / kQfK), a.stages); }
   __device__ __forceinline__ QfChains(const QfArgs &a_, int g) : a(a_) {
-    s = e = (int)((long long)a.stages * g / a.groups);
-    end = (int)((long long)a.stages * (g + 1) / a.groups);
-    b = s / (kQfBlk / kQfK);  // a block is at most 16 stages
+    base = first(a.b0);
+    const long long stages = first(a.b1) - base;
+    s = e = (int)(stages * g / a.groups);
+    end = (int)(stages * (g + 1) / a.groups);
+    b = a.b0 + s / (kQfBlk / kQfK);  // a block is at most 16 stages
     if (a.first)
-      for (int hi = a.blocks; hi - b > 1;) {
+      for (int hi = a.b1; hi - b > 1;) {
         const int mid = (b + hi) / 2;
-        if (a.first[mid] <= s) b = mid;
+        if (a.first[mid] - base <= s) b = mid;
         else hi = mid;
       }
     --b;
@@ -250,7 +286,7 @@ struct QfChains {
     s = e;
     if (s >= end) return false;
     ++b;
-    e = min(end, first(b + 1));
+    e = min(end, first(b + 1) - base);
     return true;
   }
 };
@@ -291,7 +327,10 @@ __global__ void __launch_bounds__(kQfThreads, 1) k_qf_gemm(const __grid_constant
       const uint32_t nb = (uint32_t)min(kQfN, a.rows - ct * kQfN) * 128u;
       const long long pair = (long long)a.rows * 128;
       int it = 0;
-      for (QfChains c(a, g); ok && c.next();)
+      QfChains c(a, g);
+      const char *A0 = a.A + (a.wholeA ? c.base : 0) * kQfPairs * pair + (long long)mt * kQfM * 128;
+      const char *B0 = a.B + (a.wholeB ? c.base : 0) * kQfPairs * pair + (long long)ct * kQfN * 128;
+      while (ok && c.next())
         for (int s = c.s; s < c.e; ++s, ++it) {
           const int slot = it % kQfRing, use = it / kQfRing;
           if (use > 0 && !mbar_wait(&P.empty[slot], (unsigned)((use - 1) & 1), a.err, 61)) {
@@ -300,8 +339,7 @@ __global__ void __launch_bounds__(kQfThreads, 1) k_qf_gemm(const __grid_constant
           }
           mbar_expect_tx(&P.full[slot], kQfPairs * (na + nb));
           const uint32_t dst = smem_u32(sm + slot * kQfStage);
-          const char *srcA = a.A + s * kQfPairs * pair + (long long)mt * kQfM * 128;
-          const char *srcB = a.B + s * kQfPairs * pair + (long long)ct * kQfN * 128;
+          const char *srcA = A0 + s * kQfPairs * pair, *srcB = B0 + s * kQfPairs * pair;
           for (int q = 0; q < kQfPairs; ++q) {
             bulk_copy(dst + q * kQfPairA, srcA + q * pair, na, &P.full[slot]);
             bulk_copy(dst + kQfOffB + q * kQfPairB, srcB + q * pair, nb, &P.full[slot]);
@@ -353,12 +391,15 @@ __global__ void __launch_bounds__(kQfThreads, 1) k_qf_gemm(const __grid_constant
     const int c0 = (warp >> 2) * 32, row = (warp & 3) * 32 + lane;
     const uint32_t base = tmem + ((uint32_t)((warp & 3) * 32) << 16) + c0;
     const int ra = min(mt * kQfM + row, a.n - 1), rb = min(ct * kQfN + c0 + lane, a.n - 1);
+    const bool own = mt * kQfM + row < a.n;
+    double *out = a.part + (((long long)g * a.tiles + tile) * kQfM + row) * kQfN + c0;
     double acc[32];
 #pragma unroll
-    for (int i = 0; i < 32; ++i) acc[i] = 0.0;
+    for (int i = 0; i < 32; ++i) acc[i] = a.add && own && c0 + i < rows_b ? out[i] : 0.0;
     QfChains c(a, g);
     for (int j = 0; c.next(); ++j) {
-      const int ea = a.eA[(long long)c.b * a.rows + ra], eb = a.eB[(long long)c.b * a.rows + rb];
+      const int ea = a.eA[(long long)(c.b - (a.wholeA ? 0 : a.b0)) * a.rows + ra],
+                eb = a.eB[(long long)(c.b - (a.wholeB ? 0 : a.b0)) * a.rows + rb];
       if (!mbar_wait(&P.acc_full, (unsigned)(j & 1), a.err, 63)) ok = false;
       // a warp's lanes stay together: the loads below and the shuffles are the warp's
       ok = __all_sync(0xffffffffu, ok);
@@ -398,12 +439,10 @@ __global__ void __launch_bounds__(kQfThreads, 1) k_qf_gemm(const __grid_constant
         else if (x[i] != 0 && ey > 0) acc[i] += __hiloint2double(h + (ei - 53) * (1 << 20), __double2loint(y));
       }
     }
-    if (ok && mt * kQfM + row < a.n) {
-      double *out = a.part + (((long long)g * a.tiles + tile) * kQfM + row) * kQfN + c0;
+    if (ok && own)
 #pragma unroll
       for (int i = 0; i < 32; ++i)
         if (c0 + i < rows_b) out[i] = acc[i];
-    }
   }
   tc_fence_before();
   __syncthreads();
@@ -444,19 +483,17 @@ __global__ void __launch_bounds__(256)
   }
 }
 
-// Digits of an operand; ng > 0: a field of that grid, in bricks.
+// Digits of an operand.
 struct QfForm {
   int mode = 0;
   const double *X = nullptr, *dX = nullptr, *w = nullptr, *u = nullptr;
   double dV = 0.0;
 };
-static int blocks_of(const Quad64 &q, long long N, bool grid) {
-  return grid ? (int)quad64_grid_exponents(q.n, q.ng) / quad64_rows(q.n) : (int)quad64_linear_blocks(N);
-}
-static void form(const Quad64 &q, const QfForm &f, long long N, bool grid, int *e, char *out, cudaStream_t st) {
+static void form(const Quad64 &q, const QfForm &f, long long N, bool grid, int b0, int b1, int *e, char *out,
+                 cudaStream_t st) {
   QfSource a{f.X, f.dX, f.w, f.u, f.dV, q.n, quad64_rows(q.n), q.ng, quad64_parts(q.ng), N, grid ? q.first : nullptr,
-             e, out};
-  const int blocks = blocks_of(q, N, grid), groups = ceil_div(q.n, kQfFormRows);
+             b0, e, out};
+  const int blocks = b1 - b0, groups = ceil_div(q.n, kQfFormRows);
   // few bricks: the rows over several blocks, until there are eight blocks an SM
   const dim3 g(blocks, std::max(1, std::min(groups, ceil_div(8 * 152, blocks))));
   const size_t smem = form_smem(f.mode);
@@ -470,64 +507,74 @@ static void form(const Quad64 &q, const QfForm &f, long long N, bool grid, int *
   else go(k_qf_digits<2>);
 }
 
-static void product(const Quad64 &q, const char *A, const char *B, const int *eA, const int *eB, long long N, bool grid,
-                    bool sym, bool tr, double scale, bool accumulate, double *M, cudaStream_t st) {
+// An operand of a product: digits to be formed, segment by segment, or those of the
+// AOs where the plan keeps them (X null).
+static QfForm kept() { return QfForm{}; }
+
+// M (+)= scale sum over the points; same: both operands are fa.  The sums run
+// segment by segment whether or not digits are kept, so the bits do not depend on that.
+static void product(const Quad64 &q, const QfForm &fa, const QfForm &fb, bool same, long long N, bool grid, bool sym,
+                    bool tr, double scale, bool accumulate, double *M, cudaStream_t st) {
   QfArgs a{};
-  a.A = A;
-  a.B = B;
-  a.eA = eA;
-  a.eB = eB;
+  a.wholeA = !fa.X;
+  a.wholeB = same ? a.wholeA : !fb.X;
+  a.A = a.wholeA ? q.B : q.A;
+  a.eA = a.wholeA ? q.eB : q.eA;
+  a.B = same ? a.A : a.wholeB ? q.B : q.X;
+  a.eB = same ? a.eA : a.wholeB ? q.eB : q.eX;
   a.first = grid ? q.first : nullptr;
   a.part = q.part;
   a.err = q.err;
-  a.blocks = blocks_of(q, N, grid);
   a.stages = grid ? q.stages : ceil_div(N, kQfK);
   a.n = q.n;
   a.rows = quad64_rows(q.n);
   a.tiles = quad64_tiles(q.n, sym, a.tile);
   a.groups = quad64_groups(q.n, sym);
   ensure_dyn_smem((const void *)k_qf_gemm, kQfSmem);
-  k_qf_gemm<<<dim3(a.tiles, a.groups), kQfThreads, kQfSmem, st>>>(a);
-  HQ_LAUNCH_CHECK();
+  const Segments sg = grid ? grid_segments(q.n, q.ng, q.stages) : linear_segments(q.n, N);
+  for (int k = 0; k < sg.count; ++k) {
+    a.b0 = sg.begin(k);
+    a.b1 = sg.begin(k + 1);
+    a.add = k > 0;
+    HQ_REQUIRE((size_t)(a.b1 - a.b0) * a.rows <= q.exponents, "segment beyond the plan's digit buffers");
+    if (fa.X) form(q, fa, N, grid, a.b0, a.b1, q.eA, q.A, st);
+    if (!same && fb.X) form(q, fb, N, grid, a.b0, a.b1, q.eX, q.X, st);
+    k_qf_gemm<<<dim3(a.tiles, a.groups), kQfThreads, kQfSmem, st>>>(a);
+    HQ_LAUNCH_CHECK();
+  }
   k_qf_reduce<<<dim3(ceil_div(q.n, 32), q.n), 256, 0, st>>>(a, sym, tr, scale, accumulate, M);
   HQ_LAUNCH_CHECK();
 }
 
 void quad64_basis(const Quad64 &q, const double *phi, long long N, cudaStream_t st) {
   HQ_STAGE(ST_SPLIT, st);
-  form(q, QfForm{0, phi}, N, true, q.eB, q.B, st);
+  if (q.B) form(q, QfForm{0, phi}, N, true, 0, grid_segments(q.n, q.ng, q.stages).blocks, q.eB, q.B, st);
 }
+
+static QfForm basis(const Quad64 &q, const double *phi) { return q.B ? kept() : QfForm{0, phi}; }
 
 void quad64_weighted(const Quad64 &q, const double *phi, const double *w, long long N, double scale, double *M,
                      cudaStream_t st) {
   HQ_STAGE(ST_QUAD, st);
-  if (!w) {
-    product(q, q.B, q.B, q.eB, q.eB, N, true, true, false, scale, false, M, st);
-    return;
-  }
-  form(q, QfForm{1, phi, nullptr, w}, N, true, q.eA, q.A, st);
-  product(q, q.A, q.B, q.eA, q.eB, N, true, true, false, scale, false, M, st);
+  if (w) product(q, QfForm{1, phi, nullptr, w}, basis(q, phi), false, N, true, true, false, scale, false, M, st);
+  else product(q, basis(q, phi), {}, true, N, true, true, false, scale, false, M, st);
 }
 
 void quad64_gga(const Quad64 &q, const double *phi, const double *dphi, const double *w, const double *u, double dV,
                 long long N, double *M, cudaStream_t st) {
   HQ_STAGE(ST_QUAD, st);
-  form(q, QfForm{2, phi, dphi, w, u, dV}, N, true, q.eA, q.A, st);
-  product(q, q.A, q.B, q.eA, q.eB, N, true, false, true, 1.0, false, M, st);
+  product(q, QfForm{2, phi, dphi, w, u, dV}, basis(q, phi), false, N, true, false, true, 1.0, false, M, st);
 }
 
 void quad64_gram(const Quad64 &q, const double *Q, long long N, bool accumulate, double *M, cudaStream_t st) {
   HQ_STAGE(ST_QUAD, st);
-  form(q, QfForm{0, Q}, N, false, q.eA, q.A, st);
-  product(q, q.A, q.A, q.eA, q.eA, N, false, true, false, 1.0, accumulate, M, st);
+  product(q, QfForm{0, Q}, {}, true, N, false, true, false, 1.0, accumulate, M, st);
 }
 
 void quad64_pair(const Quad64 &q, const double *phi, const double *w, const double *Y, long long N, double scale,
                  bool accumulate, double *M, cudaStream_t st) {
   HQ_STAGE(ST_QUAD, st);
-  form(q, QfForm{1, phi, nullptr, w}, N, true, q.eA, q.A, st);
-  form(q, QfForm{0, Y}, N, true, q.eX, q.X, st);
-  product(q, q.A, q.X, q.eA, q.eX, N, true, false, false, scale, accumulate, M, st);
+  product(q, QfForm{1, phi, nullptr, w}, QfForm{0, Y}, false, N, true, false, false, scale, accumulate, M, st);
 }
 
 }  // namespace hqcgb
