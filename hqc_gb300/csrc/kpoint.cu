@@ -446,6 +446,7 @@ struct hqcgb_kplan {
   // group, FP64 partial tiles and the 2n x 2n product
   long long ld = 0, ldq = 0;
   int ldk2 = 0, xg = 1;
+  bool XT_ready = false;  // XT holds this geometry
   float *X32 = nullptr, *Xhl = nullptr, *zhl = nullptr, *w32 = nullptr, *XT = nullptr, *Yhl = nullptr,
         *psi32 = nullptr, *Qhl = nullptr;
   float2 *Pc = nullptr;
@@ -652,7 +653,6 @@ static void kcreate(const hqcgb_params &P, hqcgb_kplan *p) {
     p->Xhl = p->alloc<float>((size_t)2 * n2 * p->ld);
     p->zhl = p->alloc<float>((size_t)2 * n2 * p->ld);
     p->w32 = p->alloc<float>(p->ld);
-    p->XT = p->alloc<float>((size_t)N * p->ldk2);
     p->Yhl = p->alloc<float>((size_t)2 * 64 * p->ldk2);
     const int nchunk = (nao + 31) / 32;
     p->psi32 = p->alloc<float>((size_t)nchunk * 64 * N);
@@ -781,9 +781,15 @@ static int kx_density(KCtx &c) {
     k_kx_psi_operand<<<ceil_div(npsi * p->ldk2, 256), 256, 0, c.st>>>(p->C, p->occ, n, c0, m, npsi, p->ldk2,
                                                                        p->Yhl);
     HQ_LAUNCH_CHECK();
+    // the grid-major copy, once per geometry, where more than 16 orbitals or 144 AOs need it
+    if (!tc_psi_resident(npsi, p->ldk2) && !p->XT_ready) {
+      if (!p->XT) p->XT = p->alloc<float>((size_t)N * p->ldk2);
+      launch_transpose_phi(p->X32, 2 * n, N, p->ld, p->XT, c.st);
+      p->XT_ready = true;
+    }
     double *dst = c0 == 0 ? p->rho : p->rhoc;
-    launch_tc_psi_density(p->X32, nullptr, 2 * n, p->ld, p->XT, nullptr, p->Yhl, npsi, p->ldk2, N, dst, nullptr, p->tc_err, c.st,
-                          p->psi32 + (size_t)(c0 / 32) * 64 * N, 2);
+    launch_tc_psi_density(p->X32, nullptr, 2 * n, p->ld, p->XT, nullptr, p->Yhl, npsi, p->ldk2, N, dst, nullptr,
+                          p->tc_err, c.st, p->psi32 + (size_t)(c0 / 32) * 64 * N, 2);
     if (c0 > 0) {
       k_kx_add<<<ceil_div(N, 256), 256, 0, c.st>>>(N, p->rhoc, p->rho);
       HQ_LAUNCH_CHECK();
@@ -977,11 +983,11 @@ static void kgeometry(KCtx &c, const double *xp_dev, const double *kpt_host) {
                                                                    p->nb, p->nprim, n, p->ng, p->phi,
                                                                    p->dphi);
     HQ_LAUNCH_CHECK();
-    if (p->mixed) {  // the embedded FP32 rows, their TF32 pieces and the grid-major copy
+    if (p->mixed) {  // the embedded FP32 rows and their TF32 pieces
       k_kx_embed<<<ceil_div((long long)n * p->ld, 256), 256, 0, c.st>>>(p->phi, n, N, p->ld, p->X32);
       HQ_LAUNCH_CHECK();
       launch_split_operand(p->X32, nullptr, nullptr, nullptr, 2 * n, N, p->ld, p->ld, 1.f, 0.f, p->Xhl, c.st);
-      launch_transpose_phi(p->X32, 2 * n, N, p->ld, p->XT, c.st);
+      p->XT_ready = false;
     }
   }
   launch_overlap_kinetic_kpt(p->xp, p->n, p->nb, p->nprim, p->alpha, p->coef, p->ao_l, p->ao_cart,

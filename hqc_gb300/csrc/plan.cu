@@ -379,8 +379,6 @@ static void create(const hqcgb_params *in, hqcgb_plan *p, long long digit_budget
   if (p->mixed) {
     p->phi32 = p->alloc<float>((size_t)nao * p->ld);
     if (p->gga) p->dphi32 = p->alloc<float>((size_t)3 * nao * p->ld);
-    p->phiT32 = p->alloc<float>((size_t)N * tc_ldk(nao));
-    if (p->gga) p->dphiT32 = p->alloc<float>((size_t)3 * N * tc_ldk(nao));
     p->Yhl = p->alloc<float>((size_t)2 * tc_psi_max(false) * tc_ldk(nao));
     p->hocc.resize(nao);
     p->D32 = p->alloc<float>((size_t)nao * tc_ldk(nao));
@@ -820,11 +818,14 @@ static void exchange_gradient(Ctx &c, double *grad) {
 }
 
 // The grid-major copies of phi and its gradient, once per geometry, for the
-// density forms that read them (many orbitals or AOs).
+// density forms that read them (many orbitals or AOs); a plan that takes no such form
+// never holds them (2.45 GB of an H54 dzvp PBE plan at 81^3).
 static void grid_major(Ctx &c) {
   hqcgb_plan *p = c.p;
   if (p->phiT_ready) return;
   const int n = p->nao;
+  if (!p->phiT32) p->phiT32 = p->alloc<float>((size_t)p->N * tc_ldk(n));
+  if (p->gga && !p->dphiT32) p->dphiT32 = p->alloc<float>((size_t)3 * p->N * tc_ldk(n));
   launch_transpose_phi(p->phi32, n, p->N, p->ld, p->phiT32, c.st);
   if (p->gga)
     for (int d = 0; d < 3; ++d)

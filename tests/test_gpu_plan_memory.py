@@ -24,14 +24,16 @@ def _solver(n, grid, basis="gth-dzvp", **kw):
     return make_solver(n, box(n), 1.4, basis, n_grid=grid, **kw)
 
 
-# bytes a value of an AO on the grid: phi, grad phi, D phi and the GGA force's two operands in FP64
-@pytest.mark.parametrize("precision,value_bytes", [("fp64", 7 * 8)])
-def test_a_plan_holds_little_more_than_its_grids(precision, value_bytes):
+# bytes a value of an AO on the grid: phi, grad phi, D phi and the GGA force's two operands in FP64;
+# phi, grad phi and the two pieces of phi and of the quadrature's operand in FP32, and bytes a
+# point of the orbitals and their gradients that mixed forces keep (64 of them)
+@pytest.mark.parametrize("precision,value_bytes,point_bytes", [("fp64", 7 * 8, 0), ("mixed", 8 * 4, 4 * 64 * 4)])
+def test_a_plan_holds_little_more_than_its_grids(precision, value_bytes, point_bytes):
     n, grid = 54, 61
     before = _used()
     s = _solver(n, grid, dft=True, xc="pbe", forces=True, precision=precision)
     held = _used() - before
-    assert held <= 1.25 * s.plan.nao * grid ** 3 * value_bytes
+    assert held <= 1.25 * grid ** 3 * (s.plan.nao * value_bytes + point_bytes)
 
 
 # four workers: the digits of the first plan are kept, those of the others do not fit the limit any more
