@@ -110,9 +110,12 @@ __global__ void __launch_bounds__(T * T)
   if (i0 + ty < M && j0 + tx < N) C[(long long)(i0 + ty) * ldc + j0 + tx] = acc;
 }
 
-// From these sizes on the products are the engine's own; smaller ones go to
-// cuBLAS, whose kernels split K there.
-constexpr int kDgMin = 28;
+// From this size on the products are the engine's own.  There the library changes to
+// kernels that add in the order of k, as k_dgemm does, so the two give the same bits
+// (n = 17 to 32, square and thin products compared); below, its kernels split K, and
+// bits would move.  n = 12 4.1 us (own) / 6 to 14 (library, by transposition), 16 4.1 /
+// 6 to 14, 17 4.1 / 12.4, 28 4.1 / 12.4, 64 6.2 / 22.5.
+constexpr int kDgMin = 17;
 static void dgemm(bool ta, bool tb, int M, int N, int K, const double *A, int lda, const double *B, int ldb, double *C,
                   int ldc, cudaStream_t st) {
   auto go = [&](auto kernel, int t) {
