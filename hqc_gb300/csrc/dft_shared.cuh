@@ -405,7 +405,11 @@ static __device__ double2 *fold_axis0_any(double2 *buf, double2 *tmp, int n, int
 
 // DFT along axis 0 of buf [n][ncol], n odd, with tmp of the same size: returns
 // the one of the two that holds the result.  The fixed-size transforms for 25,
-// 33, 49, 65 and 81 points, the generic routine otherwise.
+// 33, 49, 65 and 81 points (the grids of the benchmark systems), the generic routine
+// otherwise: two factors in loops over the largest length a factor may have, primes
+// and long factors as direct sums.  What that costs, FP64 Hartree potential (five
+// passes): 45 / 49 / 51 / 55 points 97 / 72 / 164 / 135 us, 61 / 63 / 65 / 69 134 / 137 /
+// 106 / 215, 73 / 75 / 77 / 81 256 / 173 / 152 / 168.
 template <typename R, typename R2>
 __device__ R2 *dft_axis0(R2 *buf, R2 *tmp, int n, int ncol, int n1, const R2 *w) {
   if constexpr (sizeof(R) == 8) {

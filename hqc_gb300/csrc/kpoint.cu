@@ -47,11 +47,14 @@ static constexpr double kMadelungK = 0.22578495;  // solver.py:404, 510
 // exx_occ_threshold): each adds f_i times a bounded matrix to K, below FP64
 // rounding of the sum; with Fermi smearing most virtual orbitals are such.
 static constexpr double kExxOccFloor = 1e-14;
-// AOs from which an FP64 plan takes the tiled contractions and folded transforms
-// (H8 dzv at 33^3, 16 AOs, two k-points of Hartree-Fock: 237 -> 71 ms).  Fewer
-// rows leave a 16 x 16 tile mostly padding, and four-atom Hartree-Fock under
-// strong smearing often runs to the iteration limit without converging, where
-// a result is the rounding's: those keep the library's sums.
+// AOs from which an FP64 plan takes the tiled contractions and folded transforms.
+// They are faster at every size (one k-point, 33^3, Hartree-Fock / LDA: 4 AOs 21 ->
+// 13 / 15 -> 11 ms, 8 AOs 62 -> 26 / 24 -> 14, 14 AOs 103 -> 34 / 24 -> 17; H8 dzv, 16
+// AOs, two k-points of Hartree-Fock 237 -> 71), so the line is not one of speed: the
+// smeared meshes of four to six atoms that lie below it are loosely determined at the
+// default tolerance, and a change of rounding alone moves their converged density
+// matrices by 4e-7 (Hartree-Fock) and 1e-9 (LDA), beyond the 1e-9 that FP64 results
+// keep from one version to the next (from 14 AOs: 2e-10 and less).
 static constexpr int kTiledNao = 16;
 
 // Factor table F[A][d][i][a][s] (complex): s = 3 l + k, k = value, first and
