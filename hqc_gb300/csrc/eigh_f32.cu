@@ -1,20 +1,22 @@
 // FP32 stage of the mixed-precision eigensolver: eigenpairs of a symmetric
 // n x n matrix to single precision, for the FP64 refinement in
-// eigh_mixed.cu.  Three kernels:
+// eigh_mixed.cu.  Three steps:
 //
-//  1. k_tridiag_f32_smem (one block): Householder reduction to tridiagonal
-//     T = Q^T A Q with the matrix in shared memory (k_tridiag_f32, the
-//     global-memory form of eigh_tridiag.cuh, above 310 AOs), reflectors
-//     stored contiguously.
-//  2. k_tri_values_f32 (a thread per eigenvalue): the eigenvalues of T by
+//  1. Householder reduction to tridiagonal T = Q^T A Q, reflectors stored
+//     contiguously: up to 95 AOs one block with the lower triangle in shared
+//     memory (k_tridiag_f32_smem), to 512 a cluster of eight SMs
+//     (k_tridiag_cluster in eigh_ql_f32.cu), above one block on global memory
+//     (k_tridiag_f32, the form of eigh_tridiag.cuh).
+//  2. k_tri_values_f32 (a warp per eigenvalue): the eigenvalues of T by
 //     bisection on Sturm counts (W. Barth, R. S. Martin, J. H.
 //     Wilkinson, "Calculation of the eigenvalues of a symmetric tridiagonal
 //     matrix by the method of bisection", Numer. Math. 9 (1967) 386-393), all
-//     in parallel; then the eigenvectors of T by inverse iteration with a
-//     partial-pivoting LU of T - lambda I (J. H. Wilkinson, "The Algebraic
-//     Eigenvalue Problem", 1965, ch. 5), eigenvalues closer than 1e-4 ||T||
-//     treated as a cluster whose vectors one thread computes in turn,
-//     orthogonalising each against the earlier ones (modified Gram-Schmidt).
+//     in parallel; k_tri_vectors_f32 (a warp per cluster): the eigenvectors of
+//     T by inverse iteration with a partial-pivoting LU of T - lambda I (J. H.
+//     Wilkinson, "The Algebraic Eigenvalue Problem", 1965, ch. 5), eigenvalues
+//     closer than 1e-4 ||T|| treated as a cluster whose vectors one warp
+//     computes in turn, orthogonalising each against the earlier ones (modified
+//     Gram-Schmidt).
 //  3. k_backtransform_f32 (a block per 32 columns): V = Q Z, the reflectors
 //     applied in reverse order to column tiles held in shared memory.
 //
@@ -53,7 +55,7 @@ __global__ void __launch_bounds__(kTriThreads)
 // The same reduction with the matrix held in shared memory as a packed lower
 // triangle (element (i, j), i >= j, at i (i + 1) / 2 + j): the symmetric
 // matrix-vector product and the rank-2 update of each step touch only shared
-// memory.  For n with n (n + 1) / 2 + 5 n floats within the shared-memory
+// memory.  Takes n with n (n + 1) / 2 + 5 n floats within the shared-memory
 // budget (n <= 310).
 __device__ inline int tri_ix(int i, int j) { return i * (i + 1) / 2 + j; }
 

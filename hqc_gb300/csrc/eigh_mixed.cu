@@ -33,18 +33,9 @@ __global__ void k_f32_to_f64(long long n, const float *__restrict__ a, double *_
   if (i < n) b[i] = (double)a[i];
 }
 
-// One block: lambda, delta, the clusters and the correction E from
-// S = X^T A X and G = X^T X.
-//
-// Clusters (Ogita, Aishima, "Iterative refinement for symmetric eigenvalue
-// decomposition II: clustered eigenvalues", Japan J. Indust. Appl. Math. 36
-// (2019) 435-459): eigenvalue estimates closer than delta form a cluster,
-// within which the basic update only re-orthogonalises.  Each cluster C is
-// therefore rotated first by the eigenvectors W_C of its block S_CC (cyclic
-// Jacobi, one thread per cluster): X_C <- X_C W_C, S <- W^T S W and
-// G <- W^T G W, after which the cluster's Ritz values are separated and the
-// next iteration converges quadratically again.  Clusters larger than
-// kMaxCluster are left unrotated and flagged in emax[2].
+// A refinement step: statistics of S = X^T A X and G = X^T X (k_oa_stats), estimates
+// and clusters (k_oa_clusters), the clusters' rotations (k_oa_jacobi, k_oa_rotate_*),
+// the correction E (k_oa_update).
 // emax[0] = max |E|, emax[1] = ||S - diag(l)||_F / ||A||_F before the
 // update, emax[2] = 1 when a cluster was too large, emax[3] = cluster count.
 constexpr int kMaxCluster = 48;      // largest cluster rotated (wide spectra)
@@ -462,9 +453,10 @@ static double oa_iteration(int n, const double *A, double *X, double *w, MixedEi
   return off;
 }
 
-// Full solve: FP32 stage (eigh_f32.cu; the QL solver of eigh_fp64.cu when
-// `wide`), then refinement until the relative
-// off-diagonal norm measured before a step is at rounding level (1e-12).
+// Full solve: FP32 stage (eigh_f32.cu; when `wide` the QL solver, of
+// eigh_ql_f32.cu up to 512 AOs and of eigh_fp64.cu above), then refinement until
+// the relative off-diagonal norm measured before a step is at rounding level
+// (1e-12).
 // Returns false when the refinement does not get there within its steps (the
 // caller then uses the FP64 solver).
 bool eigh_mixed(int n, const double *A, double *V, double *w, MixedEigWork &ws, cudaStream_t st,
