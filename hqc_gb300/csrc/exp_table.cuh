@@ -17,22 +17,39 @@ inline void exp_table(double *t) {
   for (int j = 0; j < kExpTable; ++j) t[j] = std::exp2(j / 64.0);
 }
 
-__device__ inline double exp_neg(double x, const double *__restrict__ tab) {
-  constexpr double kMagic = 6755399441055744.0;  // 1.5 * 2^52: the sum's low word is the rounded integer
-  constexpr double kInv = 64.0 / 0.693147180559945309417;
-  constexpr double kHi = 0x1.62e42feep-1 / 64.0, kLo = 0x1.a39ef35793c76p-33 / 64.0;
-  const double t = fma(x, kInv, kMagic);
-  const int k = __double2loint(t);
-  const double kd = t - kMagic;
-  double r = fma(kd, -kHi, x);
-  r = fma(kd, -kLo, r);
+constexpr double kExpMagic = 6755399441055744.0;  // 1.5 * 2^52: the sum's low word is the rounded integer
+constexpr double kExpInv = kExpTable / 0.693147180559945309417;
+constexpr double kExpHi = 0x1.62e42feep-1 / kExpTable, kExpLo = 0x1.a39ef35793c76p-33 / kExpTable;
+
+// 2^(k/64) e^r
+__device__ inline double exp_reduced(int k, double r, const double *__restrict__ tab) {
   double q = fma(r, 1.0 / 120.0, 1.0 / 24.0);
   q = fma(q, r, 1.0 / 6.0);
   q = fma(q, r, 0.5);
   const double p = fma(q, r * r, r);
   const double T = tab[k & (kExpTable - 1)];
   const double s = __hiloint2double(__double2hiint(T) + ((k >> 6) << 20), __double2loint(T));
-  return x > -708.0 ? fma(s, p, s) : (x != x ? x : 0.0);
+  return fma(s, p, s);
+}
+
+__device__ inline double exp_neg(double x, const double *__restrict__ tab) {
+  const double t = fma(x, kExpInv, kExpMagic);
+  const double kd = t - kExpMagic;
+  double r = fma(kd, -kExpHi, x);
+  r = fma(kd, -kExpLo, r);
+  const double v = exp_reduced(__double2loint(t), r, tab);
+  return x > -708.0 ? v : (x != x ? x : 0.0);
+}
+
+// exp(-al y), c = al kExpInv: the product enters the reduction unrounded (rounded, an
+// exponent of 41 costs up to 20 eps).
+__device__ inline double exp_neg_product(double al, double c, double y, const double *__restrict__ tab) {
+  const double t = fma(y, -c, kExpMagic);
+  const double kd = t - kExpMagic;
+  double r = fma(-al, y, -(kd * kExpHi));
+  r = fma(kd, -kExpLo, r);
+  const double v = exp_reduced(__double2loint(t), r, tab);
+  return kd > -708.0 * kExpInv ? v : (kd != kd ? kd : 0.0);
 }
 
 }  // namespace hqcgb

@@ -39,6 +39,12 @@ template <> __device__ inline double2 zzero<double2>() { return make_double2(0.0
 // image t0 + m contributes exp(-alpha m a (m a -+ 2 |u|)) <= 1, and the three
 // nearest ones share one exponential:
 //   f_x f_y f_z = exp(-alpha |u|^2) prod_d sum_m w_m,d  (l = 1: (u - m a) w).
+// A nearest image scaled to 1 rounds at the worst place of the mantissa, so the other
+// images are summed without it, and alpha |u|^2 is not rounded: error of the values
+// against extended precision, H8 dzv / H14 dzvp / H32 szv, the plain image sums 1.8e-16 /
+// 2.2e-16 / 1.7e-16, without either 2.5e-16 / 2.7e-16 / 2.0e-16, so 1.4e-16 / 2.0e-16 /
+// 1.65e-16.  At a k-point 1.9e-16 / 2.2e-16 / 1.8e-16 the sums, 1.6e-16 / 2.1e-16 /
+// 1.8e-16 here.
 // Factors below e^-41 (1.6e-18 of the nearest image's term) are left out;
 // their exponents are tested in FP32.  For sharp primitives no other image
 // counts, so a point and atom take about 25 exponentials of 11 FP64
@@ -52,12 +58,15 @@ __global__ void __launch_bounds__(128)
               const int *__restrict__ ao_l, const int *__restrict__ ao_cart, const double *__restrict__ xp,
               long long npts, int pts_per_group, const double *__restrict__ xe, Z *__restrict__ out) {
   constexpr bool kPhase = sizeof(Z) > sizeof(double);
-  __shared__ double s_exp[kExpTable], s_alpha[kPtMaxPrim], s_coef[NB * kPtMaxPrim];
+  __shared__ double s_exp[kExpTable], s_alpha[kPtMaxPrim], s_ac[kPtMaxPrim], s_coef[NB * kPtMaxPrim];
   __shared__ double2 s_ph[kPhase ? 3 * kPtMaxLat : 1];
   __shared__ int s_type[NB];  // 0: s, 1 + axis: p
   const int nlat = 2 * tm + 1;
   for (int k = threadIdx.x; k < kExpTable; k += blockDim.x) s_exp[k] = tables[k];
-  for (int k = threadIdx.x; k < nprim; k += blockDim.x) s_alpha[k] = tables[kExpTable + k];
+  for (int k = threadIdx.x; k < nprim; k += blockDim.x) {
+    s_alpha[k] = tables[kExpTable + k];
+    s_ac[k] = s_alpha[k] * kExpInv;
+  }
   for (int k = threadIdx.x; k < nb * nprim; k += blockDim.x) s_coef[k] = tables[kExpTable + nprim + k];
   if (kPhase)
     for (int k = threadIdx.x; k < 3 * nlat; k += blockDim.x) {
@@ -91,21 +100,29 @@ __global__ void __launch_bounds__(128)
     u[d] = __dsub_rn(x, __dmul_rn(t, a));  // the image sums' x - lat[t]
     rel[d] = 2.f * (float)(u[d] * inv_a);
   }
-  const double r2 = u[0] * u[0] + u[1] * u[1] + u[2] * u[2];
+  double r2, r2l = 0.0;  // |u|^2 and, for the complex values with their more roundings, what its sum left out
+  if (kPhase) {
+    const double p = __dmul_rn(u[0], u[0]), q = __dmul_rn(u[1], u[1]), w = __dmul_rn(u[2], u[2]);
+    const double s = p + q, z = s - p, z2 = (r2 = s + w) - s;
+    r2l = ((p - (s - z)) + (q - z)) + ((s - (r2 - z2)) + (w - z2)) + fma(u[0], u[0], -p) + fma(u[1], u[1], -q) +
+          fma(u[2], u[2], -w);
+  } else {
+    r2 = u[0] * u[0] + u[1] * u[1] + u[2] * u[2];
+  }
   Z v[NB];
 #pragma unroll
   for (int j = 0; j < NB; ++j) v[j] = zzero<Z>();
   for (int q = 0; q < nprim; ++q) {
     const double al = s_alpha[q], ala = -al * a;
     const float alf = (float)ala * (float)a;
-    Z S0[3], S1[3];
+    Z S0[3], S1[3];  // S0 without the nearest image's term, the largest, which joins last
 #pragma unroll
     for (int d = 0; d < 3; ++d) {
       auto phase = [&](int m) {
         if constexpr (kPhase) return s_ph[d * nlat + t0[d] + tm + m];
         else return 1.0;
       };
-      S0[d] = phase(0);
+      S0[d] = zzero<Z>();
       S1[d] = zmul(u[d], phase(0));
 #pragma unroll
       for (int side = -1; side <= 1; side += 2) {
@@ -123,10 +140,19 @@ __global__ void __launch_bounds__(128)
         }
       }
     }
-    const double e = exp_neg(-al * r2, s_exp);
-    const Z yz = zmul(S0[1], S0[2]), ex = zmul(e, S0[0]);
-    const Z P0 = zmul(ex, yz), P1 = zmul(zmul(e, S1[0]), yz), P2 = zmul(ex, zmul(S1[1], S0[2])),
-            P3 = zmul(ex, zmul(S0[1], S1[2]));
+    double e = exp_neg_product(al, s_ac[q], r2, s_exp);
+    if (kPhase && e > 0.0) e = fma(e, -al * r2l, e);  // not where |u|^2 is infinite
+    Z P0, P1, P2, P3;
+    if constexpr (kPhase) {
+#pragma unroll
+      for (int d = 0; d < 3; ++d) zfma(1.0, s_ph[d * nlat + t0[d] + tm], S0[d]);
+      const Z yz = zmul(S0[1], S0[2]), ex = zmul(e, S0[0]);
+      P0 = zmul(ex, yz), P1 = zmul(zmul(e, S1[0]), yz), P2 = zmul(ex, zmul(S1[1], S0[2])),
+      P3 = zmul(ex, zmul(S0[1], S1[2]));
+    } else {  // v (1 + S0) in one rounding
+      const Z ex = fma(e, S0[0], e), xy = fma(ex, S0[1], ex), px = e * S1[0], pxy = fma(px, S0[1], px), py = ex * S1[1];
+      P0 = fma(xy, S0[2], xy), P1 = fma(pxy, S0[2], pxy), P2 = fma(py, S0[2], py), P3 = xy * S1[2];
+    }
 #pragma unroll
     for (int j = 0; j < NB; ++j) {
       if (j >= nb) break;
