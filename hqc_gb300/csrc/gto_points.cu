@@ -42,7 +42,7 @@ template <> __device__ inline double2 zzero<double2>() { return make_double2(0.0
 // A nearest image scaled to 1 rounds at the worst place of the mantissa, so the other
 // images are summed without it, and alpha |u|^2 is not rounded: error of the values
 // against extended precision, H8 dzv / H14 dzvp / H32 szv, the plain image sums 1.8e-16 /
-// 2.2e-16 / 1.7e-16, without either 2.5e-16 / 2.7e-16 / 2.0e-16, so 1.4e-16 / 2.0e-16 /
+// 2.2e-16 / 1.7e-16, without either 2.5e-16 / 2.7e-16 / 2.0e-16, so 1.4e-16 / 2.1e-16 /
 // 1.65e-16.  At a k-point 1.9e-16 / 2.2e-16 / 1.8e-16 the sums, 1.6e-16 / 2.1e-16 /
 // 1.8e-16 here.
 // Factors below e^-41 (1.6e-18 of the nearest image's term) are left out;
