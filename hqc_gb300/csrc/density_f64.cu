@@ -9,16 +9,20 @@
 // psi^2, three operations an orbital and point where the sum over D takes an
 // operation an AO pair and point.
 //
-// Layout: phi^T (and the gradient's three fields) by tiles of 128 points,
-// [field][tile][block of 32 AOs][pair][128 rows][128 bytes], a stage's 64 KB in
-// one piece; Y^T by 64 orbitals, [column block][block of 32 AOs][pair][64][128].
-// Digits of all tiles are kept for a geometry where the plan affords it, otherwise
-// formed for a range of tiles at a time (the same bits: points are independent).
-// Persistent CTAs, one an SM, take tiles in turn: a copy thread, an MMA thread,
-// eight drain warps.  Bound by the drains: conversion of the TMEM sums and the
-// FP64 squares.  Measured, against the sum over D on the FP64 pipe: 64 AOs, up to 64
-// orbitals, 65^3 points 1.87 -> 0.18 ms; 70 AOs, 7 orbitals, 49^3 points with the
-// gradient 1.05 -> 0.18 ms.
+// A tile of the sum is 128 points.  Eight warps read phi (and the gradient's three
+// fields) for it and form the digits in the K-major SW128 pattern of the ring, 32 AOs a
+// stage, a lane a point and 16 AOs; kept in memory those digits would be 16 bytes a value
+// (9.8 GB of an H54 dzvp PBE plan at 81^3), written once a geometry and read for every
+// density where phi is read now.  Y^T by 64 orbitals,
+// [column block][block of 32 AOs][pair][64][128], comes by bulk copies.  Persistent CTAs,
+// one an SM, take tiles in turn: the forming warps, a copy thread, an MMA warp, eight
+// drain warps.  Bound by the MMAs (72 a stage) and the instructions that form their digits
+// (about 80 a value) together.  Measured: 64 AOs, 38 orbitals, 65^3 points 0.18 ms (sum over
+// D on the FP64 pipe 1.87, digits kept in memory 0.18); 70 AOs, 7 orbitals, 49^3 with the
+// gradient 0.23 (1.05, 0.18); 270 AOs, 27 orbitals, 65^3 with the gradient 1.36 (kept 1.06,
+// digits of a range of tiles formed in memory before its part of the density 3.5).  With
+// four forming warps 2.5; eight, whose 18 warps leave 96 registers and some spills of the
+// drains' in the gradient form, but 136 registers for those by setmaxnreg were slower.
 #include <algorithm>
 #include <cmath>
 
@@ -34,15 +38,13 @@ constexpr uint32_t kDfPairA = kDfM * 128, kDfPairB = kDfN * 128;
 constexpr uint32_t kDfOffB = kQfPairs * kDfPairA;
 constexpr uint32_t kDfStage = kQfPairs * (kDfPairA + kDfPairB);
 constexpr size_t kDfSmem = kDfRing * kDfStage + 1024;
-constexpr int kDfDrainWarps = 8;
-constexpr int kDfThreads = (kDfDrainWarps + 2) * 32;
+constexpr int kDfDrainWarps = 8, kDfFormWarps = 8;
+constexpr int kDfThreads = (kDfDrainWarps + 2 + kDfFormWarps) * 32;
+constexpr int kDfHalf = kDfFormWarps * 32 / kDfM, kDfRun = kDfK / kDfHalf;  // AOs of a stage that a lane forms
 constexpr int kDfMaxAo = 512;  // one TMEM sum holds 512 terms exactly
 
 int density64_max_ao() { return kDfMaxAo; }
 static int df_blocks(int nao) { return ceil_div(nao, kDfK); }
-int density64_tiles(long long N) { return ceil_div(N, kDfM); }
-int density64_min_tiles(long long N) { return std::min(152, density64_tiles(N)); }
-size_t density64_tile_bytes(int nao, int fields) { return (size_t)fields * df_blocks(nao) * kQfPairs * kDfPairA; }
 size_t density64_orbital_bytes(int nao) {
   return (size_t)ceil_div(nao, kDfN) * df_blocks(nao) * kQfPairs * kDfPairB;
 }
@@ -58,50 +60,6 @@ __global__ void __launch_bounds__(256)
   int k = 0;
   if (m > 0.f && m < INFINITY) frexpf(m, &k);
   scale[g] = m < INFINITY ? scalbn(1.0, k + 1) : NAN;
-}
-
-// Digits of phi^T (blockIdx.y > 0: of a gradient's field): a block takes a tile of
-// 128 points and goes through the AOs 32 at a time, read along the points into shared
-// memory while the 32 before become digits; a lane packs 8 AOs of a point, four lanes a
-// point, so that a warp's store fills the sectors it touches.  Zeros beyond N and nao.
-// Bound by memory (8 bytes read, 16 written a value).  The four fields of 270 AOs at
-// 65^3: 3.4 ms with a lane a point, whose 16-byte stores lay 128 bytes apart, 1.4 now.
-constexpr int kDfLd = kDfM + 1;  // odd: the four lanes of a point read different banks
-__global__ void __launch_bounds__(256, 2)
-    k_df_digits(const double *__restrict__ phi, const double *__restrict__ dphi, int nao, long long N, int nkb, int tile0,
-                const double *__restrict__ scale, char *__restrict__ out) {
-  __shared__ double s_x[kDfK * kDfLd];
-  __shared__ int s_e[kDfM];
-  const int tid = threadIdx.x, f = blockIdx.y, pt = tid & (kDfM - 1), p0 = tid / kDfM * (kDfK / 2);
-  const long long g = (long long)(tile0 + blockIdx.x) * kDfM + pt;
-  const double *X = (f == 0 ? phi : dphi + (long long)(f - 1) * nao * N) + g;
-  if (tid < kDfM) s_e[tid] = g < N ? ((__double2hiint(scale[f * N + g]) >> 20) & 0x7ff) - 1023 : 0;
-  double next[kDfK / 2];
-  auto fetch = [&](int kb) {
-#pragma unroll
-    for (int i = 0; i < kDfK / 2; ++i) {
-      const int p = kb * kDfK + p0 + i;
-      next[i] = g < N && p < nao ? X[(long long)p * N] : 0.0;
-    }
-  };
-  out += ((long long)f * gridDim.x + blockIdx.x) * nkb * kQfPairs * kDfPairA;
-  fetch(0);
-  for (int kb = 0; kb < nkb; ++kb, out += kQfPairs * kDfPairA) {
-#pragma unroll
-    for (int i = 0; i < kDfK / 2; ++i) s_x[(p0 + i) * kDfLd + pt] = next[i];
-    __syncthreads();
-    if (kb + 1 < nkb) fetch(kb + 1);
-#pragma unroll
-    for (int h = 0; h < 2; ++h) {
-      const int r = h * 64 + (tid >> 2), c = tid & 3;
-      const int e = s_e[r];
-      QfPack pack;
-#pragma unroll
-      for (int i = 0; i < 8; ++i) pack.put(i, s_x[(c * 8 + i) * kDfLd + r], e);
-      pack.store(out + r * 128, kDfPairA, c, r);
-    }
-    __syncthreads();
-  }
 }
 
 // Digits of Y^T: block k = orbital, Y_pk = C_pk sqrt(f_k); eY[k] its exponent
@@ -142,15 +100,14 @@ __global__ void __launch_bounds__(128)
 }
 
 struct DfArgs {
-  const char *A, *B;
+  const double *phi, *dphi;
+  const char *B;
   const double *sA;  // [fields][N]
   const int *eY;
   double *rho, *grho, *psi;  // psi [nuse][N] or null
   int *err;
   long long N;
-  size_t field;  // bytes of a field's digits
-  int tile0, tiles;  // the tiles of A
-  int nkb, nuse, cols, bufs;  // cols: TMEM columns of one P_d
+  int nao, tiles, nkb, nuse, cols, bufs;  // cols: TMEM columns of one P_d
 };
 
 struct DfPipe {
@@ -170,7 +127,7 @@ __global__ void __launch_bounds__(kDfThreads, 1) k_df_density(const DfArgs a) {
   auto columns = [&](int cb) { return min(kDfN, a.nuse - cb * kDfN); };
   if (tid == 0) {
     for (int b = 0; b < kDfRing; ++b) {
-      mbar_init(&P.full[b], 1);
+      mbar_init(&P.full[b], 1 + kDfFormWarps * 32);
       mbar_init(&P.empty[b], 1);
     }
     for (int b = 0; b < 2; ++b) {
@@ -184,6 +141,7 @@ __global__ void __launch_bounds__(kDfThreads, 1) k_df_density(const DfArgs a) {
   __syncthreads();
   tc_fence_after();
 
+  const uint32_t tmem = P.tmem_base;
   bool ok = true;
   if (warp == kDfDrainWarps + 1) {
     if (lane == 0) {
@@ -198,60 +156,109 @@ __global__ void __launch_bounds__(kDfThreads, 1) k_df_density(const DfArgs a) {
                 break;
               }
               const uint32_t nb = (uint32_t)((columns(cb) + 7) / 8 * 8) * 128u;
-              mbar_expect_tx(&P.full[slot], kQfPairs * (kDfPairA + nb));
+              mbar_expect_tx(&P.full[slot], kQfPairs * nb);
               const uint32_t dst = smem_u32(sm + slot * kDfStage);
-              bulk_copy(dst, a.A + f * a.field + ((long long)tile * a.nkb + kb) * kQfPairs * kDfPairA,
-                        kQfPairs * kDfPairA, &P.full[slot]);
               const char *srcB = a.B + ((long long)cb * a.nkb + kb) * kQfPairs * kDfPairB;
               for (int q = 0; q < kQfPairs; ++q)
                 bulk_copy(dst + kDfOffB + q * kDfPairB, srcB + q * kDfPairB, nb, &P.full[slot]);
             }
     }
   } else if (warp == kDfDrainWarps) {
-    if (lane == 0) {
-      int st = 0, chain = 0;
-      for (int tile = blockIdx.x; tile < a.tiles && ok; tile += gridDim.x)
-        for (int cb = 0; cb < ncb && ok; ++cb) {
-          const int nn = (columns(cb) + 15) / 16 * 16;
-          // kind::f16, D = F32, A = B = BF16, both K-major
-          const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(nn >> 3) << 17) |
-                                 ((uint32_t)(kDfM >> 4) << 24);
-          for (int f = 0; f < FIELDS && ok; ++f, ++chain) {
-            const int b = chain % a.bufs, use = chain / a.bufs;
-            if (use > 0 && !mbar_wait(&P.acc_empty[b], (unsigned)((use - 1) & 1), a.err, 74)) ok = false;
+    // the warp stays together and one elected lane issues, as in quad_f64.cu
+    int st = 0, chain = 0;
+    for (int tile = blockIdx.x; tile < a.tiles && ok; tile += gridDim.x)
+      for (int cb = 0; cb < ncb && ok; ++cb) {
+        const int nn = (columns(cb) + 15) / 16 * 16;
+        // kind::f16, D = F32, A = B = BF16, both K-major
+        const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(nn >> 3) << 17) |
+                               ((uint32_t)(kDfM >> 4) << 24);
+        for (int f = 0; f < FIELDS && ok; ++f, ++chain) {
+          const int b = chain % a.bufs, use = chain / a.bufs;
+          if (use > 0 && !mbar_wait(&P.acc_empty[b], (unsigned)((use - 1) & 1), a.err, 74)) ok = false;
+          ok = __all_sync(0xffffffffu, ok);
+          tc_fence_after();
+          const uint32_t d0 = tmem + b * kQfDigits * a.cols;
+          for (int kb = 0; kb < a.nkb && ok; ++kb, ++st) {
+            const int slot = st % kDfRing, su = st / kDfRing;
+            if (!mbar_wait(&P.full[slot], (unsigned)(su & 1), a.err, 72)) ok = false;
+            ok = __all_sync(0xffffffffu, ok);
             tc_fence_after();
-            const uint32_t d0 = P.tmem_base + b * kQfDigits * a.cols;
-            for (int kb = 0; kb < a.nkb && ok; ++kb, ++st) {
-              const int slot = st % kDfRing, su = st / kDfRing;
-              if (!mbar_wait(&P.full[slot], (unsigned)(su & 1), a.err, 72)) ok = false;
-              tc_fence_after();
-              if (ok) {
-                const uint64_t dA = sdesc(smem_u32(sm + slot * kDfStage)), dB = dA + (kDfOffB >> 4);
+            const bool el = elect();
+            if (ok && el) {
+              const uint64_t dA = sdesc(smem_u32(sm + slot * kDfStage)), dB = dA + (kDfOffB >> 4);
 #pragma unroll 1
-                for (int ks = 0; ks < kDfK / 16; ++ks)
+              for (int ks = 0; ks < kDfK / 16; ++ks)
 #pragma unroll
-                  for (int s = 0; s < kQfDigits; ++s) {
-                    const uint64_t da = dA + (uint32_t)((s >> 1) * (kDfPairA >> 4) + (s & 1) * 4 + 2 * ks);
+                for (int s = 0; s < kQfDigits; ++s) {
+                  const uint64_t da = dA + (uint32_t)((s >> 1) * (kDfPairA >> 4) + (s & 1) * 4 + 2 * ks);
 #pragma unroll
-                    for (int t = 0; t < kQfDigits - s; ++t)
-                      mma_bf16(d0 + (s + t) * a.cols, da,
-                               dB + (uint32_t)((t >> 1) * (kDfPairB >> 4) + (t & 1) * 4 + 2 * ks), idesc,
-                               !(kb == 0 && ks == 0 && s == 0));
-                  }
-              }
-              mma_commit(&P.empty[slot]);
+                  for (int t = 0; t < kQfDigits - s; ++t)
+                    mma_bf16(d0 + (s + t) * a.cols, da,
+                             dB + (uint32_t)((t >> 1) * (kDfPairB >> 4) + (t & 1) * 4 + 2 * ks), idesc,
+                             !(kb == 0 && ks == 0 && s == 0));
+                }
             }
-            mma_commit(&P.acc_full[b]);
+            if (el) mma_commit(&P.empty[slot]);
+          }
+          if (elect()) mma_commit(&P.acc_full[b]);
+        }
+      }
+  } else if (warp > kDfDrainWarps + 1) {
+    const int t = tid - (kDfDrainWarps + 2) * 32, r = t % kDfM, c0 = t / kDfM * (kDfRun / 8);
+    int st = 0;
+    double v[kDfRun / 8][8];  // each chunk's values are on their way while the others become digits
+    const double *X = nullptr;  // the point's values of the stage that comes next, null beyond N
+    int p0 = 0;
+    auto next = [&](int tile, int f, int kb) {
+      const long long g = (long long)tile * kDfM + r;
+      X = tile < a.tiles && g < a.N ? (f == 0 ? a.phi : a.dphi + (long long)(f - 1) * a.nao * a.N) + g : nullptr;
+      p0 = kb * kDfK + c0 * 8;
+    };
+    auto fetch = [&](int c) {
+#pragma unroll
+      for (int i = 0; i < 8; ++i) {
+        const int p = p0 + c * 8 + i;
+        v[c][i] = X && p < a.nao ? X[(long long)p * a.N] : 0.0;
+      }
+    };
+    next(blockIdx.x, 0, 0);
+#pragma unroll
+    for (int c = 0; c < kDfRun / 8; ++c) fetch(c);
+    for (int tile = blockIdx.x; tile < a.tiles && ok; tile += gridDim.x) {
+      const long long g = (long long)tile * kDfM + r;
+      for (int cb = 0; cb < ncb && ok; ++cb)
+        for (int f = 0; f < FIELDS && ok; ++f) {
+          const int e = g < a.N ? ((__double2hiint(a.sA[f * a.N + g]) >> 20) & 0x7ff) - 1023 : 0;
+          for (int kb = 0; kb < a.nkb; ++kb, ++st) {
+            const int slot = st % kDfRing, use = st / kDfRing;
+            if (kb + 1 < a.nkb) next(tile, f, kb + 1);
+            else if (f + 1 < FIELDS) next(tile, f + 1, 0);
+            else next(cb + 1 < ncb ? tile : tile + gridDim.x, 0, 0);
+            if (use > 0 && !mbar_wait(&P.empty[slot], (unsigned)((use - 1) & 1), a.err, 75)) {
+              ok = false;
+              break;
+            }
+            char *row = sm + slot * kDfStage + r * 128;
+#pragma unroll
+            for (int c = 0; c < kDfRun / 8; ++c) {
+              QfPack pack;
+#pragma unroll
+              for (int i = 0; i < 8; ++i) pack.put(i, v[c][i], e);
+              fetch(c);
+              pack.store(row, kDfPairA, c0 + c, r);
+            }
+            fence_proxy_async();
+            mbar_arrive(&P.full[slot]);
           }
         }
     }
   } else {
     // warp w: TMEM lanes 32 (w % 4) .. and half w / 4 of the columns
     const int half = warp >> 2, hc = a.cols / 2, row = (warp & 3) * 32 + lane;
-    const uint32_t base = P.tmem_base + ((uint32_t)((warp & 3) * 32) << 16) + half * hc;
+    const uint32_t base = tmem + ((uint32_t)((warp & 3) * 32) << 16) + half * hc;
     int chain = 0;
     for (int tile = blockIdx.x; tile < a.tiles; tile += gridDim.x) {
-      const long long g = (long long)(a.tile0 + tile) * kDfM + row;
+      const long long g = (long long)tile * kDfM + row;
       double acc[FIELDS];
 #pragma unroll
       for (int f = 0; f < FIELDS; ++f) acc[f] = 0.0;
@@ -324,14 +331,8 @@ __global__ void __launch_bounds__(kDfThreads, 1) k_df_density(const DfArgs a) {
   __syncthreads();
   if (warp == kDfDrainWarps) {
     tc_fence_after();
-    tmem_dealloc(P.tmem_base, 512);
+    tmem_dealloc(tmem, 512);
   }
-}
-
-static void form(const Density64 &d, const double *phi, const double *dphi, long long N, int tile0, int tiles,
-                 cudaStream_t st) {
-  k_df_digits<<<dim3(tiles, dphi ? 4 : 1), 256, 0, st>>>(phi, dphi, d.n, N, df_blocks(d.n), tile0, d.sA, d.A);
-  HQ_LAUNCH_CHECK();
 }
 
 void density64_basis(const Density64 &d, const double *phi, const double *dphi, long long N, cudaStream_t st) {
@@ -341,17 +342,17 @@ void density64_basis(const Density64 &d, const double *phi, const double *dphi, 
                                                   d.sA + f * N);
     HQ_LAUNCH_CHECK();
   }
-  if (d.keep) form(d, phi, dphi, N, 0, density64_tiles(N), st);
 }
 
 void density64(const Density64 &d, const double *phi, const double *dphi, const double *C, const double *occ, int nuse,
                long long N, double *rho, double *grho, double *psi, cudaStream_t st) {
   HQ_STAGE(ST_DENSITY, st);
-  const int nkb = df_blocks(d.n), tiles = density64_tiles(N), ranges = ceil_div(tiles, d.cap);
+  const int nkb = df_blocks(d.n);
   k_df_orbitals<<<nuse, 128, 0, st>>>(C, occ, d.n, nkb, d.eY, d.B);
   HQ_LAUNCH_CHECK();
   DfArgs a{};
-  a.A = d.A;
+  a.phi = phi;
+  a.dphi = dphi;
   a.B = d.B;
   a.sA = d.sA;
   a.eY = d.eY;
@@ -360,24 +361,20 @@ void density64(const Density64 &d, const double *phi, const double *dphi, const 
   a.psi = psi;
   a.err = d.err;
   a.N = N;
+  a.nao = d.n;
+  a.tiles = ceil_div(N, kDfM);
   a.nkb = nkb;
   a.nuse = nuse;
   a.cols = (std::min(nuse, kDfN) + 15) / 16 * 16;
   a.bufs = kQfDigits * a.cols * 2 <= 512 ? 2 : 1;
-  for (int k = 0; k < ranges; ++k) {
-    a.tile0 = (int)((long long)tiles * k / ranges);
-    a.tiles = (int)((long long)tiles * (k + 1) / ranges) - a.tile0;
-    a.field = density64_tile_bytes(d.n, 1) * a.tiles;
-    if (!d.keep) form(d, phi, dphi, N, a.tile0, a.tiles, st);
-    const int grid = std::min(152, a.tiles);
-    auto go = [&](auto kernel) {
-      ensure_dyn_smem((const void *)kernel, kDfSmem);
-      kernel<<<grid, kDfThreads, kDfSmem, st>>>(a);
-      HQ_LAUNCH_CHECK();
-    };
-    if (dphi) go(k_df_density<4>);
-    else go(k_df_density<1>);
-  }
+  const int grid = std::min(152, a.tiles);
+  auto go = [&](auto kernel) {
+    ensure_dyn_smem((const void *)kernel, kDfSmem);
+    kernel<<<grid, kDfThreads, kDfSmem, st>>>(a);
+    HQ_LAUNCH_CHECK();
+  };
+  if (dphi) go(k_df_density<4>);
+  else go(k_df_density<1>);
 }
 
 }  // namespace hqcgb

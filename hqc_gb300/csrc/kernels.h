@@ -57,22 +57,17 @@ void quad64_pair(const Quad64 &q, const double *phi, const double *w, const doub
                  bool accumulate, double *M, cudaStream_t st);
 
 // density_f64.cu: FP64 density from the orbitals on the tensor cores, up to
-// density64_max_ao() AOs.  A: digits of phi^T (and of the gradient's fields) for
-// `cap` tiles of points: all of them where the plan keeps them for a geometry (keep),
-// otherwise formed range by range of tiles for every density; sA [fields][N];
-// B, eY: digits and exponents of Y^T.
+// density64_max_ao() AOs.  sA [fields][N]: scales of the points; B, eY: digits and
+// exponents of Y^T.
 struct Density64 {
-  int n = 0, cap = 0;
-  bool keep = false;
-  char *A = nullptr, *B = nullptr;
+  int n = 0;
+  char *B = nullptr;
   double *sA = nullptr;
   int *eY = nullptr, *err = nullptr;
 };
 int density64_max_ao();
-int density64_tiles(long long N);
-int density64_min_tiles(long long N);  // fewer in a range would leave SMs idle
-size_t density64_tile_bytes(int nao, int fields);
 size_t density64_orbital_bytes(int nao);
+// scales of a geometry's AOs (and of their gradient's fields)
 void density64_basis(const Density64 &d, const double *phi, const double *dphi, long long N, cudaStream_t st);
 // rho (and grad rho, dphi not null) of the first nuse orbitals (nuse >= 1) after
 // density64_basis with the same AOs; psi not null: sqrt(f_k) psi_k into psi [nuse][N]

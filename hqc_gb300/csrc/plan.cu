@@ -289,15 +289,15 @@ static double occ_shift(const hqcgb_plan *p) {
   return -P.smearing_sigma * x;
 }
 
-// Digits of the AOs (quad_f64.cu, density_f64.cu: 16 bytes a value and operand) that
-// plans keep for a geometry instead of forming them for every density and
-// quadrature.  A bound for a plan and its batch workers together, because kept digits
-// would take twice what the AOs themselves do (H54 dzvp PBE 81^3 with forces: 8 GB
-// without, 24 with), and batches or grids that fit the device would not any more.
-// What does not fit is formed piece by piece in a scratch a few per cent of the plan's
-// size.  Kept / formed every time: H32 dzv LDA 65^3 (570 MB) 34 / 41 ms a run, H14
-// dzvp PBE 49^3 with forces (860 MB) 38 / 50.
-static constexpr long long kKeptDigits = 1LL << 30;
+// Digits of the AOs (quad_f64.cu: 16 bytes a value) that plans keep for a geometry
+// instead of forming them for every quadrature.  A bound for a plan and its batch workers
+// together: kept digits take twice what the AOs do (2.4 GB of H54 dzvp at 81^3), and
+// batches or grids that fit the device would not any more.  What does not fit is formed
+// piece by piece in a scratch a few per cent of the plan's size.  Kept / formed every time:
+// H32 dzv LDA 65^3 (300 MB) 33.4 / 36.1 ms a run, H14 dzvp PBE 49^3 with forces (150 MB)
+// 38.8 / 40.0; beyond the bound, the quadratures of an H54 dzvp PBE run at 65^3 (1.3 GB)
+// 74 / 88 ms of its 302, at 81^3 145 / 170 of 514.
+static constexpr long long kKeptDigits = 512LL << 20;
 
 static void create(const hqcgb_params *in, hqcgb_plan *p, long long digit_budget) {
   const hqcgb_params &P = *in;
@@ -500,7 +500,6 @@ static void create(const hqcgb_params *in, hqcgb_plan *p, long long digit_budget
     const Quad64Sizes field = quad64_grid_sizes(nao, p->ng), gram = quad64_linear_sizes(nao, gK);
     const bool legacy = p->hf && !p->exx_fused;
     Quad64 &q = p->q64;
-    Density64 &d = p->d64;
     q.n = nao;
     q.ng = p->ng;
     const std::vector<int> first = quad64_first(p->ng);
@@ -508,27 +507,14 @@ static void create(const hqcgb_params *in, hqcgb_plan *p, long long digit_budget
     q.first = p->alloc<int>(first.size());
     upload(q.first, first.data(), first.size() * sizeof(int));
     const size_t seg = std::max(field.seg_bytes, gram.seg_bytes);
-    const int fields = p->gga ? 4 : 1, tiles = density64_tiles(N);
-    if (!p->mixed && nao <= density64_max_ao()) d.n = nao;
-    const size_t tile = d.n ? density64_tile_bytes(nao, fields) : 0;
-    const size_t all = field.bytes + tile * tiles;
-    const bool keep = !p->mixed && (long long)all <= digit_budget;
+    const bool keep = !p->mixed && (long long)field.bytes <= digit_budget;
     const bool second = !keep || legacy;
     if (keep) {
-      p->kept_digits = (long long)all;
+      p->kept_digits = (long long)field.bytes;
       q.B = p->alloc<char>(field.bytes);
       q.eB = p->alloc<int>(field.exponents);
-      q.A = p->alloc<char>(seg * (second ? 2 : 1));
-      d.cap = tiles;
-      d.keep = true;
-      if (d.n) d.A = p->alloc<char>(tile * tiles);
-    } else {
-      // one scratch: a density and a quadrature follow one another on the plan's stream
-      const size_t want = std::max(2 * seg, tile * density64_min_tiles(N));
-      q.A = p->alloc<char>(want);
-      d.A = q.A;
-      if (tile) d.cap = (int)std::min<size_t>(tiles, want / tile);
     }
+    q.A = p->alloc<char>(seg * (second ? 2 : 1));
     if (second) q.X = q.A + seg;
     q.exponents = std::max(field.seg_exponents, gram.seg_exponents);
     q.eA = p->alloc<int>(q.exponents);
@@ -539,9 +525,11 @@ static void create(const hqcgb_params *in, hqcgb_plan *p, long long digit_budget
       HQ_CUDA(cudaMemset(p->tc_err, 0, sizeof(int)));
     }
     q.err = p->tc_err;
-    if (d.n) {
+    if (!p->mixed && nao <= density64_max_ao()) {
+      Density64 &d = p->d64;
+      d.n = nao;
       d.B = p->alloc<char>(density64_orbital_bytes(nao));
-      d.sA = p->alloc<double>(fields * N);
+      d.sA = p->alloc<double>((p->gga ? 4 : 1) * N);
       d.eY = p->alloc<int>(nao);
       d.err = p->tc_err;
     }
