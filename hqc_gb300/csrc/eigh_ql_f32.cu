@@ -17,7 +17,8 @@
 //
 // What bounds it is the chain of stage 2, about 0.85 n^2 rotations of a square
 // root and two divisions each; the block that generated a sweep used to wait
-// for the same block to apply it.  n = 270: 25.7 -> 14.2 ms (11.8 of them stage 2).
+// for the same block to apply it.  n = 270: 25.7 -> 11.4 ms (8.9 of them stage 2;
+// 11.8 where all lanes followed a sweep).
 #include <cooperative_groups.h>
 
 #include "common.cuh"
