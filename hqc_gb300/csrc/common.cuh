@@ -46,9 +46,11 @@ struct Error {
 #define HQ_CUDA(call)                                                               \
   do {                                                                              \
     cudaError_t _e = (call);                                                        \
-    if (_e != cudaSuccess)                                                          \
+    if (_e != cudaSuccess) {                                                        \
+      cudaGetLastError(); /* reported here: no later launch check may find it */    \
       throw ::hqcgb::Error{HQCGB_CUDA_ERROR, std::string(#call) + ": " +            \
                                                 cudaGetErrorString(_e)};            \
+    }                                                                               \
   } while (0)
 
 #define HQ_LAUNCH_CHECK()                                                           \
