@@ -19,7 +19,7 @@
 // drain warps.  Bound by the MMAs (72 a stage) and the instructions that form their digits
 // (about 80 a value) together.  Measured: 64 AOs, 38 orbitals, 65^3 points 0.18 ms (sum over
 // D on the FP64 pipe 1.87, digits kept in memory 0.18); 70 AOs, 7 orbitals, 49^3 with the
-// gradient 0.23 (1.05, 0.18); 270 AOs, 27 orbitals, 65^3 with the gradient 1.36 (kept 1.06,
+// gradient 0.23 (1.05, 0.18); 270 AOs, 27 orbitals, 65^3 with the gradient 1.3 (kept 1.06,
 // digits of a range of tiles formed in memory before its part of the density 3.5).  With
 // four forming warps 2.5; eight, whose 18 warps leave 96 registers and some spills of the
 // drains' in the gradient form, but 136 registers for those by setmaxnreg were slower.

@@ -2,6 +2,8 @@
 // tensor cores (the scheme is described in quad_f64.cu), and the PTX that only
 // its kernels use.
 #pragma once
+#include <cuda_bf16.h>
+
 #include "tc_ptx.cuh"
 
 namespace hqcgb {
@@ -24,19 +26,26 @@ __device__ __forceinline__ unsigned long long qf_fields(double x, int e) {
 // Eight consecutive K elements of one row: their digits as bf16, 16 bytes a
 // digit, stored into the K-major SW128 pattern (a 128-byte row holds 32
 // elements of two digits; `pair_stride` bytes from one pair of digits to the
-// next).
+// next).  Two elements at a time: 0x4300 | f is 128 + f in bf16 (256 for the first
+// digit's f = 128), and 192 less is the digit, exactly.
 struct QfPack {
   unsigned pk[kQfDigits][4];
-  float lo[kQfDigits];
+  unsigned long long even;
 
   __device__ __forceinline__ void put(int i, double x, int e) {
     const unsigned long long J = qf_fields(x, e);
+    if (!(i & 1)) {
+      even = J;
+      return;
+    }
+    const __nv_bfloat162 bias = __halves2bfloat162(__ushort_as_bfloat16(0x4340), __ushort_as_bfloat16(0x4340));
 #pragma unroll
     for (int s = 0; s < kQfDigits; ++s) {
-      const unsigned f = (unsigned)(J >> (7 * (kQfDigits - 1 - s))) & (s ? 127u : 255u);
-      const float v = __uint_as_float(0x4B000000u | f) - 8388672.f;  // 2^23 + f - (2^23 + 64), exact
-      if (i & 1) pk[s][i >> 1] = __byte_perm(__float_as_uint(lo[s]), __float_as_uint(v), 0x7632);
-      else lo[s] = v;
+      const int sh = 7 * (kQfDigits - 1 - s);
+      const unsigned mask = s ? 127u : 255u;
+      const unsigned w = ((unsigned)(even >> sh) & mask) | (((unsigned)(J >> sh) & mask) << 16) | 0x43004300u;
+      const __nv_bfloat162 v = __hsub2(*reinterpret_cast<const __nv_bfloat162 *>(&w), bias);
+      pk[s][i >> 1] = *reinterpret_cast<const unsigned *>(&v);
     }
   }
   // chunk c (0..3) of row r, `row` the row's first byte in the first pair

@@ -295,8 +295,8 @@ static double occ_shift(const hqcgb_plan *p) {
 // batches or grids that fit the device would not any more.  What does not fit is formed
 // piece by piece in a scratch a few per cent of the plan's size.  Kept / formed every time:
 // H32 dzv LDA 65^3 (300 MB) 33.4 / 36.1 ms a run, H14 dzvp PBE 49^3 with forces (150 MB)
-// 38.8 / 40.0; beyond the bound, the quadratures of an H54 dzvp PBE run at 65^3 (1.3 GB)
-// 74 / 88 ms of its 302, at 81^3 145 / 170 of 514.
+// 38.8 / 40.0; beyond the bound, an H54 dzvp PBE run with forces at 65^3 (1.3 GB) 280 / 293,
+// at 81^3 468 / 493 (from the quadratures' share).
 static constexpr long long kKeptDigits = 512LL << 20;
 
 static void create(const hqcgb_params *in, hqcgb_plan *p, long long digit_budget) {

@@ -39,7 +39,7 @@
 // by the tensor pipe, at 36 products a term.  Measured, digits
 // of the weighted operand and sums included, FP64 pipe -> this: 64 AOs and 65^3
 // points 2.24 -> 0.29 ms, 70 AOs and 49^3 points with the gradient term 2.21 ->
-// 0.30 ms, 8 AOs and 41^3 points 0.57 -> 0.07 ms (with a power of two a row 0.24,
+// 0.26 ms, 8 AOs and 41^3 points 0.57 -> 0.07 ms (with a power of two a row 0.24,
 // 0.32 and 0.08).
 #include <algorithm>
 #include <cmath>
@@ -161,13 +161,18 @@ static size_t form_smem(int mode) {
   return sizeof(double) * (kQfFormRows * kQfRowLd + (mode == 0 ? 0 : mode == 1 ? 1 : 4) * kQfBlk) + sizeof(int) * kQfBlk;
 }
 
+// Blocks an SM that the registers leave room for: the gradient form has four fields'
+// loads under way and is better off with more of them (quadratures of an H14 dzvp PBE run
+// at 49^3 with 3 / 4 / 5 blocks 5.5 / 6.2 / 6.3 ms, of an H32 dzv LDA run 7.7 / 7.0 / 6.6).
+constexpr int qf_form_blocks(int mode) { return mode == 2 ? 3 : 5; }
+
 // Grid (blocks of points, row groups).  A warp loads a row, neighbouring lanes
 // neighbouring points, and its maximum gives the exponent; then the warps take a
 // stage of all eight rows in turn, eight points of a row a lane, so that what they
 // store is 1 KB in one piece.  Points beyond a block's last become zeros; rows beyond
 // n are left alone (they only reach destination rows and columns that nothing reads).
 template <int MODE>
-__global__ void __launch_bounds__(kQfFormRows * 32) k_qf_digits(const QfSource a) {
+__global__ void __launch_bounds__(kQfFormRows * 32, qf_form_blocks(MODE)) k_qf_digits(const QfSource a) {
   extern __shared__ __align__(16) double s_x[];  // [rows][kQfRowLd]
   double *s_w = s_x + kQfFormRows * kQfRowLd, *s_u = s_w + kQfBlk;
   int *s_off = reinterpret_cast<int *>(s_w + (MODE == 0 ? 0 : MODE == 1 ? 1 : 4) * kQfBlk);  // the block's points
